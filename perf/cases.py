@@ -152,6 +152,48 @@ def work(case):
     return {"bytes": 4 * n * (5 if case["op"] == "rms_norm_swiglu" else 2), "flops": 5 * n}
 
 
+def exact(case, seed):
+    """What run() returns on prepare(case, seed), in 64 bits with torch's own operations."""
+    s = prepare(case, seed)
+    kind = case["kind"]
+    if kind == "attn":
+        return _attn_exact(case, s["q"], s["k"], s["v"])
+    if kind in ("gemm", "grouped"):
+        return s["a"].double() @ s["bt"].double().mT
+    x, w = s["x"].double(), s["w"].double()
+    if case["op"] == "softmax":
+        return torch.softmax(x, dim=1)
+    if case["op"] == "layer_norm":
+        y = x - x.mean(dim=1, keepdim=True)
+        return y * torch.rsqrt(y.square().mean(dim=1, keepdim=True) + 1e-5) * w + s["bias"].double()
+    y = x * torch.rsqrt(x.square().mean(dim=1, keepdim=True) + 1e-6) * w
+    gate = s["gate"].double()
+    return [y, gate * torch.sigmoid(gate) * s["up"].double()]
+
+
+def _attn_exact(case, q, k, v):
+    B, H, S, D = q.shape
+    group = H // case["H_kv"]
+    o = torch.empty(B, H, S, D, device=q.device, dtype=torch.float64)
+    lse = torch.empty(B, H, S, device=q.device, dtype=torch.float64)
+    rows = 4096                              # query rows of one head at a time: 0.27 GB of scores at most
+    keys = torch.arange(S, device=q.device)
+    for b in range(B):
+        for h in range(H):
+            kd, vd = k[b, h // group].double(), v[b, h // group].double()
+            for r in range(0, S, rows):
+                scores = q[b, h, r:r + rows].double() @ kd.mT
+                scores *= D ** -0.5
+                if case["causal"]:
+                    scores.masked_fill_(keys[None, :] > keys[r:r + rows, None], -math.inf)
+                top = scores.amax(dim=1, keepdim=True)
+                scores.sub_(top).exp_()
+                total = scores.sum(dim=1, keepdim=True)
+                o[b, h, r:r + rows] = (scores @ vd) / total
+                lse[b, h, r:r + rows] = (top + total.log())[:, 0]
+    return [o, lse] if case["lse"] else [o]
+
+
 def tolerance(case):
     """Four to seven times the distance to the same result computed in 64 bits, which each line gives."""
     kind = case["kind"]
