@@ -8,21 +8,30 @@
 // block*64. All four are bound by HBM: 8 bytes per element (one fp32 read, one fp32
 // write; the weight vectors stay in cache), 12 for SwiGLU.
 //
-// What is kept: one read of X, the row in registers across the passes, 128-bit
-// accesses. What is different:
-//   * the threads that share a row are chosen from the row length: one warp per row
-//     up to 2048 columns (reductions are five shuffles, no shared memory, no block
-//     barrier; four rows per CTA), 256 threads up to 8192, 1024 threads up to 32768;
-//   * any N that is a multiple of 4 (ragged rows are guarded per 128-bit access);
-//   * a persistent grid sized from the SM count, rows handed out round-robin, so
-//     small rows do not pay one CTA launch each;
-//   * X and Y are accessed with the streaming cache hints (read once, written
-//     once), the weight vectors through the read-only path;
-//   * one reduction per row instead of two: softmax merges (max, sum of exponentials)
-//     pairs by the online-softmax rule and rescales once; layer norm merges (count,
-//     mean, centred sum of squares) triples by Chan's rule, which also keeps its
-//     accuracy for rows with a large mean, where the reference's E[x^2] - mean^2
-//     cancels. With several warps per row that is one block barrier per row.
+// What is kept: one read of X, the row on chip across the passes, 128-bit accesses. What is
+// different:
+//   * one block per row (one per four rows with a warp each up to 2048 columns) and no loop
+//     over rows in the kernel: a block that ends makes room for one whose loads start at
+//     once, so reads and writes of different rows stay mixed. A persistent grid of the same
+//     blocks falls into step (all read, then all write): rows of 8192 columns, 0.5 GB in,
+//     0.5 GB out, softmax 171 us persistent, 156 us this way (6880 GB/s); rows of 1024
+//     columns 91 against 80 us; and a ring in shared memory kept full by bulk copies 170 to 203;
+//   * the threads per row follow its length, eight float4s each (any N that is a multiple
+//     of 4: the last ones are guarded), in steps of a warp: rows of 9000 columns took 300 us
+//     on a power-of-two block that they half filled, and take 157;
+//   * above 16384 columns a thread holds eight float4s in registers and up to eight in
+//     shared memory, so that two blocks still fit an SM's register file and overlap
+//     (softmax, 30000 columns: 197 us with the whole row in registers, 169 now);
+//   * few rows (at most two per SM, up to 4096 columns) are spread over four times the
+//     threads, and the weights are fetched ahead of the reduction: latency counts there (16
+//     rows of 2048 columns, layer norm: 4.2 us, now 2.1);
+//   * X and Y are accessed with the streaming cache hints (read once, written once), the
+//     weight vectors through the read-only path;
+//   * softmax merges (max, sum of exponentials) pairs by the online-softmax rule and
+//     rescales once; layer norm takes the mean, then the centred sum of squares of the
+//     values on chip, which keeps its accuracy for rows with a large mean, where the
+//     reference's E[x^2] - mean^2 cancels. With several warps per row a reduction costs one
+//     block barrier.
 #include "host_common.h"
 #include "sm100_prims.cuh"
 
@@ -44,15 +53,12 @@ struct RowParams {
   float eps;
 };
 
-// Reductions over the kTpr threads that share a row. Each op needs exactly one:
-// a sum (RMS norm), a (max, sum of exponentials) pair merged with the online-softmax
-// rule, or a (count, mean, M2) triple merged with Chan's rule (layer norm). With
-// more than one warp per row the warps' partials meet in shared memory behind ONE
-// block barrier: `red` alternates between two buffers from row to row, so a warp
-// writing the next row's partials cannot overrun a reader of this row's (it would
-// first have to pass the next row's barrier, which the reader also has to reach).
+// Reductions over the threads that share a row: a sum, or a (max, sum of exponentials)
+// pair merged with the online-softmax rule. With more than one warp per row the warps'
+// partials meet in shared memory behind ONE block barrier: the buffer alternates between
+// two from reduction to reduction, so a warp writing the next partials cannot overrun a
+// reader of these (it would first have to pass a barrier which the reader also has to reach).
 struct Pair { float m, s; };          // running max and sum of 2^((x - m) log2 e)
-struct Moments { float n, mean, m2; };
 
 __device__ __forceinline__ Pair merge(Pair a, Pair b) {
   const float m = fmaxf(a.m, b.m);
@@ -61,138 +67,156 @@ __device__ __forceinline__ Pair merge(Pair a, Pair b) {
   const float fb = b.m == m ? 1.0f : ex2_approx((b.m - m) * kLog2e);
   return {m, a.s * fa + b.s * fb};
 }
-__device__ __forceinline__ Moments merge(Moments a, Moments b) {
-  const float n = a.n + b.n;
-  const float rb = n > 0.0f ? b.n / n : 0.0f;
-  const float d = b.mean - a.mean;
-  return {n, a.mean + d * rb, a.m2 + b.m2 + d * d * a.n * rb};
-}
 __device__ __forceinline__ float merge(float a, float b) { return a + b; }
 
 __device__ __forceinline__ float shfl_xor(float v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
 __device__ __forceinline__ Pair shfl_xor(Pair v, int o) { return {shfl_xor(v.m, o), shfl_xor(v.s, o)}; }
-__device__ __forceinline__ Moments shfl_xor(Moments v, int o) {
-  return {shfl_xor(v.n, o), shfl_xor(v.mean, o), shfl_xor(v.m2, o)};
-}
 __device__ __forceinline__ float identity(float) { return 0.0f; }
 __device__ __forceinline__ Pair identity(Pair) { return {-INFINITY, 0.0f}; }
-__device__ __forceinline__ Moments identity(Moments) { return {0.0f, 0.0f, 0.0f}; }
 
-template <int kTpr, typename T>
-__device__ __forceinline__ T row_reduce(T v, T* red /* [2][32] */, int parity) {
+template <typename T>
+__device__ __forceinline__ T warp_reduce(T v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = merge(v, shfl_xor(v, o));
-  if (kTpr > 32) {
-    constexpr int kWarps = kTpr / 32;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    T* buf = red + parity * 32;
-    if (lane == 0) buf[warp] = v;
-    __syncthreads();
-    v = lane < kWarps ? buf[lane] : identity(v);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = merge(v, shfl_xor(v, o));
-  }
   return v;
 }
 
-// kTpr threads per row, up to kVec 128-bit accesses per thread.
-template <int kOp, int kTpr, int kVec>
-__global__ void __launch_bounds__(kTpr == 32 ? 128 : kTpr)
+__device__ __forceinline__ float4 load_once(const float4* p) { return __ldcs(p); }
+__device__ __forceinline__ void cp_async16(uint32_t dst_smem, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_smem), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// One row per block (kWarpRows = false: all threads of the block share it) or per warp
+// (kWarpRows = true, four rows per block). A thread holds the row's float4s t, t + T, ...
+// (T threads per row): the first kVec of them in registers, kPark more in shared memory
+// slots that no other thread touches.
+template <int kOp, bool kWarpRows, int kVec, int kPark>
+__global__ void __launch_bounds__(kWarpRows ? 128 : 512, kWarpRows ? 1 : 2)
 rowwise_kernel(const RowParams p) {
-  __shared__ float red_raw[2 * 32 * 3];
-  constexpr int kRowsPerCta = kTpr == 32 ? 4 : 1;
-  const int t = threadIdx.x % kTpr;                 // position within the row's thread group
-  const int sub = threadIdx.x / kTpr;               // which of the CTA's rows
+  __shared__ float2 red[2][32];
+  extern __shared__ __align__(16) float4 parked[];   // [kPark][T]
+  const int tpr = kWarpRows ? 32 : blockDim.x;       // threads per row
+  const int t = kWarpRows ? threadIdx.x & 31 : threadIdx.x;
+  const int row = kWarpRows ? blockIdx.x * 4 + (threadIdx.x >> 5) : blockIdx.x;
+  if (kWarpRows && row >= p.rows) return;            // the last block's rows may be fewer; no block barrier follows
+  const float4* x4 = reinterpret_cast<const float4*>(p.x) + (size_t)row * p.n4;
+  float4* y4 = reinterpret_cast<float4*>(p.y) + (size_t)row * p.n4;
   const float4* w4 = reinterpret_cast<const float4*>(p.w);
   const float4* b4 = reinterpret_cast<const float4*>(p.bias);
+  const float fill = kOp == kOpSoftmax ? -INFINITY : 0.0f;
+
   int parity = 0;
+  auto reduce = [&](auto v) {
+    v = warp_reduce(v);
+    if constexpr (!kWarpRows) {
+      decltype(v)* buf = reinterpret_cast<decltype(v)*>(red[parity]);
+      parity ^= 1;
+      if ((t & 31) == 0) buf[t >> 5] = v;
+      __syncthreads();
+      v = warp_reduce((t & 31) < (tpr >> 5) ? buf[t & 31] : identity(v));
+    }
+    return v;
+  };
 
-  for (int row0 = blockIdx.x * kRowsPerCta; row0 < p.rows;
-       row0 += gridDim.x * kRowsPerCta, parity ^= 1) {
-    const int row = row0 + sub;
-    const bool live = row < p.rows;   // a CTA's last group of rows may be partial (warp-per-row only)
-    const float4* x4 = reinterpret_cast<const float4*>(p.x) + (size_t)(live ? row : 0) * p.n4;
-    float4* y4 = reinterpret_cast<float4*>(p.y) + (size_t)(live ? row : 0) * p.n4;
-
-    float4 v[kVec];
+#pragma unroll
+  for (int i = 0; i < kPark; ++i) {
+    const int c = t + (kVec + i) * tpr;
+    if (c < p.n4) cp_async16(smem_u32(parked + i * tpr + t), x4 + c);
+    else parked[i * tpr + t] = make_float4(fill, fill, fill, fill);
+  }
+  float4 v[kVec];
+#pragma unroll
+  for (int i = 0; i < kVec; ++i) {
+    const int c = t + i * tpr;
+    v[i] = c < p.n4 ? load_once(x4 + c) : make_float4(fill, fill, fill, fill);
+  }
+  // short shares: the vectors are fetched ahead of the reduction, so that their latency
+  // does not follow it (longer shares have no registers for that)
+  constexpr bool kEarly = kOp != kOpSoftmax && kVec <= 2;
+  float4 w[kEarly ? kVec : 1], b[kEarly && kOp == kOpLayerNorm ? kVec : 1];
+  if constexpr (kEarly) {
 #pragma unroll
     for (int i = 0; i < kVec; ++i) {
-      const int c = t + i * kTpr;
-      const float fill = kOp == kOpSoftmax ? -INFINITY : 0.0f;
-      v[i] = (live && c < p.n4) ? __ldcs(x4 + c) : make_float4(fill, fill, fill, fill);
+      const int c = t + i * tpr;
+      if (c < p.n4) {
+        w[i] = __ldg(w4 + c);
+        if constexpr (kOp == kOpLayerNorm) b[i] = __ldg(b4 + c);
+      }
     }
+  }
+  if (kPark > 0) cp_async_wait_all();
 
-    if (kOp == kOpSoftmax) {
-      float m = -INFINITY;
+  // f(element group, its index in the row) over everything this thread holds
+  auto each = [&](auto f) {
 #pragma unroll
-      for (int i = 0; i < kVec; ++i) m = fmaxf(fmaxf(m, fmaxf(v[i].x, v[i].y)), fmaxf(v[i].z, v[i].w));
-      // exponentials against this thread's own maximum, rescaled once the row's is known
-      const float neg = m == -INFINITY ? 0.0f : -m * kLog2e;
-      float s = 0.0f;
-#pragma unroll
-      for (int i = 0; i < kVec; ++i) {
-        v[i].x = ex2_approx(fmaf(v[i].x, kLog2e, neg));
-        v[i].y = ex2_approx(fmaf(v[i].y, kLog2e, neg));
-        v[i].z = ex2_approx(fmaf(v[i].z, kLog2e, neg));
-        v[i].w = ex2_approx(fmaf(v[i].w, kLog2e, neg));
-        s += (v[i].x + v[i].y) + (v[i].z + v[i].w);   // padding lanes hold 2^-inf = 0
+    for (int i = 0; i < kVec; ++i) f(v[i], t + i * tpr);
+#pragma unroll 1
+    for (int i = 0; i < kPark; ++i) {
+      float4 x = parked[i * tpr + t];
+      f(x, t + (kVec + i) * tpr);
+      parked[i * tpr + t] = x;
+    }
+  };
+
+  float mul;   // what the row's (centred, exponentiated) values are scaled by
+  if constexpr (kOp == kOpSoftmax) {
+    float m = -INFINITY;
+    each([&](float4& x, int) { m = fmaxf(fmaxf(m, fmaxf(x.x, x.y)), fmaxf(x.z, x.w)); });
+    // exponentials against this thread's own maximum, rescaled once the row's is known
+    const float neg = m == -INFINITY ? 0.0f : -m * kLog2e;
+    float s = 0.0f;
+    each([&](float4& x, int) {
+      x.x = ex2_approx(fmaf(x.x, kLog2e, neg));
+      x.y = ex2_approx(fmaf(x.y, kLog2e, neg));
+      x.z = ex2_approx(fmaf(x.z, kLog2e, neg));
+      x.w = ex2_approx(fmaf(x.w, kLog2e, neg));
+      s += (x.x + x.y) + (x.z + x.w);   // padding lanes hold 2^-inf = 0
+    });
+    const Pair tot = reduce(Pair{m, s});
+    mul = (m == tot.m ? 1.0f : ex2_approx((m - tot.m) * kLog2e)) / tot.s;
+  } else if constexpr (kOp == kOpRmsNorm) {
+    float s = 0.0f;
+    each([&](float4& x, int) { s += (x.x * x.x + x.y * x.y) + (x.z * x.z + x.w * x.w); });
+    mul = rsqrtf(reduce(s) * p.inv_n + p.eps);
+  } else {
+    float s = 0.0f;
+    each([&](float4& x, int) { s += (x.x + x.y) + (x.z + x.w); });   // padding lanes hold zeros
+    const float mean = reduce(s) * p.inv_n;
+    float q = 0.0f;
+    each([&](float4& x, int c) {
+      if (c < p.n4) {
+        x.x -= mean; x.y -= mean; x.z -= mean; x.w -= mean;
+        q += (x.x * x.x + x.y * x.y) + (x.z * x.z + x.w * x.w);
       }
-      const Pair tot = row_reduce<kTpr>(Pair{m, s}, reinterpret_cast<Pair*>(red_raw), parity);
-      const float f = (m == tot.m ? 1.0f : ex2_approx((m - tot.m) * kLog2e)) / tot.s;
-#pragma unroll
-      for (int i = 0; i < kVec; ++i) {
-        const int c = t + i * kTpr;
-        if (live && c < p.n4)
-          __stcs(y4 + c, make_float4(v[i].x * f, v[i].y * f, v[i].z * f, v[i].w * f));
-      }
-    } else if (kOp == kOpRmsNorm) {
-      float s = 0.0f;
-#pragma unroll
-      for (int i = 0; i < kVec; ++i)
-        s += (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
-      s = row_reduce<kTpr>(s, red_raw, parity);
-      const float rstd = rsqrtf(s * p.inv_n + p.eps);
-#pragma unroll
-      for (int i = 0; i < kVec; ++i) {
-        const int c = t + i * kTpr;
-        if (live && c < p.n4) {
-          const float4 w = __ldg(w4 + c);
-          __stcs(y4 + c, make_float4(v[i].x * rstd * w.x, v[i].y * rstd * w.y, v[i].z * rstd * w.z,
-                                     v[i].w * rstd * w.w));
-        }
-      }
-    } else {
-      // this thread's own count, mean and centred sum of squares
-      float s = 0.0f, cnt = 0.0f;
-#pragma unroll
-      for (int i = 0; i < kVec; ++i) {
-        s += (v[i].x + v[i].y) + (v[i].z + v[i].w);   // padding lanes hold zeros
-        if (t + i * kTpr < p.n4) cnt += 4.0f;
-      }
-      const float mean_t = cnt > 0.0f ? s / cnt : 0.0f;
-      float q = 0.0f;
-#pragma unroll
-      for (int i = 0; i < kVec; ++i) {
-        if (t + i * kTpr < p.n4) {
-          const float dx = v[i].x - mean_t, dy = v[i].y - mean_t, dz = v[i].z - mean_t, dw = v[i].w - mean_t;
-          q += (dx * dx + dy * dy) + (dz * dz + dw * dw);
-        }
-      }
-      const Moments tot = row_reduce<kTpr>(Moments{cnt, mean_t, q}, reinterpret_cast<Moments*>(red_raw), parity);
-      const float rstd = rsqrtf(tot.m2 * p.inv_n + p.eps);
-#pragma unroll
-      for (int i = 0; i < kVec; ++i) {
-        const int c = t + i * kTpr;
-        if (live && c < p.n4) {
-          const float4 w = __ldg(w4 + c);
-          const float4 b = __ldg(b4 + c);
-          __stcs(y4 + c, make_float4(fmaf((v[i].x - tot.mean) * rstd, w.x, b.x),
-                                     fmaf((v[i].y - tot.mean) * rstd, w.y, b.y),
-                                     fmaf((v[i].z - tot.mean) * rstd, w.z, b.z),
-                                     fmaf((v[i].w - tot.mean) * rstd, w.w, b.w)));
-        }
+    });
+    mul = rsqrtf(reduce(q) * p.inv_n + p.eps);
+  }
+
+  auto write = [&](const float4& x, int c, const float4* early_w, const float4* early_b) {
+    float4 o = make_float4(x.x * mul, x.y * mul, x.z * mul, x.w * mul);
+    if constexpr (kOp != kOpSoftmax) {
+      const float4 wi = early_w != nullptr ? *early_w : __ldg(w4 + c);
+      if constexpr (kOp == kOpRmsNorm) {
+        o = make_float4(o.x * wi.x, o.y * wi.y, o.z * wi.z, o.w * wi.w);
+      } else {
+        const float4 bi = early_b != nullptr ? *early_b : __ldg(b4 + c);
+        o = make_float4(fmaf(o.x, wi.x, bi.x), fmaf(o.y, wi.y, bi.y), fmaf(o.z, wi.z, bi.z), fmaf(o.w, wi.w, bi.w));
       }
     }
+    __stcs(y4 + c, o);
+  };
+#pragma unroll
+  for (int i = 0; i < kVec; ++i) {
+    const int c = t + i * tpr;
+    if (c < p.n4)
+      write(v[i], c, kEarly ? &w[kEarly ? i : 0] : nullptr,
+            kEarly && kOp == kOpLayerNorm ? &b[kEarly && kOp == kOpLayerNorm ? i : 0] : nullptr);
+  }
+#pragma unroll 4
+  for (int i = 0; i < kPark; ++i) {
+    const int c = t + (kVec + i) * tpr;
+    if (c < p.n4) write(parked[i * tpr + t], c, nullptr, nullptr);
   }
 }
 
@@ -202,46 +226,41 @@ __device__ __forceinline__ float silu_mul(float g, float u) {
 }
 
 constexpr int kSwigluThreads = 256;
-constexpr int kSwigluUnroll = 4;   // independent 128-bit load pairs in flight per thread
 
+// kUnroll: independent 128-bit load pairs in flight per thread
+template <int kUnroll>
 __global__ void __launch_bounds__(kSwigluThreads)
 swiglu_kernel(float* __restrict__ out, const float* __restrict__ gate, const float* __restrict__ up,
               size_t n4) {
   const float4* g4 = reinterpret_cast<const float4*>(gate);
   const float4* u4 = reinterpret_cast<const float4*>(up);
   float4* o4 = reinterpret_cast<float4*>(out);
-  const size_t stride = (size_t)gridDim.x * kSwigluThreads;
-  for (size_t base = (size_t)blockIdx.x * kSwigluThreads + threadIdx.x; base < n4;
-       base += stride * kSwigluUnroll) {
-    float4 g[kSwigluUnroll], u[kSwigluUnroll];
+  const size_t base = (size_t)blockIdx.x * (kSwigluThreads * kUnroll) + threadIdx.x;
+  float4 g[kUnroll], u[kUnroll];
 #pragma unroll
-    for (int i = 0; i < kSwigluUnroll; ++i) {
-      const size_t c = base + i * stride;
-      if (c < n4) {
-        g[i] = __ldcs(g4 + c);
-        u[i] = __ldcs(u4 + c);
-      }
+  for (int i = 0; i < kUnroll; ++i) {
+    const size_t c = base + i * kSwigluThreads;
+    if (c < n4) {
+      g[i] = __ldcs(g4 + c);
+      u[i] = __ldcs(u4 + c);
     }
+  }
 #pragma unroll
-    for (int i = 0; i < kSwigluUnroll; ++i) {
-      const size_t c = base + i * stride;
-      if (c < n4)
-        __stcs(o4 + c, make_float4(silu_mul(g[i].x, u[i].x), silu_mul(g[i].y, u[i].y),
-                                   silu_mul(g[i].z, u[i].z), silu_mul(g[i].w, u[i].w)));
-    }
+  for (int i = 0; i < kUnroll; ++i) {
+    const size_t c = base + i * kSwigluThreads;
+    if (c < n4)
+      __stcs(o4 + c, make_float4(silu_mul(g[i].x, u[i].x), silu_mul(g[i].y, u[i].y), silu_mul(g[i].z, u[i].z),
+                                 silu_mul(g[i].w, u[i].w)));
   }
 }
 
-template <int kOp, int kTpr, int kVec>
-int launch_one(const DeviceCtx& ctx, const RowParams& p, cudaStream_t stream) {
-  constexpr int kRowsPerCta = kTpr == 32 ? 4 : 1;
-  constexpr int kThreads = kTpr == 32 ? 128 : kTpr;
-  // enough resident CTAs per SM to keep ~2048 threads' worth of loads in flight
-  const int ctas_per_sm = 2048 / kThreads > 8 ? 8 : 2048 / kThreads;
-  const long long want = ((long long)p.rows + kRowsPerCta - 1) / kRowsPerCta;
-  const long long cap = (long long)ctx.sm_count * ctas_per_sm;
-  const int grid = (int)(want < cap ? want : cap);
-  rowwise_kernel<kOp, kTpr, kVec><<<grid, kThreads, 0, stream>>>(p);
+template <int kOp, bool kWarpRows, int kVec, int kPark = 0>
+int launch_one(const RowParams& p, cudaStream_t stream) {
+  // threads per row, and blocks: one per row, or one per four rows
+  const int per = kVec + kPark;
+  const int threads = kWarpRows ? 128 : ((p.n4 + per - 1) / per + 31) / 32 * 32;
+  const int grid = kWarpRows ? (p.rows + 3) / 4 : p.rows;
+  rowwise_kernel<kOp, kWarpRows, kVec, kPark><<<grid, threads, (size_t)kPark * threads * 16, stream>>>(p);
   PTXB200_CUDA_TRY(cudaGetLastError());
   return PTXB200_OK;
 }
@@ -249,22 +268,27 @@ int launch_one(const DeviceCtx& ctx, const RowParams& p, cudaStream_t stream) {
 template <int kOp>
 int dispatch(const DeviceCtx& ctx, const RowParams& p, cudaStream_t stream) {
   const int n4 = p.n4;
+  // At most two rows per SM: nothing overlaps, so a row's own latency is the launch's. 200 rows
+  // of 2048 columns: 2.3 us against 2.6 with a warp per row (layer norm 2.4 against 4.4); above
+  // 4096 columns the shorter chain per thread no longer pays (200 rows of 8192: 5.2 against 4.4).
+  if (p.rows <= 2 * ctx.sm_count && n4 > 128 && n4 <= 2 * 512) return launch_one<kOp, false, 2>(p, stream);
   if (n4 <= 32 * 16) {
     const int per = (n4 + 31) / 32;
-    if (per <= 1) return launch_one<kOp, 32, 1>(ctx, p, stream);
-    if (per <= 2) return launch_one<kOp, 32, 2>(ctx, p, stream);
-    if (per <= 4) return launch_one<kOp, 32, 4>(ctx, p, stream);
-    if (per <= 8) return launch_one<kOp, 32, 8>(ctx, p, stream);
-    return launch_one<kOp, 32, 16>(ctx, p, stream);
+    if (per <= 1) return launch_one<kOp, true, 1>(p, stream);
+    if (per <= 2) return launch_one<kOp, true, 2>(p, stream);
+    if (per <= 4) return launch_one<kOp, true, 4>(p, stream);
+    if (per <= 8) return launch_one<kOp, true, 8>(p, stream);
+    return launch_one<kOp, true, 16>(p, stream);
   }
-  if (n4 <= 256 * 8) {
-    const int per = (n4 + 255) / 256;
-    if (per <= 4) return launch_one<kOp, 256, 4>(ctx, p, stream);
-    return launch_one<kOp, 256, 8>(ctx, p, stream);
-  }
-  const int per = (n4 + 1023) / 1024;
-  if (per <= 4) return launch_one<kOp, 1024, 4>(ctx, p, stream);
-  return launch_one<kOp, 1024, 8>(ctx, p, stream);
+  if (n4 <= 8 * 512) return launch_one<kOp, false, 8>(p, stream);
+  static PerDeviceOnce attr_once;
+  const int rc = attr_once.run(ctx.device, []() -> int {
+    PTXB200_CUDA_TRY(cudaFuncSetAttribute(rowwise_kernel<kOp, false, 8, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          512 * 8 * 16));
+    return PTXB200_OK;
+  });
+  if (rc != PTXB200_OK) return rc;
+  return launch_one<kOp, false, 8, 8>(p, stream);
 }
 
 }  // namespace
@@ -291,11 +315,15 @@ int launch_rowwise(const DeviceCtx& ctx, int op, float* y, const float* x, const
 int launch_swiglu(const DeviceCtx& ctx, float* out, const float* gate, const float* up, size_t n,
                   cudaStream_t stream) {
   const size_t n4 = n / 4;
-  const size_t per_cta = (size_t)kSwigluThreads * kSwigluUnroll;
-  const size_t want = (n4 + per_cta - 1) / per_cta;
-  const size_t cap = (size_t)ctx.sm_count * 8;
-  const int grid = (int)(want < cap ? want : cap);
-  swiglu_kernel<<<grid, kSwigluThreads, 0, stream>>>(out, gate, up, n4);
+  // one load pair per thread while that fits the machine in one round (2 us calls), else
+  // four; blocks that each run once, for the same reason as above (65536 x 4096: 459 us
+  // against 498 for a persistent grid)
+  const bool small = n4 <= (size_t)ctx.sm_count * 8 * kSwigluThreads;
+  const size_t per_block = (size_t)kSwigluThreads * (small ? 1 : 4);
+  const size_t blocks = (n4 + per_block - 1) / per_block;
+  if (blocks > 0x7fffffffu) return PTXB200_E_SHAPE;
+  if (small) swiglu_kernel<1><<<(unsigned)blocks, kSwigluThreads, 0, stream>>>(out, gate, up, n4);
+  else swiglu_kernel<4><<<(unsigned)blocks, kSwigluThreads, 0, stream>>>(out, gate, up, n4);
   PTXB200_CUDA_TRY(cudaGetLastError());
   return PTXB200_OK;
 }

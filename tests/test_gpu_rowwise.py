@@ -94,6 +94,36 @@ def test_rowwise_properties_at_full_size(pkg, gpu):
     assert pkg.ops.sync_status() == 0
 
 
+# Either side of every rule that picks the threads per row: warp / block per row (N = 2048),
+# few rows (two per SM: 296 on 148 SMs; N = 512 and 4096), float4s in shared memory (N = 16384)
+# and a last float4 of the row in each of a thread's places.
+@pytest.mark.parametrize("rows,N", [(5, 512), (5, 516), (296, 2048), (297, 2048), (297, 2052), (296, 4096), (296, 4100),
+                                    (300, 4096), (3, 16384), (3, 16388), (300, 16388), (2, 28676), (2, 32764), (150, 32768)])
+def test_rowwise_edges_against_64_bit(pkg, gpu, rows, N):
+    g = torch.Generator(device=gpu).manual_seed(rows * 31 + N)
+    X = torch.randn(rows, N, generator=g, device=gpu)
+    X[0, 1] = float("-inf")                     # a masked score weighs zero
+    W, Bias = (torch.randn(N, generator=g, device=gpu) for _ in range(2))
+    guard = torch.full((rows + 2, N), 7.0, device=gpu)
+    Y = pkg.ops.softmax(X, out=guard[1:rows + 1])
+    assert torch.all(guard[0] == 7.0) and torch.all(guard[rows + 1] == 7.0)
+    # an exponential is off by 2 ulp plus the rounding of its argument (|x| < 8: 2^-21), a
+    # sum of positive terms by about log2 N roundings
+    torch.testing.assert_close(Y.double(), torch.softmax(X.double(), dim=1), rtol=4e-6, atol=0)
+    X[0, 1] = 0.5
+    D = X.double()
+    # values up to 5.5, weights up to 4.5, and rstd within (log2 N + 8) roundings: 25 * 20 * 2^-24
+    R = D * torch.rsqrt(D.square().mean(dim=1, keepdim=True) + 1e-6) * W.double()
+    torch.testing.assert_close(pkg.ops.rms_norm(X, W).double(), R, rtol=0, atol=3e-5)
+    C = D - D.mean(dim=1, keepdim=True)
+    L = C * torch.rsqrt(C.square().mean(dim=1, keepdim=True) + 1e-5) * W.double() + Bias.double()
+    torch.testing.assert_close(pkg.ops.layer_norm(X, W, Bias).double(), L, rtol=0, atol=3e-5)
+    inplace = X.clone()
+    pkg.ops.softmax(inplace, out=inplace)
+    torch.testing.assert_close(inplace.double(), torch.softmax(D, dim=1), rtol=4e-6, atol=0)
+    assert pkg.ops.sync_status() == 0
+
+
 def test_rowwise_bad_arguments(pkg, gpu):
     n = pkg.native
     L = n.lib()
