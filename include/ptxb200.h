@@ -47,7 +47,7 @@ extern "C" {
 #define PTXB200_GEMM_NO_SPLIT 0x2u /* never cut tiles along K: every C element is one
                                       accumulation in k order whatever the tile count
                                       (see "Few tiles, long K" at gemm_bf16) */
-#define PTXB200_GEMM_ONE_CTA 0x4u  /* always the one-CTA-per-tile kernel, never the CTA-pair one */
+#define PTXB200_GEMM_ONE_CTA 0x4u  /* always one CTA per tile (or per part of K), never a CTA pair */
 
 /* fa_fwd_bf16 flags */
 #define PTXB200_FA_NO_LAZY_RESCALE 0x1u /* rescale O on every row-max increase (no 2^8 slack) */
@@ -81,17 +81,14 @@ const char* ptxb200_last_cuda_error(void);
  * Shape contract: M % 128 == 0, N % 128 == 0, K % 64 == 0, all > 0;
  * ldc * sizeof(element) % 16 == 0.
  *
- * Few tiles, long K: when the 128x256 output tiles number at most half the SMs and
- * K is long enough, every tile is cut along K and shared by at least twice as many
- * SMs; the partial sums meet in fp32 scratch that the library keeps per (device,
- * stream) -- 256 KiB per CTA of the launch, at most 38 MB, allocated (cudaMalloc) by
- * the first launch on a stream that needs it, so make that launch outside stream
- * capture or pass PTXB200_GEMM_NO_SPLIT; at most 16 such buffers exist per process (the
- * least recently used one is waited for and freed when a 17th stream asks), all freed
- * by ptxb200_shutdown -- and a second small kernel on the same stream adds them up.
- * Results stay reproducible from launch to launch; they differ in the last bits from
- * the unsplit summation order, which PTXB200_GEMM_NO_SPLIT keeps. No reference
- * counterpart (test/gpu/blackwell/gemm_highperf_blackwell.jl:27-32 leaves it).
+ * Few tiles, long K: products whose 128x128 output tiles number at most the SMs run
+ * on smaller tiles, and with K long enough every tile is shared by the two or four
+ * CTAs of a cluster, each summing a part of K; the parts meet in the CTAs' shared
+ * memory (no scratch, no second kernel), and with fp32 output a CTA also sums its part
+ * in several shorter chains. Results stay reproducible from launch to launch; they
+ * differ in the last bits from the unsplit summation order, which
+ * PTXB200_GEMM_NO_SPLIT keeps. No reference counterpart
+ * (test/gpu/blackwell/gemm_highperf_blackwell.jl:27-32 leaves it).
  *
  * Replaces the reference's _run_ghb launch of _ghb_gemm_kernel! /
  * _ghb_persistent_kernel! (test/gpu/blackwell/gemm_highperf_blackwell.jl:69-199,

@@ -1,4 +1,4 @@
-// gemm_bf16 on CTA pairs: one 256x256 output tile per pair of SMs, issued as
+// gemm_bf16 on CTA pairs: one output tile of 256 rows and 128, 192 or 256 columns per pair of SMs, issued as
 // tcgen05.mma.cta_group::2.
 //
 // Why a second GEMM kernel. The single-CTA kernel (gemm_sm100.cu) streams 48 KiB
@@ -27,6 +27,7 @@
 // cluster barrier before the first remote arrival and before exit.
 //
 // Work per launch: 2*G*M*N*K flop; compulsory bytes G*((M*K + N*K)*2 + M*N*sizeof(out)).
+#include "cta_pair.cuh"
 #include "gemm_epilogue.cuh"
 #include "host_common.h"
 #include "sm100_prims.cuh"
@@ -35,87 +36,28 @@ namespace ptxb200 {
 namespace {
 
 constexpr int kBM2 = 256;                      // rows of the pair's tile (128 per CTA)
-constexpr int kBN2 = 256;                      // columns of the pair's tile
 constexpr int kBK2 = 64;
-constexpr int kStages2 = 6;
 constexpr int kAStage2 = 128 * kBK2 * 2;       // this CTA's 128 rows of A: 16 KiB
-constexpr int kBStage2 = 128 * kBK2 * 2;       // this CTA's 128 rows of B^T: 16 KiB
-constexpr int kStage2 = kAStage2 + kBStage2;
 constexpr int kThreads2 = 192;
-constexpr int kAccCols2 = 256;
-#ifndef PTXB200_GEMM2_GROUP_M
-#define PTXB200_GEMM2_GROUP_M 8
-#endif
-constexpr int kGroupM2 = PTXB200_GEMM2_GROUP_M;   // row-tiles (of 256) per rasterisation band
+constexpr int kAccCols2 = 256;                 // distance of the two accumulators in tensor memory
+constexpr int kGroupM2 = 8;                    // row-tiles (of 256) per rasterisation band
 
-constexpr int kOffA2 = 0;
-constexpr int kOffB2 = kOffA2 + kStages2 * kAStage2;
-constexpr int kOffBars2 = kOffB2 + kStages2 * kBStage2;   // full[6] empty[6] acc_full[2] acc_empty[2]
-constexpr int kOffTmemSlot2 = kOffBars2 + (2 * kStages2 + 4) * 8;
-constexpr int kOffAbort2 = kOffTmemSlot2 + 8;
-constexpr int kSmemBytes2 = kOffAbort2 + 8;    // the base must be 1024-byte aligned (checked)
+// kBN columns of the pair's tile: 128, 192 or 256
+template <int kBN>
+struct Cfg2 {
+  static constexpr int kBStage = kBN / 2 * kBK2 * 2;   // this CTA's half of the rows of B^T
+  static constexpr int kStage = kAStage2 + kBStage;
+  static constexpr int kStages = kBN == 256 ? 6 : kBN == 192 ? 8 : 9;
+  static constexpr int kOffA = 0;
+  static constexpr int kOffB = kOffA + kStages * kAStage2;
+  static constexpr int kOffBars = kOffB + kStages * kBStage;   // full[] empty[] acc_full[2] acc_empty[2]
+  static constexpr int kOffTmemSlot = kOffBars + (2 * kStages + 4) * 8;
+  static constexpr int kOffAbort = kOffTmemSlot + 8;
+  static constexpr int kSmemBytes = kOffAbort + 8;      // the base must be 1024-byte aligned (checked)
+  static_assert(kSmemBytes <= 232448, "exceeds the 227 KiB a CTA can opt in to");
+};
 
 enum : uint32_t { kSite2Empty = 18, kSite2Full = 19, kSite2AccEmpty = 20, kSite2AccFull = 21 };
-
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// Address of `smem_addr` (an address in this CTA's shared memory) in CTA `rank` of the cluster.
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx_cluster(uint32_t cluster_addr, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cluster.b64 _, [%0], %1;" ::"r"(cluster_addr), "r"(bytes)
-               : "memory");
-}
-// TMA tile load into this CTA's shared memory whose bytes are counted on a barrier
-// that may be the pair leader's (`cluster_bar`).
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst_smem, const void* tmap, int c0, int c1,
-                                                 uint32_t cluster_bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%2, %3}], [%4];" ::"r"(dst_smem),
-      "l"((uint64_t)tmap), "r"(c0), "r"(c1), "r"(cluster_bar)
-      : "memory");
-}
-__device__ __forceinline__ void tmem_alloc_pair(uint32_t slot_smem, uint32_t ncols) {
-  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot_smem), "r"(ncols)
-               : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish_pair() {
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
-  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-// Converged warp, elected lane: D[tmem of both CTAs] (+)= A * B over the pair.
-__device__ __forceinline__ void tc_mma_ss_pair(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo,
-                                               uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
-      "mov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"
-      "setp.ne.b32 p, %6, 0;\n\telect.sync _|q, 0xffffffff;\n\t"
-      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %5, p;\n\t}" ::"r"(d_tmem),
-      "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// One arrival on `cluster_bar` (any CTA of the pair) once every MMA issued so far is done.
-__device__ __forceinline__ void tc_commit_pair(uint32_t cluster_bar) {
-  asm volatile(
-      "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
-      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(cluster_bar)
-      : "memory");
-}
 
 __device__ __forceinline__ void tile_coords2(int tile, int tiles_m, int tiles_n, int& tm, int& tn) {
   const int band_tiles = kGroupM2 * tiles_n;
@@ -127,24 +69,26 @@ __device__ __forceinline__ void tile_coords2(int tile, int tiles_m, int tiles_n,
   tn = r / rows_in_band;
 }
 
-template <bool kF32Out>
+template <int kBN, bool kF32Out>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads2, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                  void* __restrict__ c_out, int M, int N, int K, int ldc, int groups, uint32_t* status) {
+  using C = Cfg2<kBN>;
+  constexpr int kStages2 = C::kStages;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw;
   const uint32_t base = smem_u32(smem_raw);
   const uint32_t rank = cluster_ctarank();        // 0: the pair's leader
   const bool leader = rank == 0;
 
-  const uint32_t a_base = base + kOffA2;
-  const uint32_t b_base = base + kOffB2;
-  const uint32_t bar_full = base + kOffBars2;
+  const uint32_t a_base = base + C::kOffA;
+  const uint32_t b_base = base + C::kOffB;
+  const uint32_t bar_full = base + C::kOffBars;
   const uint32_t bar_empty = bar_full + kStages2 * 8;
   const uint32_t bar_acc_full = bar_empty + kStages2 * 8;
   const uint32_t bar_acc_empty = bar_acc_full + 2 * 8;
-  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + kOffTmemSlot2);
-  volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(smem + kOffAbort2);
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + C::kOffTmemSlot);
+  volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(smem + C::kOffAbort);
   const WaitCtx wctx{status, abort_flag};
 
   const int warp = threadIdx.x >> 5;
@@ -176,7 +120,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   const uint32_t tmem = *tmem_slot;
 
   const int tiles_m = (M + kBM2 - 1) / kBM2;   // M % 128 == 0: the last row-tile may be its first half only
-  const int tiles_n = (N + kBN2 - 1) / kBN2;
+  const int tiles_n = (N + kBN - 1) / kBN;
   const int tiles_per_group = tiles_m * tiles_n;
   const int total_tiles = tiles_per_group * groups;
   const int kiters = K / kBK2;
@@ -197,21 +141,21 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         const int g = tile / tiles_per_group;
         tile_coords2(tile - g * tiles_per_group, tiles_m, tiles_n, tm, tn);
         const int a_row = g * M + tm * kBM2 + (int)rank * 128;
-        const int b_row = g * N + tn * kBN2 + (int)rank * 128;
+        const int b_row = g * N + tn * kBN + (int)rank * (kBN / 2);
         for (int k = 0; k < kiters; ++k, ++it) {
           const uint32_t s = it % kStages2;
           const uint32_t ph = (it / kStages2) & 1u;
           mbar_wait(bar_empty + 8 * s, ph ^ 1u, wctx, kSite2Empty);
-          mbar_arrive_expect_tx_cluster(leader_full + 8 * s, kStage2);
+          mbar_arrive_expect_tx_cluster(leader_full + 8 * s, C::kStage);
           tma_load_2d_pair(a_base + s * kAStage2, &tmap_a, k * kBK2, a_row, leader_full + 8 * s);
-          tma_load_2d_pair(b_base + s * kBStage2, &tmap_b, k * kBK2, b_row, leader_full + 8 * s);
+          tma_load_2d_pair(b_base + s * C::kBStage, &tmap_b, k * kBK2, b_row, leader_full + 8 * s);
         }
       }
     }
   } else if (warp == 1) {
     // ---------------- MMA issue (leader only; converged warp, elected lane) ----------------
     if (leader) {
-      constexpr uint32_t idesc = make_idesc_bf16_f32(kBM2, kBN2, false, false);
+      constexpr uint32_t idesc = make_idesc_bf16_f32(kBM2, kBN, false, false);
       const uint32_t peer_empty = map_to_cta(bar_empty, 1);
       const uint32_t peer_acc_full = map_to_cta(bar_acc_full, 1);
       uint32_t it = 0, t = 0;
@@ -227,7 +171,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           mbar_wait_warp(bar_full + 8 * s, ph, wctx, kSite2Full);
           tc_fence_after();
           const uint32_t da = sdesc_lo(a_base + s * kAStage2, 16);
-          const uint32_t db = sdesc_lo(b_base + s * kBStage2, 16);
+          const uint32_t db = sdesc_lo(b_base + s * C::kBStage, 16);
           constexpr uint32_t dhi = sdesc_hi(1024, kLayoutB128);
 #pragma unroll
           for (int kk = 0; kk < kBK2 / 16; ++kk)
@@ -257,10 +201,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       // in a half-filled last row-tile the peer's 128 rows lie past M (its A box read the
       // next group's rows or zero fill): computed, not stored
       const bool rows_valid = tm * kBM2 + (int)rank * 128 < M;
-      const int col0 = tn * kBN2;
+      const int col0 = tn * kBN;
       const uint32_t t_row = tmem_addr(tmem, quad * 32, buf * kAccCols2);
 #pragma unroll 1
-      for (int c = 0; c < kBN2 / 32; ++c) {
+      for (int c = 0; c < kBN / 32; ++c) {
         uint32_t v[32];
         tmem_ld32(t_row + c * 32, v);
         tc_wait_ld_bind(v);
@@ -285,41 +229,77 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 
 }  // namespace
 
-bool gemm_pair_eligible(const DeviceCtx& ctx, int groups, int M, int N, int K) {
-  (void)K;
-  // worth it once every pair of SMs has a tile (M % 128 == 0 is the entry points' contract;
-  // a last row-tile may be half-filled)
-  const long long tiles = (long long)groups * ((M + kBM2 - 1) / kBM2) * ((N + kBN2 - 1) / kBN2);
-  return tiles >= ctx.sm_count / 2;
+// Columns of the pair's tile for a product, or 0 where 128x256 tiles of single CTAs
+// (gemm_sm100.cu) are the better choice. The estimate, in us: rounds over the machine times
+// what a tile costs, which is its steps of K (0.345, 0.27, 0.215 us for 256, 192, 128 columns;
+// single CTAs 0.36) or, for short K, its epilogue (0.013 us per column), plus one epilogue.
+// Wide tiles cost least per column; narrower ones are taken where they fill the last round
+// better: 2304x2304x1024 19.0 us with 256 columns, 15.6 with 192; 1792x1792x8192 45.8 and
+// 40.6; 3072x5120x8192 194 and 184; 8192^3 694 and 722. Single CTAs win where M leaves half
+// of a pair's last row-tile empty (32 products of 128x2048x2048: 63.0 us in pairs, 53.9
+// single). Any width gives the same bits: an element is one accumulation in k order.
+int gemm_pair_tile(const DeviceCtx& ctx, int groups, int M, int N, int K) {
+  const double kiters = K / kBK2;
+  auto cost = [&](long long tiles, long long at_once, double step, int bn) {
+    const double epilogue = 0.013 * bn, tile = kiters * step > epilogue ? kiters * step : epilogue;
+    return (double)((tiles + at_once - 1) / at_once) * tile + epilogue;
+  };
+  const int pairs = ctx.sm_count / 2;
+  const long long row_tiles = (long long)groups * ((M + kBM2 - 1) / kBM2);   // a last row-tile may be half-filled
+  int best = 0;
+  double least = cost((long long)groups * (M / 128) * ((N + 255) / 256), ctx.sm_count, 0.36, 256) + 1.0;
+  const int bns[3] = {256, 192, 128};
+  const double steps[3] = {0.345, 0.27, 0.215};
+  for (int i = 0; i < 3; ++i) {
+    const double c = cost(row_tiles * ((N + bns[i] - 1) / bns[i]), pairs, steps[i], bns[i]);
+    if (c < least) {
+      least = c;
+      best = bns[i];
+    }
+  }
+  return best;
 }
 
-int launch_gemm_pair(const DeviceCtx& ctx, void* C, const void* A, const void* Bt, int groups, int M, int N,
-                     int K, int ldc, unsigned flags, cudaStream_t stream) {
+namespace {
+
+template <int kBN, bool kF32Out>
+int launch_one2(const DeviceCtx& ctx, void* C, const void* A, const void* Bt, int groups, int M, int N, int K, int ldc,
+                cudaStream_t stream) {
   CUtensorMap ta, tb;
   int rc = encode_tmap_bf16_2d(&ta, A, (uint64_t)groups * M, (uint64_t)K, (uint64_t)K * 2, 128, kBK2);
   if (rc != PTXB200_OK) return rc;
-  rc = encode_tmap_bf16_2d(&tb, Bt, (uint64_t)groups * N, (uint64_t)K, (uint64_t)K * 2, 128, kBK2);
+  rc = encode_tmap_bf16_2d(&tb, Bt, (uint64_t)groups * N, (uint64_t)K, (uint64_t)K * 2, kBN / 2, kBK2);
   if (rc != PTXB200_OK) return rc;
-  const long long tiles = (long long)groups * ((M + kBM2 - 1) / kBM2) * ((N + kBN2 - 1) / kBN2);
-  const int max_pairs = ctx.sm_count / 2;
-  const int pairs = tiles < max_pairs ? (int)tiles : max_pairs;
-  uint32_t* status = status_word(ctx, stream);
-  const int f32 = (flags & PTXB200_GEMM_F32_OUT) ? 1 : 0;
   static PerDeviceOnce attr_once;
   rc = attr_once.run(ctx.device, []() -> int {
-    PTXB200_CUDA_TRY(cudaFuncSetAttribute(gemm_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          kSmemBytes2));
-    PTXB200_CUDA_TRY(cudaFuncSetAttribute(gemm_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          kSmemBytes2));
+    PTXB200_CUDA_TRY(cudaFuncSetAttribute(gemm_pair_kernel<kBN, kF32Out>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          Cfg2<kBN>::kSmemBytes));
     return PTXB200_OK;
   });
   if (rc != PTXB200_OK) return rc;
-  if (f32)
-    gemm_pair_kernel<true><<<2 * pairs, kThreads2, kSmemBytes2, stream>>>(ta, tb, C, M, N, K, ldc, groups, status);
-  else
-    gemm_pair_kernel<false><<<2 * pairs, kThreads2, kSmemBytes2, stream>>>(ta, tb, C, M, N, K, ldc, groups, status);
+  const long long tiles = (long long)groups * ((M + kBM2 - 1) / kBM2) * ((N + kBN - 1) / kBN);
+  const int max_pairs = ctx.sm_count / 2;
+  const int pairs = tiles < max_pairs ? (int)tiles : max_pairs;
+  gemm_pair_kernel<kBN, kF32Out><<<2 * pairs, kThreads2, Cfg2<kBN>::kSmemBytes, stream>>>(
+      ta, tb, C, M, N, K, ldc, groups, status_word(ctx, stream));
   PTXB200_CUDA_TRY(cudaGetLastError());
   return PTXB200_OK;
+}
+
+}  // namespace
+
+int launch_gemm_pair(const DeviceCtx& ctx, int bn, void* C, const void* A, const void* Bt, int groups, int M, int N,
+                     int K, int ldc, unsigned flags, cudaStream_t stream) {
+  const bool f32 = (flags & PTXB200_GEMM_F32_OUT) != 0;
+#define PTXB200_PAIR_TILE(BN)                                                                           \
+  if (bn == BN)                                                                                         \
+    return f32 ? launch_one2<BN, true>(ctx, C, A, Bt, groups, M, N, K, ldc, stream)                     \
+               : launch_one2<BN, false>(ctx, C, A, Bt, groups, M, N, K, ldc, stream)
+  PTXB200_PAIR_TILE(128);
+  PTXB200_PAIR_TILE(192);
+  PTXB200_PAIR_TILE(256);
+#undef PTXB200_PAIR_TILE
+  return PTXB200_E_INVALID;
 }
 
 }  // namespace ptxb200

@@ -27,4 +27,23 @@ __device__ __forceinline__ void store_acc_chunk(void* __restrict__ c_out, size_t
   }
 }
 
+// The same for 16 consecutive columns.
+template <bool kF32Out>
+__device__ __forceinline__ void store_acc_chunk16(void* __restrict__ c_out, size_t row, int ldc, int col,
+                                                  const float (&v)[16]) {
+  if (kF32Out) {
+    float* dst = reinterpret_cast<float*>(c_out) + row * (size_t)ldc + col;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      st_global_v4(dst + 4 * i, __float_as_uint(v[4 * i]), __float_as_uint(v[4 * i + 1]), __float_as_uint(v[4 * i + 2]),
+                   __float_as_uint(v[4 * i + 3]));
+  } else {
+    __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(c_out) + row * (size_t)ldc + col;
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      st_global_v4(dst + 8 * i, pack_bf16x2(v[8 * i], v[8 * i + 1]), pack_bf16x2(v[8 * i + 2], v[8 * i + 3]),
+                   pack_bf16x2(v[8 * i + 4], v[8 * i + 5]), pack_bf16x2(v[8 * i + 6], v[8 * i + 7]));
+  }
+}
+
 }  // namespace ptxb200

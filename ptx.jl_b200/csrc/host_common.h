@@ -72,7 +72,7 @@ class PerDeviceOnce {
 //  * At most kScratchMaxEntries buffers exist per process: when a new (device, stream,
 //    kind) needs one and the table is full, the least recently used entry is waited for
 //    (its event) and freed. Everything is freed by ptxb200_shutdown.
-enum : int { kScratchGemmSlabs = 0, kScratchAttnParts = 1 };
+enum : int { kScratchAttnParts = 1 };
 constexpr int kScratchMaxEntries = 16;
 struct ScratchLease {
   void* ptr = nullptr;
@@ -117,6 +117,11 @@ int encode_tmap_bf16_3d(CUtensorMap* out, const void* base, uint64_t slices, uin
     }                                                  \
   } while (0)
 
+struct GemmSplitPlan {
+  int bn;         // columns of a tile (128 rows): 64 or 128
+  int split;      // parts of K, one CTA of a cluster each: 1, 2 or 4
+};
+
 // Kernel launchers (one per .cu file).
 int launch_gemm(const DeviceCtx& ctx, void* C, const void* A, const void* Bt, int groups, int M, int N,
                 int K, int ldc, unsigned flags, cudaStream_t stream);
@@ -125,10 +130,16 @@ int launch_fa_fwd(const DeviceCtx& ctx, void* O, void* lse, const void* Q, const
                   unsigned flags, void* dbg, uint32_t* status, cudaStream_t stream);
 // The work distribution launch_fa_fwd would pick, as plain ints (fa_fwd_sm100.cu).
 int describe_fa_plan(int BH, int S, int causal, unsigned flags, int sm_count, int* out, int cap);
-// CTA-pair GEMM (gemm2_sm100.cu): whether it applies to a shape, and its launcher.
-bool gemm_pair_eligible(const DeviceCtx& ctx, int groups, int M, int N, int K);
-int launch_gemm_pair(const DeviceCtx& ctx, void* C, const void* A, const void* Bt, int groups, int M, int N,
+// CTA-pair GEMM (gemm2_sm100.cu): the tile width it would run a product with (0: not at
+// all), and its launcher.
+int gemm_pair_tile(const DeviceCtx& ctx, int groups, int M, int N, int K);
+int launch_gemm_pair(const DeviceCtx& ctx, int bn, void* C, const void* A, const void* Bt, int groups, int M, int N,
                      int K, int ldc, unsigned flags, cudaStream_t stream);
+// Small-tile GEMM with K split inside clusters (gemm_split_sm100.cu): false when another
+// kernel is the better choice.
+bool gemm_split_choose(const DeviceCtx& ctx, int groups, int M, int N, int K, unsigned flags, GemmSplitPlan* plan);
+int launch_gemm_split(const DeviceCtx& ctx, const GemmSplitPlan& plan, void* C, const void* A, const void* Bt, int groups,
+                      int M, int N, int K, int ldc, unsigned flags, cudaStream_t stream);
 // Row-wise fp32 kernels; op: 0 softmax, 1 RMS norm, 2 layer norm.
 int launch_rowwise(const DeviceCtx& ctx, int op, float* y, const float* x, const float* w,
                    const float* bias, int rows, int n, float eps, cudaStream_t stream);

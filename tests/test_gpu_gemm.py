@@ -242,6 +242,65 @@ def test_grouped_gemm_pair_kernel(pkg, gpu):
     torch.testing.assert_close(c_pair, torch.bmm(a.float(), bt.float().transpose(1, 2)), rtol=1e-4, atol=1e-3)
 
 
+# ---------------------------------------------------------------------------
+# Small tiles with K split in clusters, and the three tile widths of the CTA-pair kernel,
+# each at the sizes where its rule or its remainders change (148 SMs).
+# ---------------------------------------------------------------------------
+@pytest.mark.parametrize("G,M,N,K", [
+    (1, 128, 64, 64),       # one step of K: half a ring stage
+    (3, 128, 192, 192),     # one and a half stages, odd number of 64-column tiles
+    (1, 128, 128, 1024),    # split in 4, parts of 4 steps
+    (1, 128, 128, 1088),    # parts of 4, 4, 4 and 5 steps
+    (1, 128, 64, 8192),     # parts of 32 steps: four chains each with fp32 output
+    (2, 128, 64, 8128),     # parts of 31 and 32 steps
+    (1, 128, 64 * 37, 1024),    # 37 tiles of 64: the last split in 4
+    (1, 128, 64 * 38, 1024),    # 38: the first split in 2
+    (1, 128, 64 * 75, 1088),    # 75: not split
+    (1, 128, 64 * 74, 1984),    # 74: split in 2, parts of 15 and 16 steps
+    (1, 1024, 1152, 4096),      # 128 columns, split in 2
+    (3, 1024, 576, 4160),       # a half-empty last tile and an odd number of steps
+    (1, 512, 64 * 37, 512),     # 148 tiles of 64
+    (4, 256, 64 * 19, 512),     # 152 of 64: 128 columns, the last tile half-empty
+    (1, 512, 128 * 37, 576),    # 148 tiles of 128
+    (1, 512, 128 * 38, 192),    # 152: the persistent kernels
+    (1, 2304, 2304, 1024),      # pair tiles of 192 columns
+    (1, 2432, 2368, 832),       # the same, half-filled row-tile, 64 columns over
+    (5, 1024, 512, 512),        # the same, groups
+    (8, 640, 704, 832),         # pair tiles of 128 columns, half-filled row-tiles, 64 columns over
+    (1, 2048, 3008, 448),       # the same, one product
+    (40, 128, 320, 128),        # M of one half row-tile per group
+])
+@pytest.mark.parametrize("f32_out", [True, False])
+def test_gemm_tile_rules_against_64_bit(pkg, gpu, G, M, N, K, f32_out):
+    g = torch.Generator(device=gpu).manual_seed(G * M + N + K)
+    a = torch.randn(G, M, K, generator=g, device=gpu).to(torch.bfloat16)
+    bt = torch.randn(G, N, K, generator=g, device=gpu).to(torch.bfloat16)
+    dtype = torch.float32 if f32_out else torch.bfloat16
+    ldc = N + 16
+    buf = torch.full((2, G * M, ldc), 7.0, dtype=dtype, device=gpu)
+    flags = pkg.native.GEMM_F32_OUT if f32_out else 0
+    for i in range(2):
+        rc = pkg.native.lib().gemm_bf16_grouped(buf[i].data_ptr(), a.data_ptr(), bt.data_ptr(), G, M, N, K, ldc, flags,
+                                                torch.cuda.current_stream().cuda_stream)
+        assert rc == 0
+    status = pkg.ops.sync_status()
+    assert status == 0, pkg.native.strerror(status)
+    assert torch.equal(buf[0], buf[1])                  # the order of the sums is fixed
+    assert torch.all(buf[:, :, N:] == 7.0)              # nothing past a row's N columns
+    got = buf[0, :, :N].reshape(G, M, N).double()
+    ad, bd = a.double(), bt.double().mT
+    ref, size = ad @ bd, ad.abs() @ bd.abs()
+    # fp32 sums of K products in any order: K roundings of at most the sum of magnitudes;
+    # bf16 out: one more rounding of the result
+    bound = K * 2.0 ** -24 * size + (0.0 if f32_out else 2.0 ** -8) * ref.abs()
+    assert bool(((got - ref).abs() <= bound).all())
+    # whatever the tile, an unsplit element is one accumulation in k order
+    whole = pkg.ops.gemm_grouped(a, bt, f32_out=True, no_split=True)
+    plain = pkg.ops.gemm_grouped(a, bt, f32_out=True, no_split=True, one_cta=True)
+    assert torch.equal(whole, plain)
+    assert pkg.ops.sync_status() == 0
+
+
 def _random_gemm_shapes(n, seed):
     rng = np.random.default_rng(seed)
     out = []
