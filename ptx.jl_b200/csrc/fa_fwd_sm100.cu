@@ -475,7 +475,7 @@ __device__ __forceinline__ void fa_mma_role(const FaParams& p, uint32_t base, ui
   // allow for it are the per-stage q_free and the l_free barrier. At head dim 64, where
   // the MUFU rather than the issue order bounds a tile, this measured slower on causal
   // problems, so there each item starts behind the previous one's last P V.
-  constexpr bool kStream = (D == 128);
+    constexpr bool kStream = (D == 128);
   WorkIter<kCausal, kTail> items;
   WorkItem w, w2;
   int nt[2] = {0, 0};
@@ -535,6 +535,48 @@ __device__ __forceinline__ void fa_mma_role(const FaParams& p, uint32_t base, ui
     p.dbg[1] = kv_count;
     p.dbg[2] = cnt_pv[0];
     p.dbg[3] = cnt_pv[1];
+  }
+}
+
+// One correction warp's 32 rows of a finished O_s: scaled by each row's 1 / l, rounded to
+// bf16 and written. `o_tmem` is the warp's first lane at O_s's first column, `dst` the row of
+// that lane, `rows` how many of the rows exist, `inv_l` this lane's row's factor. `release` is
+// called behind the last read of O_s.
+//
+// The loads are 16 lanes x 64 columns, whose fragments a transpose within each quad of lanes
+// turns into 16-byte pieces, 64 consecutive bytes of a row per quad: a store instruction
+// touches 8 rows. With a row per lane it touched 32, and the epilogue of a stage took 3000
+// cycles, of which 2200-2900 held up the next item's first P V.
+template <int D, class Release>
+__device__ __forceinline__ void store_rows(uint32_t o_tmem, __nv_bfloat16* dst, int rows, float inv_l, Release&& release) {
+  const int lane = threadIdx.x & 31, quad = lane >> 2, col = (lane & 3) * 8;
+#pragma unroll 1
+  for (int h = 0; h < 2; ++h) {          // the warp's first and second 16 rows
+    const float f0 = __shfl_sync(0xffffffffu, inv_l, h * 16 + quad);
+    const float f1 = __shfl_sync(0xffffffffu, inv_l, h * 16 + 8 + quad);
+    const int r0 = h * 16 + quad;
+    __nv_bfloat16* const row0 = dst + (size_t)r0 * D + col;
+#pragma unroll 1
+    for (int c = 0; c < D; c += 64) {
+      uint32_t o[32];
+      tmem_ld_16x64(o_tmem + ((uint32_t)(h * 16) << 16) + c, o);
+      tc_wait_ld_bind(o);
+      if (h == 1 && c + 64 == D) release();
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {      // 32 columns at a time
+        uint32_t a[4], b[4];             // rows r0 and r0 + 8
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int k = 4 * (4 * m + i);
+          a[i] = pack_bf16x2(__uint_as_float(o[k]) * f0, __uint_as_float(o[k + 1]) * f0);
+          b[i] = pack_bf16x2(__uint_as_float(o[k + 2]) * f1, __uint_as_float(o[k + 3]) * f1);
+        }
+        quad_transpose(a[0], a[1], a[2], a[3]);
+        quad_transpose(b[0], b[1], b[2], b[3]);
+        if (r0 < rows) st_global_v4(row0 + c + 32 * m, a[0], a[1], a[2], a[3]);
+        if (r0 + 8 < rows) st_global_v4(row0 + 8 * D + c + 32 * m, b[0], b[1], b[2], b[3]);
+      }
+    }
   }
 }
 
@@ -921,8 +963,34 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
           }
         }
       }
-      if constexpr (!kTail) {
+      if constexpr (!kTail && D == 128) {
         // ---- epilogue: O / l -> bf16 -> global ----
+        const int q_row0 = bh * p.seqlen + mb * 2 * kAttnRows;
+  #pragma unroll 1
+        for (int s = 0; s < 2; ++s) {
+          const float l_mine = s == 0 ? l_part[0] : l_part[1], neg = s == 0 ? neg_prev[0] : neg_prev[1];
+          // rows past the end of the sequence were computed on zero-filled queries: not written
+          const bool row_valid = mb * 2 * kAttnRows + s * kAttnRows + row < p.seqlen;
+          mbar_wait(bar(C::kBarODone + s), item_i & 1u, wctx, kSiteCorrODone);
+          mbar_wait(bar(C::kBarLReady + s), item_i & 1u, wctx, kSiteCorrLReady);
+          tc_fence_after();
+          const float l_total = stats_l[s * 128 + row] + l_mine;
+          mbar_arrive(bar(C::kBarLFree + s));   // the softmax warps may publish the next item's sum
+          const float inv_l = 1.0f / l_total;
+          if (p.lse != nullptr && row_valid) {
+            // sum_j 2^(s_j c) = 2^(m c) * l with basis -m c in neg_prev: natural log of it
+            p.lse[q_row0 + s * kAttnRows + row] = (log2f(l_total) - neg) * 0.6931471805599453f;
+          }
+          const int warp_row = s * kAttnRows + (row & ~31);   // this warp's first row of the item
+          store_rows<D>(t_lane + C::kColO + s * D, p.o + (size_t)(q_row0 + warp_row) * D,
+                        p.seqlen - mb * 2 * kAttnRows - warp_row, inv_l, [&] {
+                          // last read of O_s: the next item may overwrite it
+                          tc_fence_before();
+                          mbar_arrive(bar(C::kBarPFull + 2 * s));
+                        });
+        }
+      } else if constexpr (!kTail) {
+        // ---- the same at head dim 64, a row per lane (store_rows: 2-3 % slower at every length) ----
         const int q_row0 = bh * p.seqlen + mb * 2 * kAttnRows;
   #pragma unroll
         for (int s = 0; s < 2; ++s) {

@@ -424,6 +424,33 @@ __device__ __forceinline__ void tc_wait_ld_bind16(uint32_t (&r)[16]) {
                : "memory");
 }
 
+// 16 lanes (from the one in `taddr`: the warp's first or its 17th) x 64 columns: registers
+// 4 i + {0, 1} of thread t hold row t / 4, columns 8 i + 2 (t % 4) + {0, 1}; registers
+// 4 i + {2, 3} the same columns of row t / 4 + 8.
+__device__ __forceinline__ void tmem_ld_16x64(uint32_t taddr, uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x8.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
+        "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]),
+        "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr)
+      : "memory");
+}
+// Transposes the 4 x 4 words held by each quad of lanes: word j of lane i goes to word i of
+// lane j (i, j within the quad).
+__device__ __forceinline__ void quad_transpose(uint32_t& w0, uint32_t& w1, uint32_t& w2, uint32_t& w3) {
+  const bool odd = (threadIdx.x & 1) != 0, high = (threadIdx.x & 2) != 0;
+  uint32_t a = __shfl_xor_sync(0xffffffffu, odd ? w0 : w1, 1), b = __shfl_xor_sync(0xffffffffu, odd ? w2 : w3, 1);
+  if (odd) { w0 = a; w2 = b; } else { w1 = a; w3 = b; }
+  a = __shfl_xor_sync(0xffffffffu, high ? w0 : w2, 2);
+  b = __shfl_xor_sync(0xffffffffu, high ? w1 : w3, 2);
+  if (high) { w0 = a; w1 = b; } else { w2 = a; w3 = b; }
+}
+
 // ---------------------------------------------------------------------------
 // Numerics
 // ---------------------------------------------------------------------------
