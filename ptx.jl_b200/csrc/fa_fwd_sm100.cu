@@ -254,7 +254,6 @@ struct ItemIter {
   // true while the item just returned by next() is this CTA's first
   __device__ __forceinline__ bool on_first() const { return v == 1; }
 };
-template <bool V> struct BoolTag { static constexpr bool value = V; };
 
 // Key tiles each stage of the item visits.
 template <bool kCausal>
@@ -740,23 +739,20 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
         for (int c = 0; c < 4; ++c) tc_wait_ld_bind(v[c]);
         FA_TSTAMP(stamp, stage, j, 2);
 
-        if (kCausal && j == jlast) {
-          // diagonal tile: key (local) column i is kept iff i <= row (keys past the end of
-          // the sequence lie beyond every valid row's diagonal)
+        // The stage's last tile: key (local) column i is kept iff i <= keep. Causal: the
+        // diagonal (keys past the end of the sequence lie beyond every valid row's diagonal);
+        // otherwise the last tile of a sequence that is not a multiple of 128, whose keys past
+        // the end loaded as zeros and must not count.
+        if ((kCausal && j == jlast) || (kRagged && !kCausal && j == jlast && kv_tail < kAttnRows)) {
+          const int keep = kCausal ? row : kv_tail - 1;
 #pragma unroll
-          for (int c = 0; c < 4; ++c)
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (c * 32 + i > row) v[c][i] = 0xFF800000u;  // -inf
-        }
-        if (kRagged && !kCausal && j == jlast && kv_tail < kAttnRows) {
-          // last tile of a sequence that is not a multiple of 128: its keys past the end
-          // loaded as zeros and must not count
-#pragma unroll
-          for (int c = 0; c < 4; ++c)
+          for (int c = 0; c < 4; ++c) {
+            const int n = keep + 1 - c * 32;   // kept columns of this chunk: its low n bits
+            const uint32_t bits = n >= 32 ? 0xFFFFFFFFu : n <= 0 ? 0u : (1u << n) - 1u;
 #pragma unroll
             for (int i = 0; i < 32; ++i)
-              if (c * 32 + i >= kv_tail) v[c][i] = 0xFF800000u;  // -inf
+              if (!((bits >> i) & 1u)) v[c][i] = 0xFF800000u;  // -inf
+          }
         }
 
         float mx[4];
@@ -859,6 +855,12 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
     const uint32_t t_lane = tmem_addr(tmem, (warp & 3) * 32, 0);
     mbar_arrive(bar(C::kBarPFull + 0));   // O is free for the first item
     mbar_arrive(bar(C::kBarPFull + 2));
+    // The loop over a tile's two stages stays rolled where the kernel carries masking code:
+    // three roles' loops share the SM's instruction cache, and unrolled this one did not fit
+    // beside the others (causal, head dim 128: 8 x 32 heads of 2048 keys 313 us unrolled, 284
+    // rolled; ragged 300 keys 126 and 117; without masking code unrolled is 1-5 % faster).
+    // Rolled, the state of the current stage is element 0 and the two change places.
+    constexpr int kStageUnroll = (kCausal || kRagged) ? 1 : 2;
     uint32_t cnt_a[2] = {0, 0};
     uint32_t cnt_h[2] = {0, 0};   // S tiles seen per stage
     uint32_t item_i = 0;
@@ -871,34 +873,35 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
       float neg_prev[2] = {0.0f, 0.0f};
 #pragma unroll 1
       for (int j = 0; j < nt_max; ++j) {
-#pragma unroll
+#pragma unroll(kStageUnroll)
         for (int s = 0; s < 2; ++s) {
-          if (j < nt[s]) {
+          const int cur = kStageUnroll == 1 ? 0 : s;
+          if (j < (s == 0 ? nt[0] : nt[1])) {
             uint32_t sv[32];
             [[maybe_unused]] uint32_t sw[16];   // head dim 64: key columns 80..95 as well
             // Only a stage's last tile can hold masked keys: those above the diagonal
             // (causal) or past the end of the sequence (non-causal, S % 128 != 0). `keep`
             // is the last key column this row keeps there.
             const int j_abs = kTail ? w.j0 + j : j;   // the tile's index within the head's sequence
-            const bool mask_tile = j == (kTail ? w.jlast[s] : nt[s] - 1) &&
+            const bool mask_tile = j == (s == 0 ? (kTail ? w.jlast[0] : nt[0] - 1) : (kTail ? w.jlast[1] : nt[1] - 1)) &&
                                    (kCausal || (kRagged && p.seqlen - j_abs * kAttnRows < kAttnRows));
             const int keep = kCausal ? row : p.seqlen - j_abs * kAttnRows - 1;
             {
               // fetch this row's last 32 scores while the softmax warp forms the maximum
-              mbar_wait(bar(C::kBarSFull + s), cnt_h[s] & 1u, wctx, kSiteSoftmaxSFull);
-              ++cnt_h[s];
+              mbar_wait(bar(C::kBarSFull + s), cnt_h[cur] & 1u, wctx, kSiteSoftmaxSFull);
+              ++cnt_h[cur];
               tc_fence_after();
               if (kHelperCols<D, kCausal || kRagged || kTail> == 48) tmem_ld16(t_lane + C::kColS + s * 128 + 80, sw);
               tmem_ld32(t_lane + C::kColS + s * 128 + 96, sv);
               if (kHelperCols<D, kCausal || kRagged || kTail> == 48) tc_wait_ld_bind16(sw);
               tc_wait_ld_bind(sv);
             }
-            mbar_wait(bar(C::kBarAlpha + s), cnt_a[s] & 1u, wctx, kSiteCorrAlpha);
-            ++cnt_a[s];
+            mbar_wait(bar(C::kBarAlpha + s), cnt_a[cur] & 1u, wctx, kSiteCorrAlpha);
+            ++cnt_a[cur];
             const float neg = stats_neg[s * 128 + row];
             // alpha = 2^((m_old - m_new) * c) = 2^(neg_new - neg_old); exactly 1 when the basis stood
-            const float alpha = (j == 0 || neg == neg_prev[s]) ? 1.0f : ex2_approx(neg - neg_prev[s]);
-            neg_prev[s] = neg;
+            const float alpha = (j == 0 || neg == neg_prev[cur]) ? 1.0f : ex2_approx(neg - neg_prev[cur]);
+            neg_prev[cur] = neg;
             if (j > 0) {
               if (__any_sync(0xffffffffu, alpha != 1.0f)) {
                 tc_fence_after();
@@ -923,43 +926,49 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
               float2 sum2 = make_float2(0.0f, 0.0f);
               uint32_t pk[16];
               [[maybe_unused]] uint32_t pk8[8];
-              // two copies of the loop, so that the tiles without masked keys (all but one
-              // per stage) carry no per-element compares
-              auto exps = [&](auto masked) {
-                if (kHelperCols<D, kCausal || kRagged || kTail> == 48) {
+              if (kHelperCols<D, kCausal || kRagged || kTail> == 48) {   // (a kernel without masks)
 #pragma unroll
-                  for (int i = 0; i < 8; ++i) {
-                    float2 e = exp2_poly2(__ffma2_rn(
-                        make_float2(__uint_as_float(sw[2 * i]), __uint_as_float(sw[2 * i + 1])), scale2, neg2));
-                    if (decltype(masked)::value) {
-                      if (80 + 2 * i > keep) e.x = 0.0f;
-                      if (80 + 2 * i + 1 > keep) e.y = 0.0f;
-                    }
-                    sum2 = __fadd2_rn(sum2, e);
-                    pk8[i] = pack_bf16x2(e.x, e.y);
-                  }
+                for (int i = 0; i < 8; ++i) {
+                  const float2 e = exp2_poly2(__ffma2_rn(
+                      make_float2(__uint_as_float(sw[2 * i]), __uint_as_float(sw[2 * i + 1])), scale2, neg2));
+                  sum2 = __fadd2_rn(sum2, e);
+                  pk8[i] = pack_bf16x2(e.x, e.y);
                 }
+              }
+              // masked keys: -inf, which the polynomial takes to 2^-126 (nothing beside a row
+              // sum, which is at least 1), and a weight of exactly zero below
+              if ((kCausal || kRagged) && mask_tile) {
+#pragma unroll
+                for (int i = 0; i < 32; ++i)
+                  if (96 + i > keep) sv[i] = 0xFF800000u;
+              }
+#pragma unroll
+              for (int i = 0; i < 16; ++i) {
+                const float2 e = exp2_poly2(__ffma2_rn(
+                    make_float2(__uint_as_float(sv[2 * i]), __uint_as_float(sv[2 * i + 1])), scale2, neg2));
+                sum2 = __fadd2_rn(sum2, e);
+                pk[i] = pack_bf16x2(e.x, e.y);
+              }
+              if ((kCausal || kRagged) && mask_tile) {
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
-                  float2 e = exp2_poly2(__ffma2_rn(
-                      make_float2(__uint_as_float(sv[2 * i]), __uint_as_float(sv[2 * i + 1])), scale2, neg2));
-                  if (decltype(masked)::value) {
-                    // masked keys weigh exactly zero (the polynomial bottoms out at 2^-126)
-                    if (96 + 2 * i > keep) e.x = 0.0f;
-                    if (96 + 2 * i + 1 > keep) e.y = 0.0f;
-                  }
-                  sum2 = __fadd2_rn(sum2, e);
-                  pk[i] = pack_bf16x2(e.x, e.y);
+                  if (96 + 2 * i > keep) pk[i] = 0u;
+                  else if (96 + 2 * i + 1 > keep) pk[i] &= 0xFFFFu;
                 }
-              };
-              if (mask_tile) exps(BoolTag<true>{}); else exps(BoolTag<false>{});
+              }
               if (kHelperCols<D, kCausal || kRagged || kTail> == 48) tmem_st8(t_lane + C::kColS + s * 128 + 40, pk8);   // P columns of keys 80..95
               tmem_st16(t_lane + C::kColS + s * 128 + 48, pk);   // P columns of keys 96..127
               tc_wait_st();
               tc_fence_before();
               mbar_arrive(bar(C::kBarPFull + 2 * s + 1));
-              l_part[s] = l_part[s] * alpha + (sum2.x + sum2.y);
+              l_part[cur] = l_part[cur] * alpha + (sum2.x + sum2.y);
             }
+          }
+          if constexpr (kStageUnroll == 1) {
+            uint32_t x = cnt_h[0]; cnt_h[0] = cnt_h[1]; cnt_h[1] = x;
+            x = cnt_a[0]; cnt_a[0] = cnt_a[1]; cnt_a[1] = x;
+            float f = neg_prev[0]; neg_prev[0] = neg_prev[1]; neg_prev[1] = f;
+            f = l_part[0]; l_part[0] = l_part[1]; l_part[1] = f;
           }
         }
       }

@@ -382,3 +382,40 @@ def test_cut_last_round_on_two_streams(pkg, gpu):
     for o, w in zip(outs, want):
         assert torch.equal(o, w)
 
+
+
+# ---------------------------------------------------------------------------
+# The edges of the last tile: its mask ends in every 32-column chunk of a row's scores (the
+# last chunk is the correction warps', packed two to a word), and the last rows written end
+# inside every group of 8 and 16 rows that the epilogue stores together.
+# ---------------------------------------------------------------------------
+@pytest.mark.parametrize("S", [1, 31, 32, 33, 64, 95, 96, 97, 98, 127, 128, 129, 135, 136, 145, 160, 223, 224, 225, 255,
+                               257, 383, 385, 481])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("causal", [False, True])
+def test_last_tile_edges_against_64_bit(pkg, gpu, S, D, causal):
+    B, H, Hkv = 2, 4, 2
+    g = torch.Generator(device=gpu).manual_seed(S * 2 + D + causal)
+    q = torch.randn(B, H, S, D, generator=g, device=gpu).to(torch.bfloat16)
+    k, v = (torch.randn(B, Hkv, S, D, generator=g, device=gpu).to(torch.bfloat16) for _ in range(2))
+    n = B * H * S * D
+    guarded = torch.full((n + 2048,), 7.0, dtype=torch.bfloat16, device=gpu)
+    lse = torch.empty(B * H * S, device=gpu)
+    o = pkg.ops.fa_fwd(q, k, v, causal=causal, out=guarded[1024:1024 + n].view(B, H, S, D), lse=lse)
+    status = pkg.ops.sync_status()
+    assert status == 0, pkg.native.strerror(status)
+    assert torch.all(guarded[:1024] == 7.0) and torch.all(guarded[1024 + n:] == 7.0)
+    kd, vd = (t.double().repeat_interleave(H // Hkv, dim=1) for t in (k, v))
+    scores = q.double() @ kd.mT * D ** -0.5
+    if causal:
+        scores.masked_fill_(torch.ones(S, S, dtype=torch.bool, device=gpu).triu(1), float("-inf"))
+    w = torch.softmax(scores, dim=-1)
+    ref = w @ vd
+    # P is rounded to bf16 (8 significant bits: half a unit in the last place is at most 2^-8 of
+    # each weight), its exponentials are off by at most 1e-4 (above and below the line of
+    # the quotient), and O is rounded to bf16 (2^-8); fp32 sums and scores add a few 1e-6
+    bound = (2.0 ** -8 + 3e-4) * (w @ vd.abs()) + 2.0 ** -8 * ref.abs() + 1e-6
+    assert bool(((o.double() - ref).abs() <= bound).all())
+    torch.testing.assert_close(lse.view(B, H, S).double(), torch.logsumexp(scores, dim=-1), rtol=1e-5, atol=1e-4)
+    if causal:
+        assert torch.equal(o[:, :, 0], v.repeat_interleave(H // Hkv, dim=1)[:, :, 0])   # masked keys weigh exactly zero
