@@ -7,7 +7,6 @@ compute-capability-10.x GPU these functions raise.
 """
 from __future__ import annotations
 
-import ctypes
 import math
 from typing import Optional
 
@@ -16,25 +15,44 @@ import torch
 from . import native
 
 
-def _ptr(t: Optional[torch.Tensor]) -> ctypes.c_void_p:
-    return ctypes.c_void_p(0 if t is None else t.data_ptr())
+# A small kernel runs for 2-5 us, and so may its launch: the calls below take the current
+# device and stream as integers straight from torch, enter a device context only when the
+# tensors' device is not the current one, and hand plain integers to ctypes (a row-wise
+# call's host time was 14 us with the stream objects, device contexts and c_void_p of before).
+_current_device = torch._C._cuda_getDevice if hasattr(torch._C, "_cuda_getDevice") else torch.cuda.current_device
 
 
-def _stream(stream: Optional[torch.cuda.Stream], device=None) -> ctypes.c_void_p:
-    s = torch.cuda.current_stream(device) if stream is None else stream
-    return ctypes.c_void_p(s.cuda_stream)
+def _raw_stream(stream: Optional[torch.cuda.Stream], index: int) -> int:
+    return torch._C._cuda_getCurrentRawStream(index) if stream is None else stream.cuda_stream
 
 
-def _require_cuda(*tensors) -> None:
+def _launch(entry: str, device, *args) -> None:
+    """Calls a library entry point with the tensors' device current; raises on an error code."""
+    fn = getattr(native.lib(), entry)
+    if _current_device() == device.index:
+        rc = fn(*args)
+    else:
+        with torch.cuda.device(device):
+            rc = fn(*args)
+    if rc:
+        native.check(rc)
+
+
+def _require_cuda(first, *others) -> None:
     """Every tensor is a contiguous CUDA tensor and all of them live on one device."""
-    for t in tensors:
+    device = first.device
+    good = first.is_cuda and first.is_contiguous()
+    for t in others:
+        good = good and t.is_contiguous() and t.device == device
+    if good:
+        return
+    for t in (first, *others):
         if not t.is_cuda:
             raise ValueError("ptxb200 ops take CUDA tensors (the library has no CPU path)")
         if not t.is_contiguous():
             raise ValueError("ptxb200 ops take contiguous tensors")
-    if len({t.device for t in tensors}) > 1:
-        raise ValueError("ptxb200 ops take tensors of ONE device; got " +
-                         ", ".join(sorted({str(t.device) for t in tensors})))
+    raise ValueError("ptxb200 ops take tensors of ONE device; got " +
+                     ", ".join(sorted({str(t.device) for t in (first, *others)})))
 
 
 def _check_out(out, like_device, shape, dtype, what: str = "out") -> None:
@@ -68,11 +86,12 @@ def fa_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, causal: bool = 
     _require_cuda(q, k, v)
     if q.dtype != torch.bfloat16 or k.dtype != torch.bfloat16 or v.dtype != torch.bfloat16:
         raise ValueError("fa_fwd takes bf16 tensors")
-    if q.dim() != 4 or k.shape != v.shape or k.dim() != 4 or (q.shape[0], q.shape[2], q.shape[3]) != (
-            k.shape[0], k.shape[2], k.shape[3]):
+    q_shape, k_shape = q.shape, k.shape
+    if len(q_shape) != 4 or len(k_shape) != 4 or k_shape != v.shape or q_shape[0] != k_shape[0] or (
+            q_shape[2:] != k_shape[2:]):
         raise ValueError("fa_fwd takes Q [B,H,S,D] and K, V [B,H_kv,S,D]")
-    B, H, S, D = q.shape
-    H_kv = k.shape[1]
+    B, H, S, D = q_shape
+    H_kv = k_shape[1]
     if lse is not None:
         _require_cuda(lse)
         if lse.device != q.device or lse.dtype != torch.float32 or lse.numel() != B * H * S:
@@ -81,20 +100,18 @@ def fa_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, causal: bool = 
         _require_cuda(dbg)
         if dbg.device != q.device or dbg.dtype != torch.int32 or dbg.numel() < 64:
             raise ValueError("dbg must be an int32 CUDA tensor of at least 64 words on the tensors' device")
-    if k.device != q.device:
-        raise ValueError("q, k and v must live on one device")
-    _check_stream(stream, q.device)
+    if stream is not None:
+        _check_stream(stream, q.device)
     if sm_scale is None:
         sm_scale = 1.0 / math.sqrt(D)
     if out is None:
         out = torch.empty_like(q)
     else:
         _check_out(out, q.device, q.shape, torch.bfloat16)
-    with torch.cuda.device(q.device):
-        rc = native.lib().fa_fwd_bf16_ex(_ptr(out), _ptr(lse), _ptr(q), _ptr(k), _ptr(v), B, H, H_kv, S, D,
-                                         ctypes.c_float(sm_scale), int(bool(causal)), flags, _ptr(dbg),
-                                         _stream(stream, q.device))
-    native.check(rc)
+    dev = q.device
+    _launch("fa_fwd_bf16_ex", dev, out.data_ptr(), None if lse is None else lse.data_ptr(), q.data_ptr(), k.data_ptr(),
+            v.data_ptr(), B, H, H_kv, S, D, sm_scale, 1 if causal else 0, flags,
+            None if dbg is None else dbg.data_ptr(), _raw_stream(stream, dev.index))
     return out
 
 
@@ -114,9 +131,10 @@ def gemm(a: torch.Tensor, bt: torch.Tensor, *, out: Optional[torch.Tensor] = Non
     M, K = a.shape
     N = bt.shape[0]
     want = torch.float32 if f32_out else torch.bfloat16
-    _check_stream(stream, a.device)
+    if stream is not None:
+        _check_stream(stream, a.device)
     if out is None:
-        out = torch.empty((M, N), device=a.device, dtype=want)
+        out = a.new_empty((M, N), dtype=want)
         ldc = N
     else:
         # a row-strided view (columns of a wider buffer) is allowed: ldc carries the pitch
@@ -129,9 +147,9 @@ def gemm(a: torch.Tensor, bt: torch.Tensor, *, out: Optional[torch.Tensor] = Non
         ldc = out.stride(0)
     flags = ((native.GEMM_F32_OUT if f32_out else 0) | (native.GEMM_NO_SPLIT if no_split else 0)
              | (native.GEMM_ONE_CTA if one_cta else 0))
-    with torch.cuda.device(a.device):
-        rc = native.lib().gemm_bf16(_ptr(out), _ptr(a), _ptr(bt), M, N, K, ldc, flags, _stream(stream, a.device))
-    native.check(rc)
+    dev = a.device
+    _launch("gemm_bf16", dev, out.data_ptr(), a.data_ptr(), bt.data_ptr(), M, N, K, ldc, flags,
+            _raw_stream(stream, dev.index))
     return out
 
 
@@ -151,30 +169,35 @@ def gemm_grouped(a: torch.Tensor, bt: torch.Tensor, *, out: Optional[torch.Tenso
     G, M, K = a.shape
     N = bt.shape[1]
     want = torch.float32 if f32_out else torch.bfloat16
-    _check_stream(stream, a.device)
+    if stream is not None:
+        _check_stream(stream, a.device)
     if out is None:
-        out = torch.empty((G, M, N), device=a.device, dtype=want)
+        out = a.new_empty((G, M, N), dtype=want)
     else:
         _check_out(out, a.device, (G, M, N), want)
     flags = ((native.GEMM_F32_OUT if f32_out else 0) | (native.GEMM_NO_SPLIT if no_split else 0)
              | (native.GEMM_ONE_CTA if one_cta else 0))
-    with torch.cuda.device(a.device):
-        rc = native.lib().gemm_bf16_grouped(_ptr(out), _ptr(a), _ptr(bt), G, M, N, K, N, flags,
-                                            _stream(stream, a.device))
-    native.check(rc)
+    dev = a.device
+    _launch("gemm_bf16_grouped", dev, out.data_ptr(), a.data_ptr(), bt.data_ptr(), G, M, N, K, N, flags,
+            _raw_stream(stream, dev.index))
     return out
 
 
 def _rowwise_check(x: torch.Tensor, *vecs: torch.Tensor) -> None:
     _require_cuda(x, *vecs)
-    if x.dtype != torch.float32 or x.dim() != 2 or any(v.dtype != torch.float32 for v in vecs):
+    good = x.dtype == torch.float32 and x.dim() == 2
+    for v in vecs:
+        good = good and v.dtype == torch.float32
+    if not good:
         raise ValueError("row-wise ops take a [rows, N] float32 matrix (and [N] float32 vectors)")
-    if any(v.numel() != x.shape[1] for v in vecs):
-        raise ValueError("weight / bias length must equal N")
+    for v in vecs:
+        if v.numel() != x.shape[1]:
+            raise ValueError("weight / bias length must equal N")
 
 
 def _rowwise_out(x, out, stream):
-    _check_stream(stream, x.device)
+    if stream is not None:
+        _check_stream(stream, x.device)
     if out is None:
         return torch.empty_like(x)
     _check_out(out, x.device, x.shape, torch.float32)
@@ -186,9 +209,9 @@ def softmax(x: torch.Tensor, *, out: Optional[torch.Tensor] = None,
     """Row-wise softmax of a [rows, N] float32 matrix (test/gpu/softmax.jl:151-163)."""
     _rowwise_check(x)
     out = _rowwise_out(x, out, stream)
-    with torch.cuda.device(x.device):
-        rc = native.lib().softmax_f32(_ptr(out), _ptr(x), x.shape[0], x.shape[1], _stream(stream, x.device))
-    native.check(rc)
+    dev = x.device
+    rows, N = x.shape
+    _launch("softmax_f32", dev, out.data_ptr(), x.data_ptr(), rows, N, _raw_stream(stream, dev.index))
     return out
 
 
@@ -197,10 +220,10 @@ def rms_norm(x: torch.Tensor, w: torch.Tensor, eps: float = 1e-6, *, out: Option
     """y = x * w / sqrt(mean(x^2) + eps) per row (test/gpu/rms_norm.jl:121-139)."""
     _rowwise_check(x, w)
     out = _rowwise_out(x, out, stream)
-    with torch.cuda.device(x.device):
-        rc = native.lib().rms_norm_f32(_ptr(out), _ptr(x), _ptr(w), x.shape[0], x.shape[1],
-                                       ctypes.c_float(eps), _stream(stream, x.device))
-    native.check(rc)
+    dev = x.device
+    rows, N = x.shape
+    _launch("rms_norm_f32", dev, out.data_ptr(), x.data_ptr(), w.data_ptr(), rows, N, eps,
+            _raw_stream(stream, dev.index))
     return out
 
 
@@ -210,10 +233,10 @@ def layer_norm(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor, eps: float 
     """y = (x - mean) / sqrt(var + eps) * w + bias per row (test/gpu/layer_norm.jl:138-156)."""
     _rowwise_check(x, w, bias)
     out = _rowwise_out(x, out, stream)
-    with torch.cuda.device(x.device):
-        rc = native.lib().layer_norm_f32(_ptr(out), _ptr(x), _ptr(w), _ptr(bias), x.shape[0],
-                                         x.shape[1], ctypes.c_float(eps), _stream(stream, x.device))
-    native.check(rc)
+    dev = x.device
+    rows, N = x.shape
+    _launch("layer_norm_f32", dev, out.data_ptr(), x.data_ptr(), w.data_ptr(), bias.data_ptr(), rows, N, eps,
+            _raw_stream(stream, dev.index))
     return out
 
 
@@ -224,9 +247,9 @@ def swiglu(gate: torch.Tensor, up: torch.Tensor, *, out: Optional[torch.Tensor] 
     if gate.dtype != torch.float32 or up.dtype != torch.float32 or gate.shape != up.shape:
         raise ValueError("swiglu takes two float32 tensors of one shape")
     out = _rowwise_out(gate, out, stream)
-    with torch.cuda.device(gate.device):
-        rc = native.lib().swiglu_f32(_ptr(out), _ptr(gate), _ptr(up), gate.numel(), _stream(stream, gate.device))
-    native.check(rc)
+    dev = gate.device
+    _launch("swiglu_f32", dev, out.data_ptr(), gate.data_ptr(), up.data_ptr(), gate.numel(),
+            _raw_stream(stream, dev.index))
     return out
 
 
@@ -235,20 +258,20 @@ def selftest(which: int, q=None, k=None, v=None, p=None):
     dev = torch.device("cuda", torch.cuda.current_device())
     if which == 0:
         out_s = torch.zeros(128 * 128, dtype=torch.int32, device=dev)
-        rc = native.lib().ptxb200_selftest(0, _ptr(out_s), None, None, None, None, None, _stream(None))
+        rc = native.lib().ptxb200_selftest(0, out_s.data_ptr(), None, None, None, None, None, _raw_stream(None, dev.index))
         native.check(rc)
         return out_s.view(128, 128), None
     if which == 3 or which == 4:
         out_s = torch.zeros(16, dtype=torch.int32, device=dev)
-        rc = native.lib().ptxb200_selftest(which, _ptr(out_s), None, None, None, None, None, _stream(None))
+        rc = native.lib().ptxb200_selftest(which, out_s.data_ptr(), None, None, None, None, None, _raw_stream(None, dev.index))
         native.check(rc)
         return out_s, None
     D = 128 if which == 1 else 64
     _require_cuda(q, k, v, p)
     out_s = torch.zeros((128, 128), dtype=torch.float32, device=dev)
     out_o = torch.zeros((128, D), dtype=torch.float32, device=dev)
-    rc = native.lib().ptxb200_selftest(which, _ptr(out_s), _ptr(out_o), _ptr(q), _ptr(k), _ptr(v),
-                                       _ptr(p), _stream(None))
+    rc = native.lib().ptxb200_selftest(which, out_s.data_ptr(), out_o.data_ptr(), q.data_ptr(), k.data_ptr(),
+                                       v.data_ptr(), p.data_ptr(), _raw_stream(None, dev.index))
     native.check(rc)
     return out_s, out_o
 
