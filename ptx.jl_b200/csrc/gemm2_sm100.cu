@@ -186,7 +186,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   } else {
     // ---------------- epilogue (both CTAs): this CTA's 128 rows of the tile ----------------
     const int quad = warp & 3;
-    const int row_in_half = quad * 32 + lane;
     const uint32_t leader_acc_empty = map_to_cta(bar_acc_empty, 0);
     uint32_t t = 0;
     for (int tile = pair; tile < total_tiles; tile += pairs, ++t) {
@@ -197,19 +196,21 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       const uint32_t aph = (t >> 1) & 1u;
       mbar_wait(bar_acc_full + 8 * buf, aph, wctx, kSite2AccFull);
       tc_fence_after();
-      const size_t row = (size_t)g * M + (size_t)tm * kBM2 + rank * 128 + row_in_half;
       // in a half-filled last row-tile the peer's 128 rows lie past M (its A box read the
       // next group's rows or zero fill): computed, not stored
       const bool rows_valid = tm * kBM2 + (int)rank * 128 < M;
       const int col0 = tn * kBN;
-      const uint32_t t_row = tmem_addr(tmem, quad * 32, buf * kAccCols2);
 #pragma unroll 1
-      for (int c = 0; c < kBN / 32; ++c) {
-        uint32_t v[32];
-        tmem_ld32(t_row + c * 32, v);
-        tc_wait_ld_bind(v);
-        const int col = col0 + c * 32;
-        if (col < N && rows_valid) store_acc_chunk<kF32Out>(c_out, row, ldc, col, v);
+      for (int h = 0; h < 2; ++h) {          // this warp's first and second 16 rows
+        const size_t row = (size_t)g * M + (size_t)tm * kBM2 + rank * 128 + quad * 32 + h * 16 + (lane >> 2);
+        const uint32_t t_row = tmem_addr(tmem, quad * 32 + h * 16, buf * kAccCols2);
+#pragma unroll 1
+        for (int c = 0; c < kBN; c += 64) {
+          uint32_t v[32];
+          tmem_ld_16x64(t_row + c, v);
+          tc_wait_ld_bind(v);
+          if (col0 + c < N && rows_valid) store_acc_16x64<kF32Out>(c_out, row, ldc, col0 + c, v);   // N % 64 == 0
+        }
       }
       tc_fence_before();
       mbar_arrive_cluster(leader_acc_empty + 8 * buf);

@@ -181,7 +181,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   } else {
     // ---------------- epilogue: warps 2..5 ----------------
     const int quad = warp & 3;                       // TMEM lane quadrant this warp may touch
-    const int row_in_tile = quad * 32 + lane;
     uint32_t t = 0;
     for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++t) {
       int tm, tn;
@@ -191,16 +190,18 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       const uint32_t aph = (t >> 1) & 1u;
       mbar_wait(bar_acc_full + 8 * buf, aph, wctx, kSiteAccFull);
       tc_fence_after();
-      const size_t row = (size_t)g * M + (size_t)tm * kBM + row_in_tile;
       const int col0 = tn * kBN;
-      const uint32_t t_row = tmem_addr(tmem, quad * 32, buf * kAccCols);
 #pragma unroll 1
-      for (int c = 0; c < kBN / 32; ++c) {
-        uint32_t v[32];
-        tmem_ld32(t_row + c * 32, v);
-        tc_wait_ld_bind(v);
-        const int col = col0 + c * 32;
-        if (col < N) store_acc_chunk<kF32Out>(c_out, row, ldc, col, v);
+      for (int h = 0; h < 2; ++h) {                  // this warp's first and second 16 rows
+        const size_t row = (size_t)g * M + (size_t)tm * kBM + quad * 32 + h * 16 + (lane >> 2);
+        const uint32_t t_row = tmem_addr(tmem, quad * 32 + h * 16, buf * kAccCols);
+#pragma unroll 1
+        for (int c = 0; c < kBN; c += 64) {
+          uint32_t v[32];
+          tmem_ld_16x64(t_row + c, v);
+          tc_wait_ld_bind(v);
+          if (col0 + c < N) store_acc_16x64<kF32Out>(c_out, row, ldc, col0 + c, v);   // N % 64 == 0
+        }
       }
       // every TMEM read of this accumulator has completed (wait::ld above)
       tc_fence_before();

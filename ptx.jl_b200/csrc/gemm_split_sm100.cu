@@ -210,11 +210,24 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   }
   if (split == 1) {
     if (epilogue) {
-#pragma unroll 2
-      for (int c = 0; c < kBN; c += 16) {
-        float x[16];
-        load_sum16<kBN>(t_row + c, chains, x);
-        if (col0 + c < N) store_acc_chunk16<kF32Out>(c_out, row, ldc, col0 + c, x);
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {          // this warp's first and second 16 rows
+        const size_t row16 = (size_t)g * M + (size_t)tm * kBM3 + quad * 32 + h * 16 + (lane >> 2);
+#pragma unroll 1
+        for (int c = 0; c < kBN; c += 64) {
+          uint32_t v[32];
+          tmem_ld_16x64(t_row + ((uint32_t)(h * 16) << 16) + c, v);
+          tc_wait_ld_bind(v);
+#pragma unroll 1
+          for (int a = 1; a < chains; ++a) {
+            uint32_t x[32];
+            tmem_ld_16x64(t_row + ((uint32_t)(h * 16) << 16) + a * kBN + c, x);
+            tc_wait_ld_bind(x);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) + __uint_as_float(x[i]));
+          }
+          if (col0 + c < N) store_acc_16x64<kF32Out>(c_out, row16, ldc, col0 + c, v);   // N % 64 == 0
+        }
       }
     }
   } else {
