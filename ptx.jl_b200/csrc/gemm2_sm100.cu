@@ -233,16 +233,17 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 // Columns of the pair's tile for a product, or 0 where 128x256 tiles of single CTAs
 // (gemm_sm100.cu) are the better choice. The estimate, in us: rounds over the machine times
 // what a tile costs, which is its steps of K (0.345, 0.27, 0.215 us for 256, 192, 128 columns;
-// single CTAs 0.36) or, for short K, its epilogue (0.013 us per column), plus one epilogue.
+// single CTAs 0.36) or, for short K, its epilogue (0.3 us + 0.004 per column), plus one epilogue.
 // Wide tiles cost least per column; narrower ones are taken where they fill the last round
-// better: 2304x2304x1024 19.0 us with 256 columns, 15.6 with 192; 1792x1792x8192 45.8 and
-// 40.6; 3072x5120x8192 194 and 184; 8192^3 694 and 722. Single CTAs win where M leaves half
-// of a pair's last row-tile empty (32 products of 128x2048x2048: 63.0 us in pairs, 53.9
+// better: 2304x2304x1024 16.2 us with 256 columns, 13.9 with 192; 1792x1792x8192 43.7 and
+// 36.8; 48 products of 256x320x512 13.1 with 256, 11.4 with 128; the other way round
+// 8192x8192x512 50.9 with 256, 65.9 with 128 and 8192^3 694 and 833. Single CTAs win where M leaves half
+// of a pair's last row-tile empty (32 products of 128x2048x2048: 59.3 us in pairs, 52.8
 // single). Any width gives the same bits: an element is one accumulation in k order.
 int gemm_pair_tile(const DeviceCtx& ctx, int groups, int M, int N, int K) {
   const double kiters = K / kBK2;
   auto cost = [&](long long tiles, long long at_once, double step, int bn) {
-    const double epilogue = 0.013 * bn, tile = kiters * step > epilogue ? kiters * step : epilogue;
+    const double epilogue = 0.3 + 0.004 * bn, tile = kiters * step > epilogue ? kiters * step : epilogue;
     return (double)((tiles + at_once - 1) / at_once) * tile + epilogue;
   };
   const int pairs = ctx.sm_count / 2;

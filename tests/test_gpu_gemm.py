@@ -266,8 +266,9 @@ def test_grouped_gemm_pair_kernel(pkg, gpu):
     (1, 2304, 2304, 1024),      # pair tiles of 192 columns
     (1, 2432, 2368, 832),       # the same, half-filled row-tile, 64 columns over
     (5, 1024, 512, 512),        # the same, groups
-    (8, 640, 704, 832),         # pair tiles of 128 columns, half-filled row-tiles, 64 columns over
-    (1, 2048, 3008, 448),       # the same, one product
+    (8, 640, 704, 832),         # pair tiles of 256 columns, half-filled row-tiles, 192 columns over
+    (3, 1280, 1088, 448),       # pair tiles of 128 columns, 64 columns over
+    (48, 256, 320, 512),        # the same, many products
     (40, 128, 320, 128),        # M of one half row-tile per group
 ])
 @pytest.mark.parametrize("f32_out", [True, False])
