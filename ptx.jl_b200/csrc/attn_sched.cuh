@@ -48,6 +48,7 @@ struct FaSched {
   int tail_units;    // units [full_units, full_units + tail_units) are cut along the line
   int tail_steps;    // length of that line
   int tail_ctas;     // CTAs [0, tail_ctas) share the line equally
+  int by_length;     // causal, no pairs, no cut: items dealt longest first over all heads, to and fro (fa_length_rank)
 };
 
 // One piece of work for a CTA: key tiles [j0, j1) of item (mb, bh), whose last stage has
@@ -65,6 +66,11 @@ PTXB200_HD int fa_item_steps(int mb, int nt_all, int causal) {
   const int x = 2 * mb + 2;
   return x < nt_all ? x : nt_all;
 }
+// by_length: place in the order by length of CTA cta's v-th item. Rounds run over the CTAs to and
+// fro, so that whoever had the longest item of one round gets the shortest of the next. Item
+// rank r is block num_mblocks - 1 - r / bh of head r % bh; a CTA is done at the first rank past
+// the last item.
+PTXB200_HD int fa_length_rank(int cta, int v, int grid) { return v * grid + ((v & 1) ? grid - 1 - cta : cta); }
 PTXB200_HD int fa_num_units(const FaSched& s) {
   return (s.causal && s.pair_mode) ? s.bh * ((s.num_mblocks + 1) >> 1) : s.bh * s.num_mblocks;
 }

@@ -221,6 +221,9 @@ enum : int { kWhole = 0, kWriter = 1, kCombiner = 2 };
 //    coarse unit when a launch has few of them; the host compares the two static
 //    schedules' longest CTA and falls back to single items where pairs lose more than
 //    a tenth (causal_pair_mode below).
+//    Launches whose K and V fit in L2 have no need to keep a head's items together: they
+//    deal the items of all heads by length where that shortens the longest CTA's work
+//    (fa_length_rank, plan_schedule).
 template <bool kCausal>
 struct ItemIter {
   int v = 0;   // items this CTA has taken so far
@@ -271,11 +274,26 @@ __device__ __forceinline__ void tile_counts(const FaParams& p, int mb, int& nt0,
 // out. kTail = true: the items of the full rounds, then this CTA's segments of the cut last
 // round from the table in shared memory (fa_fwd_kernel's prologue fills it: int count, pad,
 // FaSeg[kTailMaxSegs]).
-template <bool kCausal, bool kTail>
+template <bool kCausal, bool kTail, bool kByLen = false>
 struct WorkIter {
   ItemIter<kCausal> rr;
   int tail_i = -1;   // kTail: -1 while the round-robin part lasts, then the next table entry
   __device__ __forceinline__ bool next(const FaParams& p, const uint8_t* seg_table, WorkItem& w) {
+    if constexpr (kByLen) {
+      const int r = fa_length_rank(blockIdx.x, rr.v, gridDim.x);
+      if (r >= p.total_work) return false;
+      ++rr.v;
+      const int level = r / p.bh;
+      w.mb = p.num_mblocks - 1 - level;
+      w.bh = r - level * p.bh;
+      tile_counts<true>(p, w.mb, w.nt[0], w.nt[1]);
+      w.j0 = 0;
+      w.jlast[0] = w.nt[0] - 1;
+      w.jlast[1] = w.nt[1] - 1;
+      w.kind = kWhole;
+      w.n_other = 0;
+      return true;
+    }
     if (!kTail || tail_i < 0) {
       const int units = kTail ? p.sched.full_units
                               : ((kCausal && p.pair_mode) ? p.bh * ((p.num_mblocks + 1) >> 1) : p.total_work);
@@ -387,7 +405,7 @@ __device__ __noinline__ void tail_table(const FaSched sc, uint8_t* table) {
 // tile over the slot with every descriptor an immediate (faster in isolation, slower
 // here, most of all for causal shapes), and issuing from the converged warp with an
 // elected lane (the GEMM kernel's scheme).
-template <int D, bool kCausal, bool kConv, bool kTail>
+template <int D, bool kCausal, bool kConv, bool kTail, bool kByLen>
 __device__ __forceinline__ void fa_mma_role(const FaParams& p, uint32_t base, uint32_t tmem,
                                             const WaitCtx& wctx, const uint8_t* seg_table) {
   using C = FaCfg<D>;
@@ -475,7 +493,7 @@ __device__ __forceinline__ void fa_mma_role(const FaParams& p, uint32_t base, ui
   // the MUFU rather than the issue order bounds a tile, this measured slower on causal
   // problems, so there each item starts behind the previous one's last P V.
     constexpr bool kStream = (D == 128);
-  WorkIter<kCausal, kTail> items;
+  WorkIter<kCausal, kTail, kByLen> items;
   WorkItem w, w2;
   int nt[2] = {0, 0};
   bool have = items.next(p, seg_table, w);
@@ -589,7 +607,8 @@ __device__ __forceinline__ void store_rows(uint32_t o_tmem, __nv_bfloat16* dst, 
 // CTA runs its segments of that round after its whole items, parks or merges pieces in the
 // epilogue. A variant of its own so that launches without a cut run exactly the code they
 // ran before the cut existed.
-template <int D, bool kCausal, bool kCtaFlags = false, bool kRagged = false, bool kTail = false>
+// kByLen (causal only): the items of all heads dealt by length (fa_length_rank).
+template <int D, bool kCausal, bool kCtaFlags = false, bool kRagged = false, bool kTail = false, bool kByLen = false>
 __global__ void __launch_bounds__(kThreads, 1)
 fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
               const __grid_constant__ CUtensorMap tmap_v, const FaParams p) {
@@ -671,7 +690,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
           T::load3(kv_smem + s * T::kTileBytes, tmap, row, slice, bar(C::kBarKvFull + s));
           ++kv_it;
         };
-        WorkIter<kCausal, kTail> items;
+        WorkIter<kCausal, kTail, kByLen> items;
         for (WorkItem w; items.next(p, seg_table, w); ++item_i) {
           const int mb = w.mb, bh = w.bh, nt1 = w.nt[1];
           const int kv_row0 = kTail ? w.j0 * kAttnRows : 0;   // first key tile of this piece of the item
@@ -699,9 +718,9 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
       }
     } else if (warp == 12) {
 #ifdef PTXB200_FA_MMA_CONVERGED
-      fa_mma_role<D, kCausal, true, kTail>(p, base, tmem, wctx, seg_table);
+      fa_mma_role<D, kCausal, true, kTail, kByLen>(p, base, tmem, wctx, seg_table);
 #else
-      if (elect_one()) fa_mma_role<D, kCausal, false, kTail>(p, base, tmem, wctx, seg_table);
+      if (elect_one()) fa_mma_role<D, kCausal, false, kTail, kByLen>(p, base, tmem, wctx, seg_table);
 #endif
     }
   } else if (warp < 8) {
@@ -715,7 +734,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
     const uint32_t t_row = tmem_addr(tmem, (warp & 3) * 32, C::kColS + stage * 128);
     const float scale_log2 = p.scale_log2;
     uint32_t cnt_s = 0, items_done = 0;
-    WorkIter<kCausal, kTail> items;
+    WorkIter<kCausal, kTail, kByLen> items;
     for (WorkItem w; items.next(p, seg_table, w);) {
       const int ntiles = stage ? w.nt[1] : w.nt[0];
       // the stage's final tile of the item: the piece's last tile, unless the item is cut there
@@ -864,7 +883,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
     uint32_t cnt_a[2] = {0, 0};
     uint32_t cnt_h[2] = {0, 0};   // S tiles seen per stage
     uint32_t item_i = 0;
-    WorkIter<kCausal, kTail> items;
+    WorkIter<kCausal, kTail, kByLen> items;
     for (WorkItem w; items.next(p, seg_table, w); ++item_i) {
       const int mb = w.mb, bh = w.bh;
       const int nt[2] = {w.nt[0], w.nt[1]};
@@ -1228,53 +1247,101 @@ long long worst_round_robin(const FaSched& sc, int units, int grid) {
 
 constexpr int kSplitOverheadSteps = 3;   // what a second segment, parking and merging cost a CTA, in steps (measured: 2.5-3)
 constexpr int kSplitMaxRounds = 64;      // beyond this many full rounds the tail is noise: not split
+constexpr int kItemOverheadSteps = 1;    // what the boundary between two items costs a CTA, in steps (measured: 1-1.5)
+// K and V of all heads together up to about L2's size (126 MB) are read from HBM once or little
+// more whatever the order of the items (measured to 134 MB); above it pairs, which keep a
+// head's CTAs together, do that.
+constexpr long long kByLengthMaxKvBytes = 160ll << 20;
+constexpr int kByLengthMaxItems = 1 << 16;
 
-// Round robin over whole units (the reference's distribution), or the same with the last,
-// partly filled round cut along the key axis when that shortens the busiest CTA's work by
-// more than the overhead of the cut.
-FaSched plan_schedule(int bh, int nmb, int nt_all, int causal, unsigned flags, int sm_count, bool may_split) {
-  FaSched legacy;
-  legacy.num_mblocks = nmb;
-  legacy.bh = bh;
-  legacy.nt_all = nt_all;
-  legacy.causal = causal;
-  legacy.pair_mode = (causal && !(flags & PTXB200_FA_SINGLE_BLOCKS)) ? causal_pair_mode(bh, nmb, nt_all, sm_count) : 0;
-  const long long legacy_units = (long long)bh * (legacy.pair_mode ? (nmb + 1) / 2 : nmb);
-  legacy.grid = legacy_units < sm_count ? (int)legacy_units : sm_count;
-  legacy.full_units = (int)legacy_units;
-  legacy.tail_units = legacy.tail_steps = legacy.tail_ctas = 0;
-  if (!may_split || (flags & PTXB200_FA_NO_TAIL_SPLIT) || sm_count > 256) return legacy;
+// Steps and item boundaries of the busiest CTA when all causal items are dealt by length.
+long long worst_by_length(int bh, int nmb, int nt_all, int grid) {
+  long long worst = 0;
+  const int items = bh * nmb;
+  for (int c = 0; c < grid; ++c) {
+    long long sum = 0;
+    for (int v = 0, r; (r = fa_length_rank(c, v, grid)) < items; ++v)
+      sum += fa_item_steps(nmb - 1 - r / bh, nt_all, 1) + kItemOverheadSteps;
+    worst = sum > worst ? sum : worst;
+  }
+  return worst;
+}
 
+FaSched plan_uncached(int bh, int nmb, int nt_all, int causal, unsigned flags, int sm_count, bool may_split, bool kv_in_l2);
+
+// The distribution of a launch; the last few shapes' are kept, since finding one walks every CTA.
+FaSched plan_schedule(int bh, int nmb, int nt_all, int causal, unsigned flags, int sm_count, bool may_split,
+                      long long kv_bytes) {
+  const bool kv_in_l2 = kv_bytes <= kByLengthMaxKvBytes;
   struct Key {
     int bh, nmb, nt_all, causal, sm;
     unsigned flags;
+    bool may_split, kv_in_l2;
     bool operator==(const Key& o) const {
-      return bh == o.bh && nmb == o.nmb && nt_all == o.nt_all && causal == o.causal && sm == o.sm && flags == o.flags;
+      return bh == o.bh && nmb == o.nmb && nt_all == o.nt_all && causal == o.causal && sm == o.sm && flags == o.flags &&
+             may_split == o.may_split && kv_in_l2 == o.kv_in_l2;
     }
   };
   static std::mutex mu;
-  static std::vector<std::pair<Key, FaSched>> cache;   // the last few shapes: the decision walks every tail CTA
-  const Key key{bh, nmb, nt_all, causal, sm_count, flags};
+  static std::vector<std::pair<Key, FaSched>> cache;
+  const Key key{bh, nmb, nt_all, causal, sm_count, flags, may_split, kv_in_l2};
   {
     std::lock_guard<std::mutex> lock(mu);
     for (const auto& kv : cache)
       if (kv.first == key) return kv.second;
   }
-  auto remember = [&](const FaSched& sc) {
-    std::lock_guard<std::mutex> lock(mu);
-    if (cache.size() >= 16) cache.erase(cache.begin());
-    cache.emplace_back(key, sc);
-    return sc;
-  };
+  const FaSched sc = plan_uncached(bh, nmb, nt_all, causal, flags, sm_count, may_split, kv_in_l2);
+  std::lock_guard<std::mutex> lock(mu);
+  if (cache.size() >= 16) cache.erase(cache.begin());
+  cache.emplace_back(key, sc);
+  return sc;
+}
+
+// Round robin over whole units (the reference's distribution); causal items by length; or
+// round robin with the last, partly filled round cut along the key axis when that shortens
+// the busiest CTA's work by more than the overhead of the cut.
+FaSched plan_uncached(int bh, int nmb, int nt_all, int causal, unsigned flags, int sm_count, bool may_split, bool kv_in_l2) {
+  FaSched legacy;
+  legacy.num_mblocks = nmb;
+  legacy.bh = bh;
+  legacy.nt_all = nt_all;
+  legacy.causal = causal;
+  legacy.by_length = 0;
+  legacy.pair_mode = (causal && !(flags & PTXB200_FA_SINGLE_BLOCKS)) ? causal_pair_mode(bh, nmb, nt_all, sm_count) : 0;
+  const long long legacy_units = (long long)bh * (legacy.pair_mode ? (nmb + 1) / 2 : nmb);
+  legacy.grid = legacy_units < sm_count ? (int)legacy_units : sm_count;
+  legacy.full_units = (int)legacy_units;
+  legacy.tail_units = legacy.tail_steps = legacy.tail_ctas = 0;
+  long long legacy_cost = -1;   // of the busiest CTA, in steps, where it was worked out
+  if (causal && kv_in_l2 && !(flags & (PTXB200_FA_SINGLE_BLOCKS | PTXB200_FA_ALWAYS_TAIL_SPLIT)) &&
+      (long long)bh * nmb <= kByLengthMaxItems && (long long)bh * nmb > sm_count) {
+    // 32 heads on 8 K/V heads, head dim 128: 2048 keys 43.6 us in pairs, 40.5 by length; 3001 keys
+    // 99.9 with the last round cut, 78.8 by length (32 steps on average, the busiest CTA has 36
+    // and two boundaries, no merging); 2 x 32 heads of 4096 keys, K and V 134 MB, 293 and 257.
+    const long long by_length = worst_by_length(bh, nmb, nt_all, sm_count);
+    const long long items = (long long)bh * nmb;
+    legacy_cost = worst_round_robin(legacy, legacy.full_units, legacy.grid) +
+                  kItemOverheadSteps * (legacy.pair_mode ? 2 * ((legacy_units + sm_count - 1) / sm_count)
+                                                         : (items + sm_count - 1) / sm_count);
+    if (by_length * 100 <= legacy_cost * 97) {
+      legacy.by_length = 1;
+      legacy.pair_mode = 0;
+      legacy.full_units = (int)items;
+      legacy.grid = sm_count;
+      legacy_cost = by_length;
+    }
+  }
+  if (!may_split || (flags & PTXB200_FA_NO_TAIL_SPLIT) || sm_count > 256) return legacy;
 
   FaSched sc = legacy;
+  sc.by_length = 0;
   sc.pair_mode = (causal && !(flags & PTXB200_FA_SINGLE_BLOCKS)) ? 1 : 0;   // pairs keep a head's CTAs together; the cut balances them
   const long long units = (long long)bh * (sc.pair_mode ? (nmb + 1) / 2 : nmb);
-  if (units > (long long)kSplitMaxRounds * sm_count) return remember(legacy);
+  if (units > (long long)kSplitMaxRounds * sm_count) return legacy;
   sc.grid = sm_count;
   sc.full_units = (int)(units / sm_count) * sm_count;
   sc.tail_units = (int)units - sc.full_units;
-  if (sc.tail_units == 0) return remember(legacy);
+  if (sc.tail_units == 0) return legacy;
   std::vector<int> starts(sc.tail_units + 1, 0);
   int longest_item = 0;
   for (int u = 0; u < sc.tail_units; ++u) {
@@ -1285,11 +1352,11 @@ FaSched plan_schedule(int bh, int nmb, int nt_all, int causal, unsigned flags, i
     longest_item = lb > longest_item ? lb : longest_item;
   }
   sc.tail_steps = starts.back();
-  if ((long long)sc.tail_steps * (sm_count + 1) >= (1ll << 31)) return remember(legacy);   // cut positions are 32-bit products
+  if ((long long)sc.tail_steps * (sm_count + 1) >= (1ll << 31)) return legacy;   // cut positions are 32-bit products
   int span_min = (longest_item + kTailMaxParts - 3) / (kTailMaxParts - 2);   // at most kTailMaxParts pieces per item
   if (span_min < 2 * fa_min_seg(causal)) span_min = 2 * fa_min_seg(causal);
   sc.tail_ctas = sc.tail_steps / span_min < sm_count ? sc.tail_steps / span_min : sm_count;
-  if (sc.tail_ctas < 2) return remember(legacy);
+  if (sc.tail_ctas < 2) return legacy;
   // the kernel's per-CTA table and the combiner's reads are bounded: walk every tail CTA,
   // and take the busiest one's steps from the walk (cuts snap to item edges, so spans differ)
   HostLocator loc{starts.data(), (int)starts.size() - 1};
@@ -1297,19 +1364,24 @@ FaSched plan_schedule(int bh, int nmb, int nt_all, int causal, unsigned flags, i
   for (int c = 0; c < sc.tail_ctas; ++c) {
     FaSeg segs[kTailMaxSegs];
     const int n = fa_tail_segments(sc, c, loc, segs);
-    if (n > kTailMaxSegs) return remember(legacy);
+    if (n > kTailMaxSegs) return legacy;
     int steps = 0;
     for (int i = 0; i < n; ++i) {
-      if (segs[i].n_other + 1 > kTailMaxParts) return remember(legacy);
+      if (segs[i].n_other + 1 > kTailMaxParts) return legacy;
       steps += segs[i].j1 - segs[i].j0;
     }
     tail_worst = steps > tail_worst ? steps : tail_worst;
   }
   const long long split_worst = worst_round_robin(sc, sc.full_units, sc.grid) + tail_worst + kSplitOverheadSteps;
+  if (flags & PTXB200_FA_ALWAYS_TAIL_SPLIT) return sc;
+  // cut only for a gain of a twelfth or more
+  if (legacy.by_length) {
+    const long long boundaries = kItemOverheadSteps * ((sc.pair_mode ? 2 : 1) * (sc.full_units / sm_count) + 1);
+    return (split_worst + boundaries) * 100 > legacy_cost * 92 ? legacy : sc;
+  }
   const long long legacy_worst = worst_round_robin(legacy, legacy.full_units, legacy.grid);
-  if (!(flags & PTXB200_FA_ALWAYS_TAIL_SPLIT) && split_worst * 100 > legacy_worst * 92)
-    return remember(legacy);   // cut only for a gain of a twelfth or more
-  return remember(sc);
+  if (split_worst * 100 > legacy_worst * 92) return legacy;
+  return sc;
 }
 
 constexpr size_t kPartsHeaderBytes = 4096;   // one flag word per CTA, ahead of the slots
@@ -1329,7 +1401,11 @@ int launch_variant(const DeviceCtx& ctx, const CUtensorMap& tq, const CUtensorMa
     PTXB200_CUDA_TRY(cudaFuncSetAttribute(fa_fwd_kernel<D, kCausal, false, false, true>,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           C::kSmemBytes));
-    if (!kCausal) {
+    if (kCausal) {
+      PTXB200_CUDA_TRY(cudaFuncSetAttribute(fa_fwd_kernel<D, true, false, false, false, true>,
+                                            cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            C::kSmemBytes));
+    } else {
       PTXB200_CUDA_TRY(cudaFuncSetAttribute(fa_fwd_kernel<D, false, false, true>,
                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             C::kSmemBytes));
@@ -1353,6 +1429,8 @@ int launch_variant(const DeviceCtx& ctx, const CUtensorMap& tq, const CUtensorMa
     const int grid = units < ctx.sm_count ? units : ctx.sm_count;
     if (ragged)
       fa_fwd_kernel<D, false, false, true><<<grid, kThreads, C::kSmemBytes, stream>>>(tq, tk, tv, p);
+    else if (kCausal && p.sched.by_length)
+      fa_fwd_kernel<D, kCausal, false, false, false, kCausal><<<grid, kThreads, C::kSmemBytes, stream>>>(tq, tk, tv, p);
     else
       fa_fwd_kernel<D, kCausal><<<grid, kThreads, C::kSmemBytes, stream>>>(tq, tk, tv, p);
   }
@@ -1396,7 +1474,8 @@ int launch_fa_fwd(const DeviceCtx& ctx, void* O, void* lse, const void* Q, const
   if ((rc = encode_tmap_bf16_3d(&tv, V, (uint64_t)B * H_kv, S, D, 128, 64)) != PTXB200_OK) return rc;
   FaParams p;
   fill_params(p, O, lse, B, H, H_kv, S, sm_scale, flags, dbg, status,
-              plan_schedule(B * H, (S + 255) / 256, (S + kAttnRows - 1) / kAttnRows, causal, flags, ctx.sm_count, true));
+              plan_schedule(B * H, (S + 255) / 256, (S + kAttnRows - 1) / kAttnRows, causal, flags, ctx.sm_count, true,
+                            4ll * B * H_kv * S * D));
   ScratchLease lease;
   if (p.sched.tail_units > 0) {
     // one slot of parked pieces and one flag per CTA, kept per (device, stream)
@@ -1428,7 +1507,8 @@ int launch_fa_fwd(const DeviceCtx& ctx, void* O, void* lse, const void* Q, const
 // or -1 if `cap` is too small.
 int describe_fa_plan(int BH, int S, int causal, unsigned flags, int sm_count, int* out, int cap) {
   const int nmb = (S + 255) / 256, nt_all = (S + kAttnRows - 1) / kAttnRows;
-  const FaSched sc = plan_schedule(BH, nmb, nt_all, causal, flags, sm_count, true);
+  // as for head dim 128 with a K/V head per query head
+  const FaSched sc = plan_schedule(BH, nmb, nt_all, causal, flags, sm_count, true, 4ll * BH * S * 128);
   int n = 0;
   auto put = [&](int v) {
     if (n < cap) out[n] = v;
@@ -1573,7 +1653,8 @@ extern "C" int fa_fwd_bf16_noalloc(void* O, const void* Q, const void* K, const 
   // whole items only: cutting the last round along the key axis needs scratch in proportion
   // to the SM count, which this entry point does not have
   fill_params(p, O, nullptr, B, H, H, S, sm_scale, flags, nullptr, nd.scratch,
-              plan_schedule(B * H, (S + 255) / 256, (S + kAttnRows - 1) / kAttnRows, causal, flags, nd.sm_count, false));
+              plan_schedule(B * H, (S + 255) / 256, (S + kAttnRows - 1) / kAttnRows, causal, flags, nd.sm_count, false,
+                            kByLengthMaxKvBytes + 1));
   p.cta_flags = nd.scratch + kNoAllocFlagBase;
   const int units = (causal && p.pair_mode) ? p.bh * ((p.num_mblocks + 1) / 2) : p.total_work;
   const int grid = units < nd.sm_count ? units : nd.sm_count;
