@@ -699,14 +699,17 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
           const int kv_head = (bh - b_idx * p.heads_q) / (p.heads_q / p.heads_kv);
           const int kv_slice = b_idx * p.heads_kv + kv_head;
           const int q_row0 = mb * 2 * kAttnRows;   // within the head's sequence; rows past its end load as zeros
-          // a stage's Q may be overwritten once its last S = Q K^T of the previous item has run
-          mbar_wait(bar(C::kBarQFree + 0), (item_i & 1u) ^ 1u, wctx, kSiteLoadQFree);
-          mbar_arrive_expect_tx(bar(C::kBarQFull + 0), T::kTileBytes);
-          T::load3(q_smem, &tmap_q, q_row0, bh, bar(C::kBarQFull + 0));
+          // K_0 first: it has a ring slot of its own, while a stage's Q may be overwritten only once
+          // its last S = Q K^T of the previous item has run. (Queued behind Q, K_0 came up to 3300
+          // cycles after the previous item's last P was ready and held up its P V: 256 keys 33.6 us
+          // that way, 32.1 this; 512 keys 70.2 and 68.4. A thread of its own for Q polled too much.)
           kv_load(&tmap_k, kv_row0, kv_slice);
-          mbar_wait(bar(C::kBarQFree + 1), (item_i & 1u) ^ 1u, wctx, kSiteLoadQFree);
-          mbar_arrive_expect_tx(bar(C::kBarQFull + 1), T::kTileBytes);
-          T::load3(q_smem + T::kTileBytes, &tmap_q, q_row0 + kAttnRows, bh, bar(C::kBarQFull + 1));
+#pragma unroll 1
+          for (int s = 0; s < 2; ++s) {
+            mbar_wait(bar(C::kBarQFree + s), (item_i & 1u) ^ 1u, wctx, kSiteLoadQFree);
+            mbar_arrive_expect_tx(bar(C::kBarQFull + s), T::kTileBytes);
+            T::load3(q_smem + s * T::kTileBytes, &tmap_q, q_row0 + s * kAttnRows, bh, bar(C::kBarQFull + s));
+          }
           for (int j = 0; j < nt1; ++j) {
             FA_TSTAMP(blockIdx.x == 0 && items.on_first(), 3, j, 0);
             kv_load(&tmap_v, kv_row0 + j * kAttnRows, kv_slice);
