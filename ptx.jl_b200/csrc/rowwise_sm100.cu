@@ -259,7 +259,7 @@ int launch_one(const RowParams& p, cudaStream_t stream) {
   // threads per row, and blocks: one per row, or one per four rows
   const int per = kVec + kPark;
   const int threads = kWarpRows ? 128 : ((p.n4 + per - 1) / per + 31) / 32 * 32;
-  const int grid = kWarpRows ? (p.rows + 3) / 4 : p.rows;
+  const int grid = kWarpRows ? (p.rows - 1) / 4 + 1 : p.rows;
   rowwise_kernel<kOp, kWarpRows, kVec, kPark><<<grid, threads, (size_t)kPark * threads * 16, stream>>>(p);
   PTXB200_CUDA_TRY(cudaGetLastError());
   return PTXB200_OK;
