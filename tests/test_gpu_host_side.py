@@ -90,3 +90,22 @@ def test_status_word_is_per_stream(pkg, gpu):
     code = pkg.ops.sync_status()                    # device-wide
     assert code > 0 and "probe" in pkg.native.strerror(code)
     assert pkg.ops.sync_status() == 0 and pkg.ops.sync_status(s_bad) == 0
+
+
+def test_attention_scratch_recycles_beyond_its_capacity(pkg, gpu):
+    """The same with attention launches whose last round is cut, which park pieces in the table's
+    buffers: results stay those of the first launch on twenty streams, twice over."""
+    g = torch.Generator().manual_seed(17)
+    q, k, v = ((torch.randn(1, 2, 1024, 64, generator=g)).to(torch.bfloat16).to(gpu) for _ in range(3))
+    cut = dict(causal=True, flags=pkg.native.FA_ALWAYS_TAIL_SPLIT)
+    want = pkg.ops.fa_fwd(q, k, v, **cut)
+    streams = [torch.cuda.Stream() for _ in range(20)]
+    outs = [torch.empty_like(want) for _ in streams]
+    torch.cuda.synchronize()
+    for _ in range(2):
+        for st, o in zip(streams, outs):
+            pkg.ops.fa_fwd(q, k, v, out=o, stream=st, **cut)
+    torch.cuda.synchronize()
+    assert pkg.ops.sync_status() == 0
+    for o in outs:
+        assert torch.equal(o, want)
