@@ -258,6 +258,12 @@ struct ItemIter {
   __device__ __forceinline__ bool on_first() const { return v == 1; }
 };
 
+// The K/V slice of query head bh: with grouped heads, head h reads key/value head h / (heads_q / heads_kv).
+__device__ __forceinline__ int fa_kv_slice(const FaParams& p, int bh) {
+  const int b = bh / p.heads_q;
+  return b * p.heads_kv + (bh - b * p.heads_q) / (p.heads_q / p.heads_kv);
+}
+
 // Key tiles each stage of the item visits.
 template <bool kCausal>
 __device__ __forceinline__ void tile_counts(const FaParams& p, int mb, int& nt0, int& nt1) {
@@ -638,7 +644,14 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
 
-  if (tid == 0) {
+  // Warp 13's first lane sets up the barriers and sends for the first item's K_0 and Q before
+  // the block meets: the tensor maps' and the loads' latency then runs beside the set-up
+  // of tensor memory (one item per CTA: 2 heads of 512 keys 12.1 us, 11.6 this way; 16 x 4 causal heads
+  // of 512 keys 16.3 and 15.7; one head of 128 keys 6.1 and 5.6).
+  if (tid == 13 * 32) {
+    tma_prefetch_desc(&tmap_k);
+    tma_prefetch_desc(&tmap_q);
+    tma_prefetch_desc(&tmap_v);
     *abort_flag = 0;
     mbar_init(bar(C::kBarQFull + 0), 1);
     mbar_init(bar(C::kBarQFull + 1), 1);
@@ -658,7 +671,21 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
       mbar_init(bar(C::kBarLFree + s), 128);
     }
     mbar_fence_init();
+    if constexpr (!kTail) {
+      WorkIter<kCausal, kTail, kByLen> items;
+      WorkItem w;
+      if (items.next(p, seg_table, w)) {
+        mbar_arrive_expect_tx(bar(C::kBarKvFull), T::kTileBytes);
+        T::load3(kv_smem, &tmap_k, 0, fa_kv_slice(p, w.bh), bar(C::kBarKvFull));
+#pragma unroll 1
+        for (int s = 0; s < 2; ++s) {
+          mbar_arrive_expect_tx(bar(C::kBarQFull + s), T::kTileBytes);
+          T::load3(q_smem + s * T::kTileBytes, &tmap_q, (w.mb * 2 + s) * kAttnRows, w.bh, bar(C::kBarQFull + s));
+        }
+      }
+    }
   }
+  __syncwarp();
   if (warp == 12) {
     tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
     tmem_relinquish();
@@ -678,10 +705,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
     setmaxnreg_dec<kRegsOther>();
     if (warp == 13) {
       if (elect_one()) {
-        tma_prefetch_desc(&tmap_q);
-        tma_prefetch_desc(&tmap_k);
-        tma_prefetch_desc(&tmap_v);
-        uint32_t kv_it = 0, item_i = 0;
+        uint32_t kv_it = kTail ? 0 : 1, item_i = 0;   // the first item's K_0 and Q are on their way
         auto kv_load = [&](const void* tmap, int row, int slice) {
           const uint32_t s = kv_it % C::kSlots;
           const uint32_t ph = (kv_it / C::kSlots) & 1u;
@@ -694,21 +718,20 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
         for (WorkItem w; items.next(p, seg_table, w); ++item_i) {
           const int mb = w.mb, bh = w.bh, nt1 = w.nt[1];
           const int kv_row0 = kTail ? w.j0 * kAttnRows : 0;   // first key tile of this piece of the item
-          // grouped heads: query head h reads key/value head h / (heads_q / heads_kv)
-          const int b_idx = bh / p.heads_q;
-          const int kv_head = (bh - b_idx * p.heads_q) / (p.heads_q / p.heads_kv);
-          const int kv_slice = b_idx * p.heads_kv + kv_head;
+          const int kv_slice = fa_kv_slice(p, bh);
           const int q_row0 = mb * 2 * kAttnRows;   // within the head's sequence; rows past its end load as zeros
           // K_0 first: it has a ring slot of its own, while a stage's Q may be overwritten only once
           // its last S = Q K^T of the previous item has run. (Queued behind Q, K_0 came up to 3300
           // cycles after the previous item's last P was ready and held up its P V: 256 keys 33.6 us
           // that way, 32.1 this; 512 keys 70.2 and 68.4. A thread of its own for Q polled too much.)
-          kv_load(&tmap_k, kv_row0, kv_slice);
+          if (kTail || item_i > 0) {
+            kv_load(&tmap_k, kv_row0, kv_slice);
 #pragma unroll 1
-          for (int s = 0; s < 2; ++s) {
-            mbar_wait(bar(C::kBarQFree + s), (item_i & 1u) ^ 1u, wctx, kSiteLoadQFree);
-            mbar_arrive_expect_tx(bar(C::kBarQFull + s), T::kTileBytes);
-            T::load3(q_smem + s * T::kTileBytes, &tmap_q, q_row0 + s * kAttnRows, bh, bar(C::kBarQFull + s));
+            for (int s = 0; s < 2; ++s) {
+              mbar_wait(bar(C::kBarQFree + s), (item_i & 1u) ^ 1u, wctx, kSiteLoadQFree);
+              mbar_arrive_expect_tx(bar(C::kBarQFull + s), T::kTileBytes);
+              T::load3(q_smem + s * T::kTileBytes, &tmap_q, q_row0 + s * kAttnRows, bh, bar(C::kBarQFull + s));
+            }
           }
           for (int j = 0; j < nt1; ++j) {
             FA_TSTAMP(blockIdx.x == 0 && items.on_first(), 3, j, 0);
