@@ -18,8 +18,8 @@
 //     mask only the diagonal tile, and are handed out longest first within a head;
 //   * the exponentials of a tile are split between two warps and two pipes: the
 //     stage's softmax warp does key columns 0-95 on the MUFU, the correction warp
-//     of the same rows does columns 96-127 with a polynomial on the FMA pipe (0-79 and
-//     80-127 in the head-dim-64 kernel without masking code, where the MUFU binds);
+//     of the same rows does columns 96-127 with a polynomial on the FMA pipe (0-87 and
+//     88-127 in the head-dim-64 kernel without masking code, where the MUFU binds);
 //   * a protocol of mbarrier phases in which no producer can run two phases ahead
 //     of its consumer: within an item each producer's next arrival is downstream of
 //     an MMA issue that waited for the consumer's previous arrival, so no padding
@@ -76,15 +76,17 @@ constexpr int kRegsOther = PTXB200_FA_REGS_OTHER;
 static_assert(256 * kRegsSoftmax + 128 * kRegsCorrection + 128 * kRegsOther <= 65536,
               "register re-split must fit the register file");
 // Head dim 64: the exponential unit is the binding pipe there (one ex2 per score, half the
-// tensor work per score), so the correction warps take 48 instead of 32 of a tile's 128 key
-// columns onto the FMA pipe and get the registers for it. (At head dim 128 the same
-// split measured 2.4 % slower non-causal and spilled in the causal kernel.)
+// tensor work per score), so the correction warps take 40 instead of 32 of a tile's 128 key
+// columns onto the FMA pipe and get the registers for it. With 48 an event log showed them
+// done 320 cycles after the softmax warps and busy for 2200 of a step's 2850: 16 x 16 heads of
+// 2048 keys 372 us with 48, 361 with 40; 512 keys 59.9 and 57.8. (At head dim 128 40 measured
+// 1-2.5 % slower than 32.)
 constexpr int kRegsSoftmax64 = 160, kRegsCorrection64 = 120;
 static_assert(256 * kRegsSoftmax64 + 128 * kRegsCorrection64 + 128 * kRegsOther <= 65536,
               "register re-split must fit the register file");
-// (only in the plain kernel: the causal and the ragged-length kernels measured a quarter to a
-// third slower with it at head dim 64, and the kernels with a cut last round spill with it)
-template <int D, bool kOther> constexpr int kHelperCols = (D == 64 && !kOther) ? 48 : 32;   // key columns per tile on the correction warps
+// (only in the plain kernel: with 40 in the kernels with masks or a cut last round these were
+// 2-13 % slower at either head dim)
+template <int D, bool kOther> constexpr int kHelperCols = (D == 64 && !kOther) ? 40 : 32;   // key columns per tile on the correction warps
 
 // Which of the 16 element pairs of every 32-column chunk take the FMA-pipe
 // polynomial exp2 instead of the MUFU ex2 (bit i = pair i). The MUFU pipe
@@ -754,7 +756,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
     // softmax: warpgroup `stage` owns the 128 rows of that stage; one row
     // per thread, the whole 128-column tile of scores in registers.
     // =====================================================================
-    setmaxnreg_inc<(kHelperCols<D, kCausal || kRagged || kTail> == 48 ? kRegsSoftmax64 : kRegsSoftmax)>();
+    setmaxnreg_inc<(kHelperCols<D, kCausal || kRagged || kTail> == 40 ? kRegsSoftmax64 : kRegsSoftmax)>();
     const int stage = warp >> 2;
     const int row = tid & 127;
     const uint32_t t_row = tmem_addr(tmem, (warp & 3) * 32, C::kColS + stage * 128);
@@ -838,17 +840,17 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
           // batches of kBatch pairs: all scaled inputs, then all exponentials back to
           // back (so the MUFU latency of one is hidden behind the issue of the next),
           // then the sums and the bf16 packing
-          constexpr int kPairsLast = (128 - kHelperCols<D, kCausal || kRagged || kTail> - 64) / 2;   // pairs of the third chunk: 16, or 8 at D = 64
+          constexpr int kPairsLast = (128 - kHelperCols<D, kCausal || kRagged || kTail> - 64) / 2;   // pairs of the third chunk: 16, or 12 at D = 64
 #pragma unroll
           for (int b = 0; b < 16; b += kBatch) {
-            if (c == 2 && b >= kPairsLast) break;
+            const int n = c == 2 && b + kBatch > kPairsLast ? kPairsLast - b : kBatch;   // the last batch may be a half
             float2 x[kBatch], e[kBatch];
 #pragma unroll
-            for (int i = 0; i < kBatch; ++i)
+            for (int i = 0; i < n; ++i)
               x[i] = __ffma2_rn(make_float2(__uint_as_float(v[c][2 * (b + i)]),
                                             __uint_as_float(v[c][2 * (b + i) + 1])), scale2, neg2);
 #pragma unroll
-            for (int i = 0; i < kBatch; ++i) {
+            for (int i = 0; i < n; ++i) {
               if ((kEmuMask >> (b + i)) & 1u) {
                 e[i] = exp2_poly2(x[i]);
               } else {
@@ -857,16 +859,17 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
               }
             }
 #pragma unroll
-            for (int i = 0; i < kBatch; ++i) {
+            for (int i = 0; i < n; ++i) {
               sum2[i & 1] = __fadd2_rn(sum2[i & 1], e[i]);
               pk[b + i] = pack_bf16x2(e[i].x, e[i].y);
             }
           }
-          if (c == 2 && kPairsLast == 8) {
+          if (c == 2 && kPairsLast == 12) {
             uint32_t pk8[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) pk8[i] = pk[i];
             tmem_st8(t_row + 32, pk8);
+            tmem_st4(t_row + 40, pk[8], pk[9], pk[10], pk[11]);
           } else {
             tmem_st16(t_row + c * 16, pk);
           }
@@ -895,7 +898,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
     // =====================================================================
     // 104 registers is below the 128 the kernel launches with: a release, like the
     // MMA/load warpgroup's, that the two softmax warpgroups' increase draws on
-    setmaxnreg_dec<(kHelperCols<D, kCausal || kRagged || kTail> == 48 ? kRegsCorrection64 : kRegsCorrection)>();
+    setmaxnreg_dec<(kHelperCols<D, kCausal || kRagged || kTail> == 40 ? kRegsCorrection64 : kRegsCorrection)>();
     const int row = tid & 127;
     const uint32_t t_lane = tmem_addr(tmem, (warp & 3) * 32, 0);
     mbar_arrive(bar(C::kBarPFull + 0));   // O is free for the first item
@@ -923,7 +926,8 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
           const int cur = kStageUnroll == 1 ? 0 : s;
           if (j < (s == 0 ? nt[0] : nt[1])) {
             uint32_t sv[32];
-            [[maybe_unused]] uint32_t sw[16];   // head dim 64: key columns 80..95 as well
+            constexpr bool kExtra = kHelperCols<D, kCausal || kRagged || kTail> == 40;
+            [[maybe_unused]] uint32_t sw[8];   // head dim 64: key columns 88..95 as well
             // Only a stage's last tile can hold masked keys: those above the diagonal
             // (causal) or past the end of the sequence (non-causal, S % 128 != 0). `keep`
             // is the last key column this row keeps there.
@@ -936,9 +940,9 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
               mbar_wait(bar(C::kBarSFull + s), cnt_h[cur] & 1u, wctx, kSiteSoftmaxSFull);
               ++cnt_h[cur];
               tc_fence_after();
-              if (kHelperCols<D, kCausal || kRagged || kTail> == 48) tmem_ld16(t_lane + C::kColS + s * 128 + 80, sw);
+              if (kExtra) tmem_ld8(t_lane + C::kColS + s * 128 + 88, sw);
               tmem_ld32(t_lane + C::kColS + s * 128 + 96, sv);
-              if (kHelperCols<D, kCausal || kRagged || kTail> == 48) tc_wait_ld_bind16(sw);
+              if (kExtra) tc_wait_ld_bind8(sw);
               tc_wait_ld_bind(sv);
             }
             mbar_wait(bar(C::kBarAlpha + s), cnt_a[cur] & 1u, wctx, kSiteCorrAlpha);
@@ -970,14 +974,14 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
               const float2 neg2 = make_float2(neg, neg);
               float2 sum2 = make_float2(0.0f, 0.0f);
               uint32_t pk[16];
-              [[maybe_unused]] uint32_t pk8[8];
-              if (kHelperCols<D, kCausal || kRagged || kTail> == 48) {   // (a kernel without masks)
+              [[maybe_unused]] uint32_t pk4[4];
+              if (kExtra) {   // (a kernel without masks)
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
+                for (int i = 0; i < 4; ++i) {
                   const float2 e = exp2_poly2(__ffma2_rn(
                       make_float2(__uint_as_float(sw[2 * i]), __uint_as_float(sw[2 * i + 1])), scale2, neg2));
                   sum2 = __fadd2_rn(sum2, e);
-                  pk8[i] = pack_bf16x2(e.x, e.y);
+                  pk4[i] = pack_bf16x2(e.x, e.y);
                 }
               }
               // masked keys: -inf, which the polynomial takes to 2^-126 (nothing beside a row
@@ -1001,7 +1005,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
                   else if (96 + 2 * i + 1 > keep) pk[i] &= 0xFFFFu;
                 }
               }
-              if (kHelperCols<D, kCausal || kRagged || kTail> == 48) tmem_st8(t_lane + C::kColS + s * 128 + 40, pk8);   // P columns of keys 80..95
+              if (kExtra) tmem_st4(t_lane + C::kColS + s * 128 + 44, pk4[0], pk4[1], pk4[2], pk4[3]);   // P columns of keys 88..95
               tmem_st16(t_lane + C::kColS + s * 128 + 48, pk);   // P columns of keys 96..127
               tc_wait_st();
               tc_fence_before();
@@ -1533,8 +1537,8 @@ int launch_fa_fwd(const DeviceCtx& ctx, void* O, void* lse, const void* Q, const
 // or -1 if `cap` is too small.
 int describe_fa_plan(int BH, int S, int causal, unsigned flags, int sm_count, int* out, int cap) {
   const int nmb = (S + 255) / 256, nt_all = (S + kAttnRows - 1) / kAttnRows;
-  // as for head dim 128 with a K/V head per query head
-  const FaSched sc = plan_schedule(BH, nmb, nt_all, causal, flags, sm_count, true, 4ll * BH * S * 128);
+  // neither head dim nor K/V heads are known here: as for K and V too large for the order by length
+  const FaSched sc = plan_schedule(BH, nmb, nt_all, causal, flags, sm_count, true, kByLengthMaxKvBytes + 1);
   int n = 0;
   auto put = [&](int v) {
     if (n < cap) out[n] = v;
