@@ -13,8 +13,8 @@
 // fixed, so results are reproducible (they differ in the last bits from the unsplit order).
 // One-shot blocks: the first loads are issued before the block's threads even meet.
 //
-// With fp32 output a CTA sums its part of K in up to 8 (64 columns) or 4 (128) chains of at
-// least 8 steps, one accumulator in tensor memory each, and adds them up in the epilogue: the
+// With fp32 output a CTA sums its part of K in chains of at most 8 steps, up to 8 chains (64
+// columns) or 4 (128), one accumulator in tensor memory each, and adds them up in the epilogue: the
 // tensor core's fp32 accumulation loses about 3e-8 of the result per step of a chain, so
 // one chain over 64 steps (1024x1152x8192 split in 2) is off by 4.0e-6, four of 16 steps by
 // 8.5e-7 (the 35-step shares of the schedule before: 1.9e-6). bf16 output rounds 1.7e-3.
@@ -40,7 +40,7 @@ constexpr int kMaxStages3 = 7;
 constexpr int kSmemMax3 = 232448;
 constexpr int kABytes3 = kBM3 * kBK3 * 2;
 constexpr int kBandM3 = 8;            // row-tiles per rasterisation band
-constexpr int kChainSteps3 = 8;       // least steps of K per accumulator with fp32 output
+constexpr int kChainSteps3 = 8;       // steps of K per accumulator with fp32 output, more only where accumulators run out
 // full[], empty[], acc_full, parts_in, TMEM slot, abort flag
 constexpr int kCtrlBytes3 = ((2 * kMaxStages3 + 2) * 8 + 8 + 15) / 16 * 16;
 static_assert(kCtrlBytes3 % 16 == 0, "the parts handed over behind it are 16-byte pieces");
@@ -303,10 +303,9 @@ int launch_one3(const DeviceCtx& ctx, int split, void* C, const void* A, const v
   int stages = (kSmemMax3 - kCtrlBytes3 - recv) / stage_bytes3(kBN);
   if (stages > kMaxStages3) stages = kMaxStages3;
   if (stages > steps) stages = steps;
-  // chains of at least kChainSteps3 steps, as many accumulators as tensor memory holds
-  int chains = one_chain || !kF32Out ? 1 : steps * stage_k3(kBN) / kChainSteps3;
+  // chains of at most kChainSteps3 steps, as far as tensor memory holds accumulators
+  int chains = one_chain || !kF32Out ? 1 : (steps * stage_k3(kBN) + kChainSteps3 - 1) / kChainSteps3;
   if (chains > 512 / kBN) chains = 512 / kBN;
-  if (chains < 1) chains = 1;
   const int chain_stages = (steps + chains - 1) / chains;
   uint32_t tmem_cols = kBN;
   while (tmem_cols < (uint32_t)(chains * kBN)) tmem_cols *= 2;
