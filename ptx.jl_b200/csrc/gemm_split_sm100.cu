@@ -250,6 +250,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             st_async_v4(dst + (c / 4 + j) * (kBM3 * 16), dst_bar, x[4 * j], x[4 * j + 1], x[4 * j + 2], x[4 * j + 3]);
         }
       }
+    }
+    // "this CTA stores nothing more into its peers": waited for before any of them leaves
+    __syncwarp();
+    cluster_arrive();
+    if (epilogue) {
       mbar_wait(bar_parts, 0, wctx, kSite3Parts);
 #pragma unroll 1
       for (int c = 0; c < width; c += 16) {
@@ -279,6 +284,17 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   if (warp == 1 && !misaligned) {
     tc_fence_after();
     tmem_dealloc(tmem, tmem_cols);
+  }
+  // A CTA whose wait for the parts ran out gets here while a peer may still be sending, and storing
+  // into a CTA that has left is a fault: it stays until every peer has issued its stores and
+  // these have landed. (Where no wait ran out both have happened by now.)
+  if (split > 1) {
+    __syncwarp();
+    cluster_wait();
+    if (threadIdx.x == 0 && !misaligned && !mbar_try_wait(bar_parts, 0)) {
+      const uint64_t t0 = globaltimer_ns();
+      while (!mbar_try_wait(bar_parts, 0) && globaltimer_ns() - t0 < kWaitLimitNs) {}
+    }
   }
 }
 

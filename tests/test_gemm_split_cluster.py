@@ -1,0 +1,27 @@
+"""What the clusters of gemm_split_sm100.cu owe each other, read from the kernel's source: a
+cluster whose waits run out cannot be brought about on a GPU without risking a fault."""
+import os
+import re
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+def kernel_body():
+    with open(os.path.join(ROOT, "ptx.jl_b200", "csrc", "gemm_split_sm100.cu")) as f:
+        text = re.sub(r"//[^\n]*", "", f.read())
+    start = text.index("gemm_split_kernel(")
+    return text[start:text.index("\n}\n", start)]
+
+
+def test_no_cta_leaves_before_its_peers_stop_storing_into_it():
+    """The cluster barrier's second phase: every CTA arrives behind its last store into a
+    peer and ahead of its wait for the parts, and waits behind everything else it does."""
+    body = kernel_body()
+    at = lambda token: [m.start() for m in re.finditer(re.escape(token), body)]
+    arrive, wait, store = at("cluster_arrive()"), at("cluster_wait()"), at("st_async_v4(")
+    assert len(arrive) == 2 and len(wait) == 2 and len(store) == 1
+    assert arrive[0] < wait[0] < store[0] < arrive[1] < at("kSite3Parts")[0]
+    assert wait[1] > max(at("__syncthreads()")[-1], at("tmem_dealloc(")[-1], at("store_acc_chunk16")[-1])
+    # stores are asynchronous: a peer that has issued them may still have them on the way
+    assert at("mbar_try_wait(bar_parts")[0] > wait[1]
+    assert "return" not in body          # no way past the closing wait
