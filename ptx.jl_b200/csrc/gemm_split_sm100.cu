@@ -255,7 +255,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     __syncwarp();
     cluster_arrive();
     if (epilogue) {
-      mbar_wait(bar_parts, 0, wctx, kSite3Parts);
+      mbar_wait<true>(bar_parts, 0, wctx, kSite3Parts);   // other CTAs' stores are read behind it
 #pragma unroll 1
       for (int c = 0; c < width; c += 16) {
         float own[16], sum[16];

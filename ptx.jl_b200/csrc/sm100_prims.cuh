@@ -136,15 +136,27 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t byt
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                : "memory");
 }
+// kCluster: the wait also orders this thread behind what other CTAs of the cluster stored
+// ahead of completing the phase (without it the wait's scope is this CTA).
+template <bool kCluster = false>
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
+  if constexpr (kCluster)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
   return ok != 0;
 }
 
@@ -154,12 +166,13 @@ constexpr uint64_t kWaitLimitNs = 1500ull * 1000ull * 1000ull;
 
 // Bounded wait on phase `parity`. Returns true on completion, false if the wait
 // ran out (or the CTA was already aborting); callers carry on either way.
+template <bool kCluster = false>
 __device__ __forceinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, const WaitCtx& ctx,
                                             uint32_t site) {
   const uint64_t t0 = globaltimer_ns();
   uint32_t spins = 0;
   while (true) {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (mbar_try_wait<kCluster>(bar, parity)) return true;
     if (*ctx.abort != 0) return false;
     if ((++spins & 63u) == 0 && globaltimer_ns() - t0 > kWaitLimitNs) {
       *ctx.abort = 1;
@@ -170,10 +183,11 @@ __device__ __forceinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, co
     }
   }
 }
+template <bool kCluster = false>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const WaitCtx& ctx,
                                           uint32_t site) {
-  if (mbar_try_wait(bar, parity)) return true;   // already complete: the common case on hot paths
-  return mbar_wait_slow(bar, parity, ctx, site);
+  if (mbar_try_wait<kCluster>(bar, parity)) return true;   // already complete: the common case on hot paths
+  return mbar_wait_slow<kCluster>(bar, parity, ctx, site);
 }
 
 // ---------------------------------------------------------------------------

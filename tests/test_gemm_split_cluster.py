@@ -25,3 +25,17 @@ def test_no_cta_leaves_before_its_peers_stop_storing_into_it():
     # stores are asynchronous: a peer that has issued them may still have them on the way
     assert at("mbar_try_wait(bar_parts")[0] > wait[1]
     assert "return" not in body          # no way past the closing wait
+
+
+def test_the_wait_for_the_parts_acquires_at_cluster_scope():
+    """Other CTAs store the parts, so a wait of this CTA's scope (the default) orders nothing."""
+    assert "mbar_wait<true>(bar_parts" in kernel_body()
+    with open(os.path.join(ROOT, "ptx.jl_b200", "csrc", "sm100_prims.cuh")) as f:
+        prims = f.read()
+    wait = prims[prims.index("bool mbar_try_wait("):]
+    wait = wait[:wait.index("return ok")]
+    assert "if constexpr (kCluster)" in wait and "mbarrier.try_wait.parity.acquire.cluster.shared::cta" in wait
+    for caller in ("bool mbar_wait_slow(", "bool mbar_wait("):
+        body = prims[prims.index(caller):]
+        body = body[:body.index("\n}\n")]
+        assert "mbar_try_wait<kCluster>" in body and "mbar_try_wait(" not in body
