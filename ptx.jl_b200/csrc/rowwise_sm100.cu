@@ -28,8 +28,8 @@
 //   * X and Y are accessed with the streaming cache hints (read once, written once), the
 //     weight vectors through the read-only path;
 //   * softmax merges (max, sum of exponentials) pairs by the online-softmax rule and
-//     rescales once; layer norm takes the mean, then the centred sum of squares of the
-//     values on chip, which keeps its accuracy for rows with a large mean, where the
+//     rescales once; layer norm takes the mean, then the centred sums of the values on chip and
+//     of their squares, which keeps its accuracy for rows with a large mean, where the
 //     reference's E[x^2] - mean^2 cancels. With several warps per row a reduction costs one
 //     block barrier.
 #include "host_common.h"
@@ -53,7 +53,7 @@ struct RowParams {
   float eps;
 };
 
-// Reductions over the threads that share a row: a sum, or a (max, sum of exponentials)
+// Reductions over the threads that share a row: a sum, two sums, or a (max, sum of exponentials)
 // pair merged with the online-softmax rule. With more than one warp per row the warps'
 // partials meet in shared memory behind ONE block barrier: the buffer alternates between
 // two from reduction to reduction, so a warp writing the next partials cannot overrun a
@@ -68,10 +68,14 @@ __device__ __forceinline__ Pair merge(Pair a, Pair b) {
   return {m, a.s * fa + b.s * fb};
 }
 __device__ __forceinline__ float merge(float a, float b) { return a + b; }
+struct Sums { float a, b; };
+__device__ __forceinline__ Sums merge(Sums x, Sums y) { return {x.a + y.a, x.b + y.b}; }
 
 __device__ __forceinline__ float shfl_xor(float v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
 __device__ __forceinline__ Pair shfl_xor(Pair v, int o) { return {shfl_xor(v.m, o), shfl_xor(v.s, o)}; }
+__device__ __forceinline__ Sums shfl_xor(Sums v, int o) { return {shfl_xor(v.a, o), shfl_xor(v.b, o)}; }
 __device__ __forceinline__ float identity(float) { return 0.0f; }
+__device__ __forceinline__ Sums identity(Sums) { return {0.0f, 0.0f}; }
 __device__ __forceinline__ Pair identity(Pair) { return {-INFINITY, 0.0f}; }
 
 template <typename T>
@@ -159,7 +163,8 @@ rowwise_kernel(const RowParams p) {
     }
   };
 
-  float mul;   // what the row's (centred, exponentiated) values are scaled by
+  float mul;   // what the row's (centred, exponentiated) values are scaled by,
+  [[maybe_unused]] float add;   // and layer norm: what is added then
   if constexpr (kOp == kOpSoftmax) {
     float m = -INFINITY;
     each([&](float4& x, int) { m = fmaxf(fmaxf(m, fmaxf(x.x, x.y)), fmaxf(x.z, x.w)); });
@@ -180,21 +185,36 @@ rowwise_kernel(const RowParams p) {
     each([&](float4& x, int) { s += (x.x * x.x + x.y * x.y) + (x.z * x.z + x.w * x.w); });
     mul = rsqrtf(reduce(s) * p.inv_n + p.eps);
   } else {
+    // The mean is a sum in fp32 and off by its rounding, up to a few 1e-7 of itself. The mean of
+    // the centred values is that error: it is taken off the values and, squared, off their mean
+    // square. Rows around 1000 with unit spread: error 5.5e-5 without, 6e-8 with it; rows of one
+    // value give zeros. (Each thread's sum is scaled ahead of the reduction, which then cannot
+    // overflow where the mean does not.)
     float s = 0.0f;
     each([&](float4& x, int) { s += (x.x + x.y) + (x.z + x.w); });   // padding lanes hold zeros
-    const float mean = reduce(s) * p.inv_n;
-    float q = 0.0f;
+    const float mean = reduce(s * p.inv_n);
+    Sums d = {0.0f, 0.0f};
     each([&](float4& x, int c) {
       if (c < p.n4) {
         x.x -= mean; x.y -= mean; x.z -= mean; x.w -= mean;
-        q += (x.x * x.x + x.y * x.y) + (x.z * x.z + x.w * x.w);
+        d.a += (x.x + x.y) + (x.z + x.w);
+        d.b += (x.x * x.x + x.y * x.y) + (x.z * x.z + x.w * x.w);
       }
     });
-    mul = rsqrtf(reduce(q) * p.inv_n + p.eps);
+    d = reduce(d);
+    const float off = d.a * p.inv_n;
+    float var = d.b * p.inv_n;
+    if (var < INFINITY) var = fmaxf(fmaf(-off, off, var), 0.0f);   // two rounded values: may cross zero (NaN: left alone)
+    mul = rsqrtf(var + p.eps);
+    add = -off * mul;
   }
 
   auto write = [&](const float4& x, int c, const float4* early_w, const float4* early_b) {
-    float4 o = make_float4(x.x * mul, x.y * mul, x.z * mul, x.w * mul);
+    float4 o;
+    if constexpr (kOp == kOpLayerNorm)
+      o = make_float4(fmaf(x.x, mul, add), fmaf(x.y, mul, add), fmaf(x.z, mul, add), fmaf(x.w, mul, add));
+    else
+      o = make_float4(x.x * mul, x.y * mul, x.z * mul, x.w * mul);
     if constexpr (kOp != kOpSoftmax) {
       const float4 wi = early_w != nullptr ? *early_w : __ldg(w4 + c);
       if constexpr (kOp == kOpRmsNorm) {

@@ -63,6 +63,32 @@ def test_layer_norm_large_mean(pkg, gpu, oracle_mod):
     np.testing.assert_allclose(Y.numpy(), ref, atol=5e-3, rtol=5e-3)   # fp32 input spacing at 300 is 3e-5 of a 0.05 spread
 
 
+@pytest.mark.parametrize("rows,N,mean", [(5, 36, 1000.0), (64, 1000, 1000.0), (64, 3000, 1000.0), (300, 2048, -30.0),
+                                         (300, 8196, 100.0), (3, 12000, 1000.0), (3, 30000, 1e5), (2, 32768, 1e5)])
+def test_layer_norm_takes_off_the_rounding_of_the_mean(pkg, gpu, rows, N, mean):
+    """Rows far from zero: the fp32 mean is off by up to a few 2^-24 of itself, which must not
+    reach the centred values. Rows of one value: zeros, whatever the value and the length."""
+    g = torch.Generator(device=gpu).manual_seed(N)
+    X = torch.randn(rows, N, generator=g, device=gpu) + mean
+    W, Bias = torch.ones(N, device=gpu), torch.zeros(N, device=gpu)
+    D = X.double()
+    C = D - D.mean(dim=1, keepdim=True)
+    want = C * torch.rsqrt(C.square().mean(dim=1, keepdim=True) + 1e-5)
+    got = pkg.ops.layer_norm(X, W, Bias).double()
+    # a centred value: exact (Sterbenz) or one rounding of at most |x - mean| 2^-24, the mean of
+    # the centred values, the mean square (log2 N roundings and its own), rsqrt, two products:
+    # under 32 roundings of values up to 6
+    assert float((got - want).abs().max()) < 32 * 6 * 2.0 ** -24
+    same = torch.full((rows, N), mean + 0.1, device=gpu)
+    assert float(pkg.ops.layer_norm(same, W, Bias).abs().max()) < 1e-4
+    # a row's sum may overflow where its mean does not; the squares do, so the row scales to nothing
+    huge = torch.where(torch.rand(rows, N, generator=g, device=gpu) < 0.9, 1e36, -1e36)
+    assert float(pkg.ops.layer_norm(huge, W, Bias).abs().max()) == 0.0
+    X[0, 3] = float("nan")
+    assert bool(torch.isnan(pkg.ops.layer_norm(X, W, Bias)[0]).all())
+    assert pkg.ops.sync_status() == 0
+
+
 def test_rowwise_properties_at_full_size(pkg, gpu):
     """1 GiB in, 1 GiB out per call: softmax rows sum to one and do not move under a
     row shift; RMS norm is invariant to a positive row scale; layer norm output has
