@@ -16,15 +16,15 @@
 //     blocks falls into step (all read, then all write): rows of 8192 columns, 0.5 GB in,
 //     0.5 GB out, softmax 171 us persistent, 156 us this way (6880 GB/s); rows of 1024
 //     columns 91 against 80 us; and a ring in shared memory kept full by bulk copies 170 to 203;
-//   * the threads per row follow its length, eight float4s each (any N that is a multiple
-//     of 4: the last ones are guarded), in steps of a warp: rows of 9000 columns took 300 us
-//     on a power-of-two block that they half filled, and take 157;
+//   * the threads per row follow its length, eight float4s each or four (any N that is a
+//     multiple of 4: the last ones are guarded), in steps of a warp: rows of 9000 columns took
+//     300 us on a power-of-two block that they half filled, and take 157;
 //   * above 16384 columns a thread holds eight float4s in registers and up to eight in
 //     shared memory, so that two blocks still fit an SM's register file and overlap
 //     (softmax, 30000 columns: 197 us with the whole row in registers, 169 now);
 //   * few rows (at most two per SM, up to 4096 columns) are spread over four times the
 //     threads, and the weights are fetched ahead of the reduction: latency counts there (16
-//     rows of 2048 columns, layer norm: 4.2 us, now 2.1);
+//     rows of 2048 columns, layer norm: 4.2 us, now 2.1); long ones over 1024 threads;
 //   * X and Y are accessed with the streaming cache hints (read once, written once), the
 //     weight vectors through the read-only path;
 //   * softmax merges (max, sum of exponentials) pairs by the online-softmax rule and
@@ -94,9 +94,9 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // One row per block (kWarpRows = false: all threads of the block share it) or per warp
 // (kWarpRows = true, four rows per block). A thread holds the row's float4s t, t + T, ...
 // (T threads per row): the first kVec of them in registers, kPark more in shared memory
-// slots that no other thread touches.
-template <int kOp, bool kWarpRows, int kVec, int kPark>
-__global__ void __launch_bounds__(kWarpRows ? 128 : 512, kWarpRows ? 1 : 2)
+// slots that no other thread touches. Blocks have up to kMaxT threads, kMinBlocks of them fit an SM.
+template <int kOp, bool kWarpRows, int kVec, int kPark, int kMaxT, int kMinBlocks>
+__global__ void __launch_bounds__(kMaxT, kMinBlocks)
 rowwise_kernel(const RowParams p) {
   __shared__ float2 red[2][32];
   extern __shared__ __align__(16) float4 parked[];   // [kPark][T]
@@ -274,41 +274,68 @@ swiglu_kernel(float* __restrict__ out, const float* __restrict__ gate, const flo
   }
 }
 
-template <int kOp, bool kWarpRows, int kVec, int kPark = 0>
-int launch_one(const RowParams& p, cudaStream_t stream) {
-  // threads per row, and blocks: one per row, or one per four rows
-  const int per = kVec + kPark;
-  const int threads = kWarpRows ? 128 : ((p.n4 + per - 1) / per + 31) / 32 * 32;
-  const int grid = kWarpRows ? (p.rows - 1) / 4 + 1 : p.rows;
-  rowwise_kernel<kOp, kWarpRows, kVec, kPark><<<grid, threads, (size_t)kPark * threads * 16, stream>>>(p);
+template <int kOp, int kVec>
+int launch_warp_rows(const RowParams& p, cudaStream_t stream) {
+  rowwise_kernel<kOp, true, kVec, 0, 128, 1><<<(p.rows - 1) / 4 + 1, 128, 0, stream>>>(p);
   PTXB200_CUDA_TRY(cudaGetLastError());
   return PTXB200_OK;
 }
 
+// A block per row, of as many threads as the row needs, in steps of a warp.
+template <int kOp, int kVec, int kMaxT, int kMinBlocks, int kPark = 0>
+int launch_block_rows(const RowParams& p, cudaStream_t stream) {
+  constexpr int per = kVec + kPark;
+  const int threads = kMaxT == 1024 ? 1024 : ((p.n4 + per - 1) / per + 31) / 32 * 32;
+  rowwise_kernel<kOp, false, kVec, kPark, kMaxT, kMinBlocks>
+      <<<p.rows, threads, (size_t)kPark * threads * 16, stream>>>(p);
+  PTXB200_CUDA_TRY(cudaGetLastError());
+  return PTXB200_OK;
+}
+
+// The lines lie where measured device times cross (inputs beyond L2); the norms, which fetch
+// weights behind their reduction, want more threads per row than softmax.
 template <int kOp>
 int dispatch(const DeviceCtx& ctx, const RowParams& p, cudaStream_t stream) {
   const int n4 = p.n4;
+  constexpr bool kNorm = kOp != kOpSoftmax;
   // At most two rows per SM: nothing overlaps, so a row's own latency is the launch's. 200 rows
   // of 2048 columns: 2.3 us against 2.6 with a warp per row (layer norm 2.4 against 4.4); above
   // 4096 columns the shorter chain per thread no longer pays (200 rows of 8192: 5.2 against 4.4).
-  if (p.rows <= 2 * ctx.sm_count && n4 > 128 && n4 <= 2 * 512) return launch_one<kOp, false, 2>(p, stream);
-  if (n4 <= 32 * 16) {
-    const int per = (n4 + 31) / 32;
-    if (per <= 1) return launch_one<kOp, true, 1>(p, stream);
-    if (per <= 2) return launch_one<kOp, true, 2>(p, stream);
-    if (per <= 4) return launch_one<kOp, true, 4>(p, stream);
-    if (per <= 8) return launch_one<kOp, true, 8>(p, stream);
-    return launch_one<kOp, true, 16>(p, stream);
+  // Norms of 512 to 1024 columns up to eight rows per SM: layer norm, 1000 x 512 2.68 against
+  // 3.11 with a warp per row, RMS norm, 600 x 1024 2.39 against 2.86.
+  const bool few = p.rows <= 2 * ctx.sm_count;
+  if (n4 <= 1024 && (few ? n4 >= (kNorm ? 128 : 129) : kNorm && n4 >= 128 && n4 <= 256 && p.rows <= 8 * ctx.sm_count))
+    return launch_block_rows<kOp, 2, 512, 2>(p, stream);
+  // At most one long row per SM: all of an SM's threads on it (148 x 20000, RMS norm: 5.9 us
+  // against 7.0 with half in shared memory, layer norm 7.2 and 8.6, softmax 6.3 and 7.3).
+  if (p.rows <= ctx.sm_count) {
+    if (n4 > 4096) return launch_block_rows<kOp, 8, 1024, 1>(p, stream);
+    if constexpr (kOp == kOpRmsNorm)
+      if (n4 > 2048) return launch_block_rows<kOp, 4, 1024, 1>(p, stream);   // 148 x 12000: 4.4 against 4.9
   }
-  if (n4 <= 8 * 512) return launch_one<kOp, false, 8>(p, stream);
+  // A warp per row; not for norms above 1024 columns (layer norm, 4000 x 2048: 14.5 us against
+  // 12.0 on a block per row).
+  if (n4 <= (kNorm ? 256 : 512)) {
+    const int per = (n4 + 31) / 32;
+    if (per <= 1) return launch_warp_rows<kOp, 1>(p, stream);
+    if (per <= 2) return launch_warp_rows<kOp, 2>(p, stream);
+    if (per <= 4) return launch_warp_rows<kOp, 4>(p, stream);
+    if (kNorm || per <= 8) return launch_warp_rows<kOp, 8>(p, stream);
+    if constexpr (!kNorm) return launch_warp_rows<kOp, 16>(p, stream);
+  }
+  // Four float4s per thread keep more rows in flight: RMS norm, 2000 x 4096 12.2 us with eight and
+  // 11.5, 600 x 8192 9.1 and 8.5; layer norm, 4000 x 3000 17.3 and 16.8, but 2000 x 8192 23.0 and 24.2.
+  if constexpr (kNorm)
+    if (n4 <= (kOp == kOpRmsNorm || few ? 2048 : 1024)) return launch_block_rows<kOp, 4, 512, 3>(p, stream);
+  if (n4 <= 8 * 512) return launch_block_rows<kOp, 8, 512, 2>(p, stream);
   static PerDeviceOnce attr_once;
   const int rc = attr_once.run(ctx.device, []() -> int {
-    PTXB200_CUDA_TRY(cudaFuncSetAttribute(rowwise_kernel<kOp, false, 8, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          512 * 8 * 16));
+    PTXB200_CUDA_TRY(cudaFuncSetAttribute(rowwise_kernel<kOp, false, 8, 8, 512, 2>,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, 512 * 8 * 16));
     return PTXB200_OK;
   });
   if (rc != PTXB200_OK) return rc;
-  return launch_one<kOp, false, 8, 8>(p, stream);
+  return launch_block_rows<kOp, 8, 512, 2, 8>(p, stream);
 }
 
 }  // namespace

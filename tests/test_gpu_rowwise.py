@@ -124,7 +124,13 @@ def test_rowwise_properties_at_full_size(pkg, gpu):
 # few rows (two per SM: 296 on 148 SMs; N = 512 and 4096), float4s in shared memory (N = 16384)
 # and a last float4 of the row in each of a thread's places.
 @pytest.mark.parametrize("rows,N", [(5, 512), (5, 516), (296, 2048), (297, 2048), (297, 2052), (296, 4096), (296, 4100),
-                                    (300, 4096), (3, 16384), (3, 16388), (300, 16388), (2, 28676), (2, 32764), (150, 32768)])
+                                    (300, 4096), (3, 16384), (3, 16388), (300, 16388), (2, 28676), (2, 32764), (150, 32768),
+                                    # norms: 512 and 1024 columns up to eight rows per SM (1184), a warp per row up to
+                                    # 1024 columns, four float4s per thread up to 4096 or 8192; all: 1024 threads on at
+                                    # most one long row per SM (148)
+                                    (297, 508), (297, 512), (1184, 1024), (1185, 1024), (297, 1028), (297, 4100), (297, 8192),
+                                    (297, 8196), (296, 8192), (148, 8196), (149, 8196), (148, 16384), (149, 16384),
+                                    (148, 16388), (149, 16388), (148, 32768)])
 def test_rowwise_edges_against_64_bit(pkg, gpu, rows, N):
     g = torch.Generator(device=gpu).manual_seed(rows * 31 + N)
     X = torch.randn(rows, N, generator=g, device=gpu)
