@@ -251,9 +251,6 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         }
       }
     }
-    // "this CTA stores nothing more into its peers": waited for before any of them leaves
-    __syncwarp();
-    cluster_arrive();
     if (epilogue) {
       mbar_wait<true>(bar_parts, 0, wctx, kSite3Parts);   // other CTAs' stores are read behind it
 #pragma unroll 1
@@ -285,13 +282,14 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     tc_fence_after();
     tmem_dealloc(tmem, tmem_cols);
   }
-  // A CTA whose wait for the parts ran out gets here while a peer may still be sending, and storing
-  // into a CTA that has left is a fault: it stays until every peer has issued its stores and
-  // these have landed. (Where no wait ran out both have happened by now.)
-  if (split > 1) {
-    __syncwarp();
-    cluster_wait();
-    if (threadIdx.x == 0 && !misaligned && !mbar_try_wait(bar_parts, 0)) {
+  // A CTA in which a wait ran out gets here while peers may still be sending, and storing into a
+  // CTA that has left is a fault: it stays until every peer has left or stays as well, and these
+  // have all issued their stores, and until the stores have landed. (Otherwise it has received
+  // all parts and nobody stores into it any more. A barrier in every launch costs 0.5 us.)
+  if (split > 1 && !misaligned && *abort_flag != 0) {
+    cluster_arrive();
+    cluster_wait();   // for all threads of the cluster that have not left
+    if (threadIdx.x == 0 && !mbar_try_wait(bar_parts, 0)) {
       const uint64_t t0 = globaltimer_ns();
       while (!mbar_try_wait(bar_parts, 0) && globaltimer_ns() - t0 < kWaitLimitNs) {}
     }

@@ -14,15 +14,17 @@ def kernel_body():
 
 
 def test_no_cta_leaves_before_its_peers_stop_storing_into_it():
-    """The cluster barrier's second phase: every CTA arrives behind its last store into a
-    peer and ahead of its wait for the parts, and waits behind everything else it does."""
+    """A CTA leaves when it has received everything its peers send it; if one of its waits ran
+    out (its abort flag is up), only behind a cluster barrier that every peer reaches or leaves
+    behind its last store, and behind the landing of the stores, which are asynchronous."""
     body = kernel_body()
     at = lambda token: [m.start() for m in re.finditer(re.escape(token), body)]
     arrive, wait, store = at("cluster_arrive()"), at("cluster_wait()"), at("st_async_v4(")
     assert len(arrive) == 2 and len(wait) == 2 and len(store) == 1
-    assert arrive[0] < wait[0] < store[0] < arrive[1] < at("kSite3Parts")[0]
+    assert arrive[0] < wait[0] < store[0] < at("mbar_wait<true>(bar_parts")[0] < arrive[1] < wait[1]
     assert wait[1] > max(at("__syncthreads()")[-1], at("tmem_dealloc(")[-1], at("store_acc_chunk16")[-1])
-    # stores are asynchronous: a peer that has issued them may still have them on the way
+    closing = body[at("__syncthreads()")[-1]:]
+    assert re.search(r"if \((kSplit|split > 1) && !misaligned && \*abort_flag != 0\) \{\s*cluster_arrive\(\);\s*cluster_wait\(\);", closing)
     assert at("mbar_try_wait(bar_parts")[0] > wait[1]
     assert "return" not in body          # no way past the closing wait
 
