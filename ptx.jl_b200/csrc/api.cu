@@ -280,6 +280,7 @@ const char* ptxb200_strerror(int code) {
         "gemm2:empty", "gemm2:full", "gemm2:acc_empty", "gemm2:acc_full",
         "fa:softmax.l_free", "fa:corr.combine_piece",
         "gemm_split:empty", "gemm_split:full", "gemm_split:acc_full", "gemm_split:parts",
+        "gemm_split:acc_empty",
     };
     unsigned site = ((unsigned)code >> 8) & 0xFFu;
     const char* name = site < sizeof(sites) / sizeof(sites[0]) ? sites[site] : "?";

@@ -1,0 +1,91 @@
+// Sizes of gemm_split_sm100.cu that the kernel, its launcher and the CPU tests share: ring
+// stages, chains of partial sums, shared and tensor memory of a CTA. Plain C++.
+#pragma once
+
+#if defined(__CUDACC__)
+#define PTXB200_PLAN_HD __host__ __device__
+#else
+#define PTXB200_PLAN_HD
+#endif
+
+namespace ptxb200 {
+
+constexpr int kBM3 = 128;             // rows of a tile
+constexpr int kBK3 = 64;              // a step of K: one 128-byte swizzle row of bf16
+constexpr int kMaxStages3 = 7;
+constexpr int kSmemMax3 = 232448;     // what a CTA can opt in to
+constexpr int kABytes3 = kBM3 * kBK3 * 2;
+constexpr int kChainSteps3 = 8;       // steps of K per accumulator
+// full[], empty[], acc_full[2], acc_empty[2], parts_in, TMEM slot, abort flag
+constexpr int kCtrlBytes3 = ((2 * kMaxStages3 + 5) * 8 + 8 + 15) / 16 * 16;
+static_assert(kCtrlBytes3 % 16 == 0, "the parts handed over behind it are 16-byte pieces");
+
+// steps of K per ring stage: two of 24 KiB (64 columns), or one of 32 KiB
+PTXB200_PLAN_HD constexpr int stage_k3(int bn) { return bn == 64 ? 2 : 1; }
+PTXB200_PLAN_HD constexpr int stage_bytes3(int bn) { return stage_k3(bn) * (kABytes3 + bn * kBK3 * 2); }
+// accumulators that tensor memory (512 columns) holds; with more chains of sums than that, two
+// take turns and a third block of columns keeps what has been added up
+PTXB200_PLAN_HD constexpr int max_accs3(int bn) { return 512 / bn; }
+// what the other parts of the tile hand a CTA: [split - 1][bn / split / 4][128 rows] float4
+PTXB200_PLAN_HD constexpr int recv_bytes3(int bn, int split) { return (split - 1) * kBM3 * (bn / split) * 4; }
+// steps [part_begin3(.., part), part_begin3(.., part + 1)) of K are one CTA's
+PTXB200_PLAN_HD constexpr int part_begin3(int kiters, int split, int part) {
+  return (int)((long long)kiters * part / split);
+}
+
+struct GemmSplitPlan {
+  int bn;         // columns of a tile (128 rows): 64 or 128
+  int split;      // parts of K, one CTA of a cluster each: 1, 2 or 4
+};
+
+// Few 128x256 tiles, cut along K: the steps of all tiles as one line, dealt out in equal shares of
+// at least kLineMinSteps to at most one CTA per SM, where that gives every tile two CTAs or more.
+constexpr int kLineMinSteps = 8;
+struct GemmLine {
+  int ctas;       // 0: not cut
+  int share;      // steps of the longest share, or all of K
+};
+inline GemmLine gemm_line(int sm_count, int groups, int M, int N, int kiters) {
+  const long long tiles = (long long)groups * (M / kBM3) * ((N + 255) / 256), line = tiles * kiters;
+  long long ctas = line / kLineMinSteps;
+  if (ctas > sm_count) ctas = sm_count;
+  if (tiles * 2 > sm_count || ctas < 2 * tiles) return {0, kiters};
+  return {(int)ctas, (int)((line + ctas - 1) / ctas)};
+}
+
+struct GemmSplitLayout {
+  int stages;         // of the ring
+  int chain_stages;   // stages a chain of sums runs over
+  bool fold;          // K split, more chains than accumulators (in the longest part; the same for all)
+  int tmem_cols;
+  int smem_bytes;
+};
+
+// `longest`: steps that no chain of sums may exceed (but kChainSteps3), 0: one chain over all of a
+// part's K. fp32 output has chains of kChainSteps3 steps, longer ones only where that saves folding.
+inline GemmSplitLayout gemm_split_layout(const GemmSplitPlan& p, int kiters, bool f32, int longest) {
+  GemmSplitLayout l;
+  // a ring as deep as shared memory allows, but no deeper than the work
+  const int recv = recv_bytes3(p.bn, p.split), per = stage_k3(p.bn);
+  const int steps = ((kiters + p.split - 1) / p.split + per - 1) / per;   // of the longest part, in stages
+  l.stages = (kSmemMax3 - kCtrlBytes3 - recv) / stage_bytes3(p.bn);
+  if (l.stages > kMaxStages3) l.stages = kMaxStages3;
+  if (l.stages > steps) l.stages = steps;
+  const int shortest = kChainSteps3 / per, limit = longest / per > shortest ? longest / per : shortest;   // stages
+  l.chain_stages = longest == 0 || steps <= shortest ? steps : f32 ? shortest : limit;
+  int chains = (steps + l.chain_stages - 1) / l.chain_stages;
+  const int accs = max_accs3(p.bn);
+  if (p.split > 1 && chains > accs && (steps + accs - 1) / accs <= limit) chains = accs;
+  l.fold = p.split > 1 && chains > accs;
+  l.chain_stages = (steps + chains - 1) / chains;
+  l.tmem_cols = p.bn;
+  const int blocks = l.fold ? 3 : p.split > 1 || chains < 2 ? chains : 2;
+  while (l.tmem_cols < blocks * p.bn) l.tmem_cols *= 2;
+  l.smem_bytes = l.stages * stage_bytes3(p.bn) + kCtrlBytes3 + recv;
+  // Two CTAs of different clusters never share an SM: each could hold the tensor memory that the
+  // other's peers wait for. (An SM has 1 KiB more than a CTA can take, and a CTA costs it 1 KiB.)
+  if (p.split > 1 && l.smem_bytes <= kSmemMax3 / 2) l.smem_bytes = kSmemMax3 / 2 + 16;
+  return l;
+}
+
+}  // namespace ptxb200

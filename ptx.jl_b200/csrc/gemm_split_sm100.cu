@@ -13,11 +13,16 @@
 // fixed, so results are reproducible (they differ in the last bits from the unsplit order).
 // One-shot blocks: the first loads are issued before the block's threads even meet.
 //
-// With fp32 output a CTA sums its part of K in chains of at most 8 steps, up to 8 chains (64
-// columns) or 4 (128), one accumulator in tensor memory each, and adds them up in the epilogue: the
-// tensor core's fp32 accumulation loses about 3e-8 of the result per step of a chain, so
-// one chain over 64 steps (1024x1152x8192 split in 2) is off by 4.0e-6, four of 16 steps by
-// 8.5e-7 (the 35-step shares of the schedule before: 1.9e-6). bf16 output rounds 1.7e-3.
+// A CTA sums its part of K in several chains: the tensor core's fp32 accumulation loses about
+// 5e-8 of the result per step of a chain (1024x1152x8192 split in 2, fp32 out: one chain of 64
+// steps 4.0e-6, four of 16 8.5e-7, of 8 4.0e-7). With fp32 output a chain has at most 8 steps where
+// the accumulators suffice (64 columns: 8 of them, 128: 4), and with either output never more
+// than the shares of one line of steps over all SMs would (gemm_line: 8 to 62). Where K is split each chain has
+// an accumulator of its own and the epilogue adds them up; with more chains than that two
+// accumulators take turns and the epilogue's warps fold them into a third as they end, which
+// costs 0.1 us per chain (128x256x65536 fp32 out, 32 chains: 48.5 us and 4.1e-7; 8 chains of 32:
+// 47.4 and 1.9e-6). Where K is not split the epilogue's warps take each chain into registers while the
+// next one runs (1024x1280x4096: fp32 out 18.6 us in chains of 8, bf16 17.8 in chains of 16, 17.0 in one).
 //
 // Measured (device time, bf16 out unless noted; before: 128x256 tiles cut into shares of
 // one k-iteration line, partial tiles parked in global memory, a second kernel to add
@@ -33,36 +38,21 @@
 namespace ptxb200 {
 namespace {
 
-constexpr int kBM3 = 128;
-constexpr int kBK3 = 64;              // one 128-byte swizzle row of bf16
 constexpr int kThreads3 = 192;        // warp 0 TMA producer, warp 1 MMA, warps 2-5 epilogue
-constexpr int kMaxStages3 = 7;
-constexpr int kSmemMax3 = 232448;
-constexpr int kABytes3 = kBM3 * kBK3 * 2;
 constexpr int kBandM3 = 8;            // row-tiles per rasterisation band
-constexpr int kChainSteps3 = 8;       // steps of K per accumulator with fp32 output, more only where accumulators run out
-// full[], empty[], acc_full, parts_in, TMEM slot, abort flag
-constexpr int kCtrlBytes3 = ((2 * kMaxStages3 + 2) * 8 + 8 + 15) / 16 * 16;
-static_assert(kCtrlBytes3 % 16 == 0, "the parts handed over behind it are 16-byte pieces");
 
-enum : uint32_t { kSite3Empty = 24, kSite3Full = 25, kSite3AccFull = 26, kSite3Parts = 27 };
+enum : uint32_t { kSite3Empty = 24, kSite3Full = 25, kSite3AccFull = 26, kSite3Parts = 27, kSite3AccEmpty = 28 };
 
-// steps of K per ring stage: two of 24 KiB (64 columns), or one of 32 KiB
-__host__ __device__ constexpr int stage_k3(int bn) { return bn == 64 ? 2 : 1; }
-__host__ __device__ constexpr int stage_bytes3(int bn) { return stage_k3(bn) * (kABytes3 + bn * kBK3 * 2); }
-// what the other parts of the tile hand a CTA: [split - 1][bn / split / 4][128 rows] float4
-__host__ __device__ constexpr int recv_bytes3(int bn, int split) { return (split - 1) * kBM3 * (bn / split) * 4; }
-
-// 16 columns of this thread's row, summed over the chains (accumulators kBN columns apart)
+// 16 columns of this thread's row, summed over `pieces` blocks of kBN columns
 template <int kBN>
-__device__ __forceinline__ void load_sum16(uint32_t taddr, int chains, float (&x)[16]) {
+__device__ __forceinline__ void load_sum16(uint32_t taddr, int pieces, float (&x)[16]) {
   uint32_t v[16];
   tmem_ld16(taddr, v);
   tc_wait_ld_bind16(v);
 #pragma unroll
   for (int i = 0; i < 16; ++i) x[i] = __uint_as_float(v[i]);
 #pragma unroll 1
-  for (int a = 1; a < chains; ++a) {
+  for (int a = 1; a < pieces; ++a) {
     tmem_ld16(taddr + a * kBN, v);
     tc_wait_ld_bind16(v);
 #pragma unroll
@@ -70,22 +60,60 @@ __device__ __forceinline__ void load_sum16(uint32_t taddr, int chains, float (&x
   }
 }
 
-template <int kBN, bool kF32Out>
+// Adds a finished chain (kBN columns at `acc`) to the columns at `run`, or copies it there.
+template <int kBN>
+__device__ __forceinline__ void fold_chain(uint32_t run, uint32_t acc, bool copy) {
+#pragma unroll 1
+  for (int c = 0; c < kBN; c += 32) {
+    uint32_t v[32];
+    tmem_ld32(acc + c, v);
+    tc_wait_ld_bind(v);
+    if (!copy) {
+      uint32_t x[32];
+      tmem_ld32(run + c, x);
+      tc_wait_ld_bind(x);
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(x[i]) + __uint_as_float(v[i]));
+    }
+    tmem_st32(run + c, v);
+  }
+  tc_wait_st();
+}
+
+// Adds a finished chain (kBN columns at t_row) to this thread's sums, or takes it as they are: the
+// fragments of 16 rows x 64 columns that store_acc_16x64 writes, of the warp's first and second
+// 16 rows in turn.
+template <int kBN>
+__device__ __forceinline__ void take_chain(uint32_t t_row, bool copy, float (&sum)[kBN]) {
+#pragma unroll
+  for (int b = 0; b < kBN / 32; ++b) {
+    uint32_t v[32];
+    tmem_ld_16x64(t_row + ((uint32_t)(b & 1) << 20) + (b >> 1) * 64, v);
+    tc_wait_ld_bind(v);
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      sum[b * 32 + i] = copy ? __uint_as_float(v[i]) : sum[b * 32 + i] + __uint_as_float(v[i]);
+  }
+}
+
+// kSplit: K is split over the CTAs of a cluster; kFold: into more chains than accumulators.
+template <int kBN, bool kF32Out, bool kSplit, bool kFold>
 __global__ void __launch_bounds__(kThreads3, 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                   void* __restrict__ c_out, int M, int N, int K, int ldc, int split, int stages, int chain_stages,
                   uint32_t tmem_cols, uint32_t* status) {
+  if constexpr (!kSplit) split = 1;
   constexpr int kStageK = stage_k3(kBN), kStageBytes = stage_bytes3(kBN);
   constexpr int kAtomBytes = kABytes3 + kBN * kBK3 * 2;
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t base = smem_u32(smem);
-  const int part = split > 1 ? (int)cluster_ctarank() : 0;   // which part of K this CTA of the cluster sums
+  const int part = kSplit ? (int)cluster_ctarank() : 0;   // which part of K this CTA of the cluster sums
 
   const uint32_t ctrl = base + stages * kStageBytes;
   uint8_t* ctrl_ptr = smem + stages * kStageBytes;
-  const uint32_t bar_full = ctrl, bar_empty = ctrl + 8 * kMaxStages3, bar_acc = ctrl + 16 * kMaxStages3;
-  const uint32_t bar_parts = bar_acc + 8;
-  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(ctrl_ptr + 16 * kMaxStages3 + 16);
+  const uint32_t bar_full = ctrl, bar_empty = ctrl + 8 * kMaxStages3, bar_acc_full = ctrl + 16 * kMaxStages3;
+  const uint32_t bar_acc_empty = bar_acc_full + 16, bar_parts = bar_acc_empty + 16;
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(ctrl_ptr + 16 * kMaxStages3 + 40);
   volatile uint32_t* abort_flag = tmem_slot + 1;
   const uint32_t recv = ctrl + kCtrlBytes3;
   const float4* recv_ptr = reinterpret_cast<const float4*>(ctrl_ptr + kCtrlBytes3);
@@ -109,8 +137,12 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     tn = q / rows;
   }
   const int kiters = K / kBK3;
-  const int k0 = (int)((long long)kiters * part / split), k1 = (int)((long long)kiters * (part + 1) / split);
+  const int k0 = part_begin3(kiters, split, part), k1 = part_begin3(kiters, split, part + 1);
   const int steps = (k1 - k0 + kStageK - 1) / kStageK;       // ring stages this CTA fills; the last may be a half
+  // Chains of sums over chain_stages each. K split: every one in an accumulator of its own, or
+  // (kFold) in the second and the third in turn and added to what the first holds as they end;
+  // otherwise in two accumulators in turn, and taken into registers as they end.
+  const int chains = (steps + chain_stages - 1) / chain_stages;
 
   auto load = [&](int i, int s) {
     const uint32_t full = bar_full + 8 * s, dst = base + s * kStageBytes;
@@ -132,10 +164,13 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       mbar_init(bar_full + 8 * s, 1);
       mbar_init(bar_empty + 8 * s, 1);
     }
-    mbar_init(bar_acc, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(bar_acc_full + 8 * i, 1);
+      mbar_init(bar_acc_empty + 8 * i, 128);
+    }
     mbar_init(bar_parts, 1);
     mbar_fence_init();
-    if (split > 1) mbar_arrive_expect_tx(bar_parts, recv_bytes3(kBN, split));
+    if (kSplit) mbar_arrive_expect_tx(bar_parts, recv_bytes3(kBN, split));
     if (!misaligned)
       for (int i = 0; i < stages && i < steps; ++i) load(i, i);
   }
@@ -146,7 +181,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   __syncwarp();
   tc_fence_before();
   __syncthreads();
-  if (split > 1) cluster_arrive();          // "this CTA has started": waited for ahead of the first store to a peer
+  if (kSplit) cluster_arrive();          // "this CTA has started": waited for ahead of the first store to a peer
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
@@ -166,35 +201,61 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     constexpr uint32_t dhi = sdesc_hi(1024, kLayoutB128);
     int s = 0;
     uint32_t ph = 0, acc = tmem, first = 0;     // the chain's accumulator; 0: its first product overwrites it
-    int left = chain_stages;                    // stages until the next chain begins
-    auto mma = [&](int a, int slot, uint32_t accumulate) {   // one step of K: 4 instructions of 16
+    auto mma = [&](int a, int slot) {           // one step of K: 4 instructions of 16
       const uint32_t da = sdesc_lo(base + slot * kStageBytes + a * kAtomBytes, 16);
       const uint32_t db = sdesc_lo(base + slot * kStageBytes + a * kAtomBytes + kABytes3, 16);
 #pragma unroll
       for (int kk = 0; kk < kBK3 / 16; ++kk)   // 2 descriptor units = 32 bytes = 16 elements of K
-        tc_mma_ss_warp(acc, da + 2 * kk, dhi, db + 2 * kk, dhi, idesc, kk == 0 ? accumulate : 1u);
+        tc_mma_ss_warp(acc, da + 2 * kk, dhi, db + 2 * kk, dhi, idesc, a == 0 && kk == 0 ? first : 1u);
+    };
+    auto full_stage = [&]() {
+      mbar_wait_warp(bar_full + 8 * s, ph, wctx, kSite3Full);
+      tc_fence_after();
+      mma(0, s);
+      if constexpr (kStageK == 2) mma(1, s);
+      tc_commit_warp(bar_empty + 8 * s);
+      if (++s == stages) { s = 0; ph ^= 1u; }
+    };
+    auto half_stage = [&]() {
+      mbar_wait_warp(bar_full + 8 * s, ph, wctx, kSite3Full);
+      tc_fence_after();
+      mma(0, s);
     };
     // full stages first, without a branch around any instruction (one in this loop costs
     // about a hundred cycles a step), then a last half stage
     const int full_steps = (k1 - k0) / kStageK;
-    for (int i = 0; i < full_steps; ++i) {
-      mbar_wait_warp(bar_full + 8 * s, ph, wctx, kSite3Full);
-      tc_fence_after();
-      mma(0, s, first);
-      if constexpr (kStageK == 2) mma(1, s, 1u);
-      tc_commit_warp(bar_empty + 8 * s);
-      if (++s == stages) { s = 0; ph ^= 1u; }
-      const bool next = --left == 0;
-      first = next ? 0u : 1u;
-      acc += next ? (uint32_t)kBN : 0u;
-      left = next ? chain_stages : left;
+    if constexpr (kSplit && !kFold) {
+      int left = chain_stages;                  // stages until the next chain begins
+      for (int i = 0; i < full_steps; ++i) {
+        full_stage();
+        const bool next = --left == 0;
+        first = next ? 0u : 1u;
+        acc += next ? (uint32_t)kBN : 0u;
+        left = next ? chain_stages : left;
+      }
+      if (full_steps < steps) half_stage();
+      tc_commit_warp(bar_acc_full);
+    } else {
+      int i = 0;
+      for (int c = 0; c < chains; ++c) {
+        const int buf = c & 1, end = min(i + chain_stages, steps), full_end = min(end, full_steps);
+        if (c >= 2) {
+          mbar_wait_warp(bar_acc_empty + 8 * buf, (uint32_t)(c / 2 - 1) & 1u, wctx, kSite3AccEmpty);
+          tc_fence_after();
+        }
+        acc = tmem + (buf + (kFold ? 1 : 0)) * kBN;
+        first = 0;
+        for (; i < full_end; ++i) {
+          full_stage();
+          first = 1u;
+        }
+        if (i < end) {
+          half_stage();
+          ++i;
+        }
+        tc_commit_warp(bar_acc_full + 8 * buf);
+      }
     }
-    if (full_steps < steps) {
-      mbar_wait_warp(bar_full + 8 * s, ph, wctx, kSite3Full);
-      tc_fence_after();
-      mma(0, s, first);
-    }
-    tc_commit_warp(bar_acc);
   }
 
   const int quad = warp & 3;
@@ -203,34 +264,41 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   const uint32_t t_row = tmem_addr(tmem, quad * 32, 0);
   const size_t row = (size_t)g * M + (size_t)tm * kBM3 + row_in_tile;
   const int col0 = tn * kBN;
-  const int chains = kF32Out ? (steps + chain_stages - 1) / chain_stages : 1;
-  if (epilogue) {
-    mbar_wait(bar_acc, 0, wctx, kSite3AccFull);
-    tc_fence_after();
-  }
-  if (split == 1) {
+  // f(chain's accumulator, number) as the chains end, beside the products of the next
+  auto each_chain = [&](auto f) {
+#pragma unroll 1
+    for (int c = 0; c < chains; ++c) {
+      mbar_wait(bar_acc_full + 8 * (c & 1), (uint32_t)(c / 2) & 1u, wctx, kSite3AccFull);
+      tc_fence_after();
+      f(t_row + ((c & 1) + (kFold ? 1 : 0)) * kBN, c);
+      tc_fence_before();
+      mbar_arrive(bar_acc_empty + 8 * (c & 1));
+    }
+  };
+  if constexpr (!kSplit) {
     if (epilogue) {
-#pragma unroll 1
-      for (int h = 0; h < 2; ++h) {          // this warp's first and second 16 rows
-        const size_t row16 = (size_t)g * M + (size_t)tm * kBM3 + quad * 32 + h * 16 + (lane >> 2);
-#pragma unroll 1
-        for (int c = 0; c < kBN; c += 64) {
-          uint32_t v[32];
-          tmem_ld_16x64(t_row + ((uint32_t)(h * 16) << 16) + c, v);
-          tc_wait_ld_bind(v);
-#pragma unroll 1
-          for (int a = 1; a < chains; ++a) {
-            uint32_t x[32];
-            tmem_ld_16x64(t_row + ((uint32_t)(h * 16) << 16) + a * kBN + c, x);
-            tc_wait_ld_bind(x);
+      float sum[kBN];
+      each_chain([&](uint32_t acc, int c) { take_chain<kBN>(acc, c == 0, sum); });
 #pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) + __uint_as_float(x[i]));
-          }
-          if (col0 + c < N) store_acc_16x64<kF32Out>(c_out, row16, ldc, col0 + c, v);   // N % 64 == 0
-        }
+      for (int b = 0; b < kBN / 32; ++b) {
+        const size_t row16 = (size_t)g * M + (size_t)tm * kBM3 + quad * 32 + (b & 1) * 16 + (lane >> 2);
+        const int c = (b >> 1) * 64;
+        uint32_t v[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(sum[b * 32 + i]);
+        if (col0 + c < N) store_acc_16x64<kF32Out>(c_out, row16, ldc, col0 + c, v);   // N % 64 == 0
       }
     }
   } else {
+    if (epilogue) {
+      if constexpr (kFold) {
+        each_chain([&](uint32_t acc, int c) { fold_chain<kBN>(t_row, acc, c == 0); });
+      } else {
+        mbar_wait(bar_acc_full, 0, wctx, kSite3AccFull);
+        tc_fence_after();
+      }
+    }
+    const int pieces = kFold ? 1 : chains;   // blocks of columns to add up
     // every part sums up and writes bn / split columns: it sends the others theirs
     const int width = kBN / split;
     cluster_wait();
@@ -244,7 +312,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 #pragma unroll 2
         for (int c = 0; c < width; c += 16) {
           float x[16];
-          load_sum16<kBN>(t_row + q * width + c, chains, x);
+          load_sum16<kBN>(t_row + q * width + c, pieces, x);
 #pragma unroll
           for (int j = 0; j < 4; ++j)
             st_async_v4(dst + (c / 4 + j) * (kBM3 * 16), dst_bar, x[4 * j], x[4 * j + 1], x[4 * j + 2], x[4 * j + 3]);
@@ -252,11 +320,24 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       }
     }
     if (epilogue) {
+      if (pieces > 1) {
+        // this CTA's own share is added up while the others' is on its way
+#pragma unroll 1
+        for (int c = 0; c < width; c += 16) {
+          float x[16];
+          load_sum16<kBN>(t_row + part * width + c, pieces, x);
+          uint32_t v[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(x[i]);
+          tmem_st16(t_row + part * width + c, v);
+        }
+        tc_wait_st();
+      }
       mbar_wait<true>(bar_parts, 0, wctx, kSite3Parts);   // other CTAs' stores are read behind it
 #pragma unroll 1
       for (int c = 0; c < width; c += 16) {
         float own[16], sum[16];
-        load_sum16<kBN>(t_row + part * width + c, chains, own);
+        load_sum16<kBN>(t_row + part * width + c, 1, own);
 #pragma unroll
         for (int i = 0; i < 16; ++i) sum[i] = 0.0f;
         // in the order of the parts, whoever adds them up
@@ -286,7 +367,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   // CTA that has left is a fault: it stays until every peer has left or stays as well, and these
   // have all issued their stores, and until the stores have landed. (Otherwise it has received
   // all parts and nobody stores into it any more. A barrier in every launch costs 0.5 us.)
-  if (split > 1 && !misaligned && *abort_flag != 0) {
+  if (kSplit && !misaligned && *abort_flag != 0) {
     cluster_arrive();
     cluster_wait();   // for all threads of the cluster that have not left
     if (threadIdx.x == 0 && !mbar_try_wait(bar_parts, 0)) {
@@ -296,9 +377,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   }
 }
 
-template <int kBN, bool kF32Out>
-int launch_one3(const DeviceCtx& ctx, int split, void* C, const void* A, const void* Bt, int groups, int M, int N, int K,
-                int ldc, bool one_chain, cudaStream_t stream) {
+template <int kBN, bool kF32Out, bool kSplit, bool kFold>
+int launch_one3(const DeviceCtx& ctx, const GemmSplitPlan& p, const GemmSplitLayout& l, void* C, const void* A, const void* Bt, int groups, int M,
+                int N, int K, int ldc, cudaStream_t stream) {
   CUtensorMap ta, tb;
   int rc = encode_tmap_bf16_2d(&ta, A, (uint64_t)groups * M, (uint64_t)K, (uint64_t)K * 2, kBM3, kBK3);
   if (rc != PTXB200_OK) return rc;
@@ -306,36 +387,31 @@ int launch_one3(const DeviceCtx& ctx, int split, void* C, const void* A, const v
   if (rc != PTXB200_OK) return rc;
   static PerDeviceOnce attr_once;
   rc = attr_once.run(ctx.device, []() -> int {
-    PTXB200_CUDA_TRY(cudaFuncSetAttribute(gemm_split_kernel<kBN, kF32Out>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          kSmemMax3));
+    PTXB200_CUDA_TRY(cudaFuncSetAttribute(gemm_split_kernel<kBN, kF32Out, kSplit, kFold>,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax3));
     return PTXB200_OK;
   });
   if (rc != PTXB200_OK) return rc;
-  // a ring as deep as shared memory allows, but no deeper than the work
-  const int recv = recv_bytes3(kBN, split);
-  const int steps = ((K / kBK3 + split - 1) / split + stage_k3(kBN) - 1) / stage_k3(kBN);   // of the longest part
-  int stages = (kSmemMax3 - kCtrlBytes3 - recv) / stage_bytes3(kBN);
-  if (stages > kMaxStages3) stages = kMaxStages3;
-  if (stages > steps) stages = steps;
-  // chains of at most kChainSteps3 steps, as far as tensor memory holds accumulators
-  int chains = one_chain || !kF32Out ? 1 : (steps * stage_k3(kBN) + kChainSteps3 - 1) / kChainSteps3;
-  if (chains > 512 / kBN) chains = 512 / kBN;
-  const int chain_stages = (steps + chains - 1) / chains;
-  uint32_t tmem_cols = kBN;
-  while (tmem_cols < (uint32_t)(chains * kBN)) tmem_cols *= 2;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(groups * (M / kBM3) * ((N + kBN - 1) / kBN) * split));
+  cfg.gridDim = dim3((unsigned)(groups * (M / kBM3) * ((N + kBN - 1) / kBN) * p.split));
   cfg.blockDim = dim3(kThreads3);
-  cfg.dynamicSmemBytes = (size_t)stages * stage_bytes3(kBN) + kCtrlBytes3 + recv;
+  cfg.dynamicSmemBytes = (size_t)l.smem_bytes;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim = {(unsigned)split, 1, 1};
+  attr[0].val.clusterDim = {(unsigned)p.split, 1, 1};
   cfg.attrs = attr;
-  cfg.numAttrs = split > 1 ? 1 : 0;
-  PTXB200_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_split_kernel<kBN, kF32Out>, ta, tb, C, M, N, K, ldc, split, stages,
-                                      chain_stages, tmem_cols, status_word(ctx, stream)));
+  cfg.numAttrs = kSplit ? 1 : 0;
+  PTXB200_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_split_kernel<kBN, kF32Out, kSplit, kFold>, ta, tb, C, M, N, K, ldc, p.split,
+                                      l.stages, l.chain_stages, (uint32_t)l.tmem_cols, status_word(ctx, stream)));
   return PTXB200_OK;
+}
+
+template <int kBN, bool kF32Out, class... Args>
+int launch_parts3(const DeviceCtx& ctx, const GemmSplitPlan& p, const GemmSplitLayout& l, Args... args) {
+  if (p.split == 1) return launch_one3<kBN, kF32Out, false, false>(ctx, p, l, args...);
+  return l.fold ? launch_one3<kBN, kF32Out, true, true>(ctx, p, l, args...)
+                : launch_one3<kBN, kF32Out, true, false>(ctx, p, l, args...);
 }
 
 }  // namespace
@@ -368,12 +444,15 @@ bool gemm_split_choose(const DeviceCtx& ctx, int groups, int M, int N, int K, un
 
 int launch_gemm_split(const DeviceCtx& ctx, const GemmSplitPlan& p, void* C, const void* A, const void* Bt, int groups,
                       int M, int N, int K, int ldc, unsigned flags, cudaStream_t stream) {
-  const bool f32 = (flags & PTXB200_GEMM_F32_OUT) != 0, one_chain = (flags & PTXB200_GEMM_NO_SPLIT) != 0;
+  const bool f32 = (flags & PTXB200_GEMM_F32_OUT) != 0;
+  const int kiters = K / kBK3;
+  const int longest = (flags & PTXB200_GEMM_NO_SPLIT) ? 0 : gemm_line(ctx.sm_count, groups, M, N, kiters).share;
+  const GemmSplitLayout l = gemm_split_layout(p, kiters, f32, longest);
   if (p.bn == 64)
-    return f32 ? launch_one3<64, true>(ctx, p.split, C, A, Bt, groups, M, N, K, ldc, one_chain, stream)
-               : launch_one3<64, false>(ctx, p.split, C, A, Bt, groups, M, N, K, ldc, one_chain, stream);
-  return f32 ? launch_one3<128, true>(ctx, p.split, C, A, Bt, groups, M, N, K, ldc, one_chain, stream)
-             : launch_one3<128, false>(ctx, p.split, C, A, Bt, groups, M, N, K, ldc, one_chain, stream);
+    return f32 ? launch_parts3<64, true>(ctx, p, l, C, A, Bt, groups, M, N, K, ldc, stream)
+               : launch_parts3<64, false>(ctx, p, l, C, A, Bt, groups, M, N, K, ldc, stream);
+  return f32 ? launch_parts3<128, true>(ctx, p, l, C, A, Bt, groups, M, N, K, ldc, stream)
+             : launch_parts3<128, false>(ctx, p, l, C, A, Bt, groups, M, N, K, ldc, stream);
 }
 
 }  // namespace ptxb200

@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "../../include/ptxb200.h"
+#include "gemm_split_plan.h"
 
 namespace ptxb200 {
 
@@ -116,11 +117,6 @@ int encode_tmap_bf16_3d(CUtensorMap* out, const void* base, uint64_t slices, uin
       return PTXB200_E_CUDA;                           \
     }                                                  \
   } while (0)
-
-struct GemmSplitPlan {
-  int bn;         // columns of a tile (128 rows): 64 or 128
-  int split;      // parts of K, one CTA of a cluster each: 1, 2 or 4
-};
 
 // Kernel launchers (one per .cu file).
 int launch_gemm(const DeviceCtx& ctx, void* C, const void* A, const void* Bt, int groups, int M, int N,

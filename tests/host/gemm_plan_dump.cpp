@@ -1,0 +1,24 @@
+// Prints what ptx.jl_b200/csrc/gemm_split_plan.h says, for tests/test_gemm_split_plan.py.
+#include <cstdio>
+#include <initializer_list>
+
+#include "gemm_split_plan.h"
+
+using namespace ptxb200;
+
+int main() {
+  const int steps[] = {1, 2, 3, 7, 8, 9, 15, 16, 17, 31, 32, 33, 64, 127, 128, 129, 255, 256, 512, 1024, 1027, 4096};
+  for (int bn = 64; bn <= 128; bn *= 2)
+    for (int split = 1; split <= 4; split *= 2)
+      for (int kiters : steps)
+        for (int f32 = 0; f32 < 2; ++f32)
+          for (int longest : {0, 8, 9, 18, 35, 1024}) {
+            if (kiters < split) continue;
+            const GemmSplitLayout l = gemm_split_layout({bn, split}, kiters, f32 != 0, longest);
+            std::printf("layout %d %d %d %d %d %d %d %d %d %d %d %d", bn, split, kiters, f32, longest, l.stages,
+                        l.chain_stages, l.fold ? 1 : 0, l.tmem_cols, l.smem_bytes, recv_bytes3(bn, split), stage_k3(bn));
+            for (int part = 0; part <= split; ++part) std::printf(" %d", part_begin3(kiters, split, part));
+            std::printf("\n");
+          }
+  return 0;
+}

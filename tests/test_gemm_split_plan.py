@@ -1,0 +1,80 @@
+"""The sizes and rules that gemm_split_sm100.cu runs by, from its own header compiled on the
+host: every step of K once, chains of at most eight steps, shared and tensor memory within
+what an SM has, a slot of its own for everything one CTA of a cluster hands another."""
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+@pytest.fixture(scope="module")
+def dump(tmp_path_factory):
+    exe = str(tmp_path_factory.mktemp("plan") / "gemm_plan_dump")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", os.path.join(ROOT, "ptx.jl_b200", "csrc"),
+                    os.path.join(ROOT, "tests", "host", "gemm_plan_dump.cpp"), "-o", exe], check=True)
+    out = subprocess.run([exe], check=True, stdout=subprocess.PIPE, text=True).stdout
+    return [line.split() for line in out.strip().splitlines()]
+
+
+def layouts(dump):
+    names = "bn split kiters f32 longest stages chain fold tmem smem recv per".split()
+    for line in dump:
+        if line[0] == "layout":
+            values = list(map(int, line[1:]))
+            yield dict(zip(names, values), cuts=values[len(names):])
+
+
+def test_parts_cover_k_once_and_chains_are_short(dump):
+    n = 0
+    for l in layouts(dump):
+        cuts, bn, per = l["cuts"], l["bn"], l["per"]
+        assert cuts[0] == 0 and cuts[-1] == l["kiters"] and len(cuts) == l["split"] + 1
+        for a, b in zip(cuts, cuts[1:]):
+            assert b > a                                        # no part without a step
+            ring = -(-(b - a) // per)                           # stages this part fills
+            chains = -(-ring // l["chain"])
+            if l["longest"] == 0:
+                assert chains == 1                              # one accumulation in k order
+            else:                                               # never above what the caller allows, or 8
+                assert l["chain"] * per <= max(8, l["longest"]) or chains == 1 and b - a <= max(8, l["longest"])
+            most = -(-max(y - x for x, y in zip(cuts, cuts[1:])) // 8)     # chains of 8 that the longest part takes
+            if l["f32"] and l["longest"] and (l["split"] == 1 or most * bn <= 512):
+                assert l["chain"] * per <= 8                    # longer only where accumulators run out
+            # accumulators: two in turn, with another for what they add up to where K is split, or all
+            blocks = 3 if l["fold"] else min(chains, 2) if l["split"] == 1 else chains
+            assert bn * blocks <= l["tmem"] <= 512 and l["tmem"] & (l["tmem"] - 1) == 0
+        n += 1
+    assert n > 1000
+
+
+def test_memory_fits_and_clusters_do_not_share_an_sm(dump):
+    for l in layouts(dump):
+        assert 1 <= l["stages"] <= 7
+        ring = l["stages"] * l["per"] * (128 + l["bn"]) * 128
+        assert ring + 160 + l["recv"] <= l["smem"] <= 232448
+        if l["split"] > 1:
+            assert 2 * (l["smem"] + 1024) > 233472              # an SM's 228 KiB
+
+
+@pytest.mark.parametrize("bn,split", [(64, 2), (64, 4), (128, 2), (128, 4)])
+def test_each_pair_of_parts_has_a_slot_of_its_own(dump, bn, split):
+    """The kernel's indexing: sender p's 16-byte pieces of the columns that q sums up go to slot
+    (p < q ? p : p - 1) of q, [columns / 4][128 rows] of them."""
+    recv = next(l["recv"] for l in layouts(dump) if l["bn"] == bn and l["split"] == split)
+    width = bn // split
+    assert width % 16 == 0
+    for q in range(split):
+        seen = set()
+        for p in range(split):
+            if p == q:
+                continue
+            slot = p if p < q else p - 1
+            for c in range(0, bn, 16):
+                if c // width != q:
+                    continue
+                for j in range(4):
+                    for row in range(128):
+                        seen.add(slot * (128 * width * 4) + ((c - q * width) // 4 + j) * (128 * 16) + row * 16)
+        assert len(seen) * 16 == recv and min(seen) == 0 and max(seen) == recv - 16

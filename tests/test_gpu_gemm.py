@@ -302,6 +302,23 @@ def test_gemm_tile_rules_against_64_bit(pkg, gpu, G, M, N, K, f32_out):
     assert pkg.ops.sync_status() == 0
 
 
+@pytest.mark.parametrize("M,N,K,steps", [
+    (128, 64, 512, 8), (128, 64, 65536, 8), (128, 256, 32768, 8), (256, 128, 16448, 8), (512, 512, 16384, 8),
+    (1024, 1152, 8192, 16), (1152, 2048, 8128, 16),     # four accumulators of 128 columns for 64 steps
+    (1024, 1280, 8192, 8),                              # K not split
+])
+def test_gemm_fp32_sums_run_in_short_chains(pkg, gpu, M, N, K, steps):
+    """Few tiles, fp32 out: the tensor core's fp32 accumulation is off by about 5e-8 of the result
+    (2-norm) per step of 64 of a chain (measured: 4.0e-7 after 8 steps, 8.5e-7 after 16, 1.9e-6
+    after 32), so that chains of n steps stay below (n + 4) * 5e-8 whatever K is."""
+    g = torch.Generator(device=gpu).manual_seed(M + N + K)
+    a, bt = (torch.rand(1, n, K, generator=g, device=gpu).mul_(2).sub_(1).to(torch.bfloat16) for n in (M, N))
+    c = pkg.ops.gemm_grouped(a, bt, f32_out=True)
+    ref = a.double() @ bt.double().mT
+    assert pkg.ops.sync_status() == 0
+    assert float((c.double() - ref).norm() / ref.norm()) < (steps + 4) * 5e-8
+
+
 def _random_gemm_shapes(n, seed):
     rng = np.random.default_rng(seed)
     out = []
