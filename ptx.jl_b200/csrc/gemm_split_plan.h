@@ -38,6 +38,33 @@ struct GemmSplitPlan {
   int split;      // parts of K, one CTA of a cluster each: 1, 2 or 4
 };
 
+// Which products run on small tiles, and how: those whose 128x128 tiles fit the SMs in one round
+// (more tiles are better off in the persistent kernels: 2048x2048x512 9.1 us there, 9.1-11.2 here).
+// Tiles of 64 columns if those fit too, since a step of K costs a CTA nearly the same for
+// 64 columns as for 128 (1024^3: 6.7 against 7.7 us). K is split where SMs are left over and a
+// part keeps at least 4 (split in 4) or 8 (in 2) steps: handing the parts over costs
+// 1-2 us (384x640x1024: 5.8 in 4 parts, 6.7 whole; 512^3: 5.4 in 2 or 4 parts, 4.9 whole).
+// In 4 only where all clusters run at once (`clusters4`): 34 products of 128x64x1024 take two
+// rounds and 11.8 us in 4 parts, 8.0 in 2; 33 take 7.8 and 8.0.
+// Half of K on tiles of 128 columns against all of it on tiles of 64, which use equally
+// many CTAs, pays from about 64 steps on (1024x1152: 16.1 against 16.5 us at 64 steps, 21.0
+// against 25.3 at 128, 11.7 against 10.5 at 32).
+inline bool gemm_split_rule(int sm_count, int clusters4, int groups, int M, int N, int kiters, bool may_split,
+                            GemmSplitPlan* plan) {
+  const long long sms = sm_count, rows = (long long)groups * (M / kBM3);
+  const long long tiles128 = rows * ((N + 127) / 128), tiles64 = rows * ((N + 63) / 64);
+  if (tiles128 > sms) return false;
+  plan->split = 1;
+  if (tiles64 > sms || (may_split && kiters >= 64 && tiles64 * 2 > sms && tiles128 * 2 <= sms)) {
+    plan->bn = 128;
+    if (may_split && kiters >= 16 && tiles128 * 2 <= sms) plan->split = 2;
+    return true;
+  }
+  plan->bn = 64;
+  if (may_split && kiters >= 16) plan->split = tiles64 <= clusters4 ? 4 : tiles64 * 2 <= sms ? 2 : 1;
+  return true;
+}
+
 // Few 128x256 tiles, cut along K: the steps of all tiles as one line, dealt out in equal shares of
 // at least kLineMinSteps to at most one CTA per SM, where that gives every tile two CTAs or more.
 constexpr int kLineMinSteps = 8;

@@ -416,30 +416,37 @@ int launch_parts3(const DeviceCtx& ctx, const GemmSplitPlan& p, const GemmSplitL
 
 }  // namespace
 
-// Which products run here, and how: those whose 128x128 tiles fit the SMs in one round (more
-// tiles are better off in the persistent kernels: 2048x2048x512 9.1 us there, 9.1-11.2 here).
-// Tiles of 64 columns if those fit too, since a step of K costs a CTA nearly the same for
-// 64 columns as for 128 (1024^3: 6.7 against 7.7 us). K is split where SMs are left over and a
-// part keeps at least 4 (split in 4) or 8 (in 2) steps: handing the parts over costs
-// 1-2 us (384x640x1024: 5.8 in 4 parts, 6.7 whole; 512^3: 5.4 in 2 or 4 parts, 4.9 whole).
-// Half of K on tiles of 128 columns against all of it on tiles of 64, which use equally
-// many CTAs, pays from about 64 steps on (1024x1152: 16.1 against 16.5 us at 64 steps, 21.0
-// against 25.3 at 128, 11.7 against 10.5 at 32).
 bool gemm_split_choose(const DeviceCtx& ctx, int groups, int M, int N, int K, unsigned flags, GemmSplitPlan* plan) {
-  const long long sms = ctx.sm_count, rows = (long long)groups * (M / kBM3);
-  const long long tiles128 = rows * ((N + 127) / 128), tiles64 = rows * ((N + 63) / 64);
-  if (tiles128 > sms) return false;
-  const int kiters = K / kBK3;
-  const bool may_split = !(flags & PTXB200_GEMM_NO_SPLIT);
-  plan->split = 1;
-  if (tiles64 > sms || (may_split && kiters >= 64 && tiles64 * 2 > sms && tiles128 * 2 <= sms)) {
-    plan->bn = 128;
-    if (may_split && kiters >= 16 && tiles128 * 2 <= sms) plan->split = 2;
-    return true;
+  // Clusters of four CTAs that fill their SMs which the device runs at once: they do not straddle
+  // its groups of SMs, so that these are fewer than a quarter of its SMs (33 of 37).
+  static std::mutex mu;
+  static std::vector<int> clusters4;
+  int at_once = 0;
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    if ((int)clusters4.size() <= ctx.device) clusters4.resize(ctx.device + 1, -1);
+    int& known = clusters4[ctx.device];
+    if (known < 0) {
+      auto* kernel = gemm_split_kernel<64, false, true, false>;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3((unsigned)(ctx.sm_count / 4 * 4));
+      cfg.blockDim = dim3(kThreads3);
+      cfg.dynamicSmemBytes = kSmemMax3;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim = {4, 1, 1};
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      known = 0;
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax3) != cudaSuccess ||
+          cudaOccupancyMaxActiveClusters(&known, kernel, &cfg) != cudaSuccess) {
+        known = 0;              // pairs then
+        cudaGetLastError();
+      }
+    }
+    at_once = known;
   }
-  plan->bn = 64;
-  if (may_split && kiters >= 16) plan->split = tiles64 * 4 <= sms ? 4 : tiles64 * 2 <= sms ? 2 : 1;
-  return true;
+  return gemm_split_rule(ctx.sm_count, at_once, groups, M, N, K / kBK3, (flags & PTXB200_GEMM_NO_SPLIT) == 0, plan);
 }
 
 int launch_gemm_split(const DeviceCtx& ctx, const GemmSplitPlan& p, void* C, const void* A, const void* Bt, int groups,

@@ -20,5 +20,14 @@ int main() {
             for (int part = 0; part <= split; ++part) std::printf(" %d", part_begin3(kiters, split, part));
             std::printf("\n");
           }
+  // the rule, for products of one row-tile and n columns of 64, on 148 SMs
+  for (int clusters4 : {0, 33, 37})
+    for (int n = 1; n <= 300; ++n)
+      for (int kiters : {1, 8, 15, 16, 63, 64, 1024})
+        for (int may = 0; may < 2; ++may) {
+          GemmSplitPlan p = {0, 0};
+          const bool here = gemm_split_rule(148, clusters4, 1, 128, 64 * n, kiters, may != 0, &p);
+          std::printf("rule %d %d %d %d %d %d %d\n", clusters4, n, kiters, may, here ? 1 : 0, p.bn, p.split);
+        }
   return 0;
 }

@@ -78,3 +78,21 @@ def test_each_pair_of_parts_has_a_slot_of_its_own(dump, bn, split):
                     for row in range(128):
                         seen.add(slot * (128 * width * 4) + ((c - q * width) // 4 + j) * (128 * 16) + row * 16)
         assert len(seen) * 16 == recv and min(seen) == 0 and max(seen) == recv - 16
+
+
+def test_rule_runs_every_cluster_at_once(dump):
+    rules = [list(map(int, line[1:])) for line in dump if line[0] == "rule"]
+    assert len(rules) == 3 * 300 * 7 * 2
+    for clusters4, n, kiters, may, here, bn, split in rules:
+        tiles128 = (n + 1) // 2
+        assert bool(here) == (tiles128 <= 148)
+        if not here:
+            continue
+        tiles = n if bn == 64 else tiles128
+        assert tiles * split <= 148 and split <= kiters
+        assert split == 1 or may and kiters >= 16
+        if split == 4:
+            assert tiles <= clusters4       # clusters of four do not fill all SMs: 33 of 37 fit
+    split = lambda n, k, c: next(r[6] for r in rules if r[:4] == [c, n, k, 1])
+    assert [split(n, 64, 33) for n in (32, 33, 34, 37, 74)] == [4, 4, 2, 2, 2]
+    assert split(75, 16, 33) == 1 and split(75, 64, 33) == 2        # the latter on 128 columns

@@ -253,8 +253,9 @@ def test_grouped_gemm_pair_kernel(pkg, gpu):
     (1, 128, 128, 1088),    # parts of 4, 4, 4 and 5 steps
     (1, 128, 64, 8192),     # parts of 32 steps: four chains each with fp32 output
     (2, 128, 64, 8128),     # parts of 31 and 32 steps
-    (1, 128, 64 * 37, 1024),    # 37 tiles of 64: the last split in 4
-    (1, 128, 64 * 38, 1024),    # 38: the first split in 2
+    (1, 128, 64 * 33, 1024),    # 33 tiles of 64: as many clusters of 4 as run at once
+    (1, 128, 64 * 37, 1024),    # 37 and 38: clusters of 2
+    (1, 128, 64 * 38, 1024),
     (1, 128, 64 * 75, 1088),    # 75: not split
     (1, 128, 64 * 74, 1984),    # 74: split in 2, parts of 15 and 16 steps
     (1, 1024, 1152, 4096),      # 128 columns, split in 2
