@@ -82,11 +82,11 @@ const char* ptxb200_last_cuda_error(void);
  * ldc * sizeof(element) % 16 == 0.
  *
  * Few tiles, long K: products whose 128x128 output tiles number at most the SMs run
- * on smaller tiles, and with K long enough every tile is shared by the two or four
- * CTAs of a cluster, each summing a part of K; the parts meet in the CTAs' shared
- * memory (no scratch, no second kernel), and with fp32 output a CTA also sums its part
- * in several shorter chains. Results stay reproducible from launch to launch; they
- * differ in the last bits from the unsplit summation order, which
+ * on smaller tiles, and with K long enough every tile is shared by the two to eight
+ * CTAs of a cluster, each summing a part of K, in several shorter chains; the parts meet
+ * in the CTAs' shared memory (no scratch, no second kernel). Results stay reproducible
+ * from launch to launch on one GPU (how many clusters it runs at once decides between
+ * numbers of parts); they differ in the last bits from the unsplit summation order, which
  * PTXB200_GEMM_NO_SPLIT keeps. No reference counterpart
  * (test/gpu/blackwell/gemm_highperf_blackwell.jl:27-32 leaves it).
  *

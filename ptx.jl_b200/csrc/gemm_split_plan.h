@@ -20,22 +20,28 @@ constexpr int kChainSteps3 = 8;       // steps of K per accumulator
 constexpr int kCtrlBytes3 = ((2 * kMaxStages3 + 5) * 8 + 8 + 15) / 16 * 16;
 static_assert(kCtrlBytes3 % 16 == 0, "the parts handed over behind it are 16-byte pieces");
 
-// steps of K per ring stage: two of 24 KiB (64 columns), or one of 32 KiB
+// steps of K per ring stage: two of 24 KiB (64 columns), or one of 32 or 40 KiB
 PTXB200_PLAN_HD constexpr int stage_k3(int bn) { return bn == 64 ? 2 : 1; }
 PTXB200_PLAN_HD constexpr int stage_bytes3(int bn) { return stage_k3(bn) * (kABytes3 + bn * kBK3 * 2); }
 // accumulators that tensor memory (512 columns) holds; with more chains of sums than that, two
 // take turns and a third block of columns keeps what has been added up
 PTXB200_PLAN_HD constexpr int max_accs3(int bn) { return 512 / bn; }
-// what the other parts of the tile hand a CTA: [split - 1][bn / split / 4][128 rows] float4
-PTXB200_PLAN_HD constexpr int recv_bytes3(int bn, int split) { return (split - 1) * kBM3 * (bn / split) * 4; }
+// columns [part_col3(.., part), part_col3(.., part + 1)) of a tile are added up by one of its CTAs
+PTXB200_PLAN_HD constexpr int part_col3(int bn, int split, int part) { return bn / 16 * part / split * 16; }
+// what the other parts of the tile hand a CTA: [split - 1][columns / 4][128 rows] float4; a slot
+// has room for the widest share
+PTXB200_PLAN_HD constexpr int slot_bytes3(int bn, int split) { return kBM3 * ((bn / 16 + split - 1) / split * 16) * 4; }
+PTXB200_PLAN_HD constexpr int recv_bytes3(int bn, int split) { return (split - 1) * slot_bytes3(bn, split); }
 // steps [part_begin3(.., part), part_begin3(.., part + 1)) of K are one CTA's
 PTXB200_PLAN_HD constexpr int part_begin3(int kiters, int split, int part) {
   return (int)((long long)kiters * part / split);
 }
 
+constexpr int kMaxParts3 = 8;
+constexpr int kLongSteps3 = 192;      // steps of K from which handing over up to 7 shares pays
 struct GemmSplitPlan {
-  int bn;         // columns of a tile (128 rows): 64 or 128
-  int split;      // parts of K, one CTA of a cluster each: 1, 2 or 4
+  int bn;         // columns of a tile (128 rows): 64, 128 or 192
+  int split;      // parts of K, one CTA of a cluster each: 1 to 8
 };
 
 // Which products run on small tiles, and how: those whose 128x128 tiles fit the SMs in one round
@@ -44,16 +50,36 @@ struct GemmSplitPlan {
 // 64 columns as for 128 (1024^3: 6.7 against 7.7 us). K is split where SMs are left over and a
 // part keeps at least 4 (split in 4) or 8 (in 2) steps: handing the parts over costs
 // 1-2 us (384x640x1024: 5.8 in 4 parts, 6.7 whole; 512^3: 5.4 in 2 or 4 parts, 4.9 whole).
-// In 4 only where all clusters run at once (`clusters4`): 34 products of 128x64x1024 take two
+// In 4 only where all clusters run at once (`clusters[4]`): 34 products of 128x64x1024 take two
 // rounds and 11.8 us in 4 parts, 8.0 in 2; 33 take 7.8 and 8.0.
 // Half of K on tiles of 128 columns against all of it on tiles of 64, which use equally
 // many CTAs, pays from about 64 steps on (1024x1152: 16.1 against 16.5 us at 64 steps, 21.0
 // against 25.3 at 128, 11.7 against 10.5 at 32).
-inline bool gemm_split_rule(int sm_count, int clusters4, int groups, int M, int N, int kiters, bool may_split,
+// Long K: 128 columns in as many parts as run at once, down to 3 (but 8 or none where 64 columns
+// go in 4: 512x512x32768 34.1 us in 6 parts of 128 columns, 30.7 in 4 of 64), and 192 columns in 2
+// where a whole K on 128 leaves up to half of the SMs idle. 512x640x32768 47.7 -> 35.0 us,
+// 256x512x65536 49.0 -> 40.3, 640x1024x16384 33 (shares of one line of steps over all SMs) -> 29.3,
+// 1024x1280x16384 57.2 -> 49.0. The lines cross between 64 and 192 steps: at 128, 640x1024 21.2
+// and 18.6 but 128x10240 38.6 and 40.4; from 192 on no shape of a sweep was slower.
+inline bool gemm_split_rule(int sm_count, const int* clusters, int groups, int M, int N, int kiters, bool may_split,
                             GemmSplitPlan* plan) {
   const long long sms = sm_count, rows = (long long)groups * (M / kBM3);
   const long long tiles128 = rows * ((N + 127) / 128), tiles64 = rows * ((N + 63) / 64);
   if (tiles128 > sms) return false;
+  if (may_split && kiters >= kLongSteps3) {
+    const int parts[] = {8, 6, 5, 4, 3};
+    for (int s : parts)
+      if (tiles128 <= clusters[s] && (s == 8 || tiles64 > clusters[4])) {
+        plan->bn = 128;
+        plan->split = s;
+        return true;
+      }
+    if (tiles128 * 2 > sms && rows * ((N + 191) / 192) * 2 <= sms) {
+      plan->bn = 192;
+      plan->split = 2;
+      return true;
+    }
+  }
   plan->split = 1;
   if (tiles64 > sms || (may_split && kiters >= 64 && tiles64 * 2 > sms && tiles128 * 2 <= sms)) {
     plan->bn = 128;
@@ -61,7 +87,7 @@ inline bool gemm_split_rule(int sm_count, int clusters4, int groups, int M, int 
     return true;
   }
   plan->bn = 64;
-  if (may_split && kiters >= 16) plan->split = tiles64 <= clusters4 ? 4 : tiles64 * 2 <= sms ? 2 : 1;
+  if (may_split && kiters >= 16) plan->split = tiles64 <= clusters[4] ? 4 : tiles64 * 2 <= sms ? 2 : 1;
   return true;
 }
 
@@ -105,7 +131,7 @@ inline GemmSplitLayout gemm_split_layout(const GemmSplitPlan& p, int kiters, boo
   if (p.split > 1 && chains > accs && (steps + accs - 1) / accs <= limit) chains = accs;
   l.fold = p.split > 1 && chains > accs;
   l.chain_stages = (steps + chains - 1) / chains;
-  l.tmem_cols = p.bn;
+  l.tmem_cols = 64;      // a power of two
   const int blocks = l.fold ? 3 : p.split > 1 || chains < 2 ? chains : 2;
   while (l.tmem_cols < blocks * p.bn) l.tmem_cols *= 2;
   l.smem_bytes = l.stages * stage_bytes3(p.bn) + kCtrlBytes3 + recv;

@@ -1,9 +1,9 @@
 // gemm_bf16 for products with too few large tiles to fill the machine: one 128-row tile of
-// 64 or 128 columns per CTA, with K split over the 1, 2 or 4 CTAs of a cluster.
+// 64, 128 or 192 columns per CTA, with K split over the 1 to 8 CTAs of a cluster.
 //
 // What bounds such a product is not the tensor pipe but one CTA's chain: launch, tensor
-// maps, first loads, then about 0.16 us (64 columns) or 0.19 us (128) per 64 steps of K --
-// shared memory takes in and feeds out 24 or 32 KiB per step -- and the epilogue. So the
+// maps, first loads, then about 0.16 us (64 columns), 0.19 (128) or 0.25 (192) per step of 64
+// of K -- shared memory takes in and feeds out 24, 32 or 40 KiB per step -- and the epilogue. So the
 // work is spread over as many CTAs as there are SMs: small tiles first, then K. The parts
 // of a tile meet inside the cluster: every CTA sends each other one its share of the
 // columns of the partial sums with asynchronous stores into that CTA's shared memory
@@ -31,6 +31,8 @@
 //
 // Algorithmic work per launch: 2*G*M*N*K flop; compulsory bytes G*((M*K + N*K)*2 +
 // M*N*sizeof(out)).
+#include <array>
+
 #include "cta_pair.cuh"
 #include "gemm_epilogue.cuh"
 #include "host_common.h"
@@ -170,7 +172,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     }
     mbar_init(bar_parts, 1);
     mbar_fence_init();
-    if (kSplit) mbar_arrive_expect_tx(bar_parts, recv_bytes3(kBN, split));
+    if (kSplit) mbar_arrive_expect_tx(bar_parts, (split - 1) * kBM3 * 4 * (part_col3(kBN, split, part + 1) - part_col3(kBN, split, part)));
     if (!misaligned)
       for (int i = 0; i < stages && i < steps; ++i) load(i, i);
   }
@@ -299,20 +301,21 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       }
     }
     const int pieces = kFold ? 1 : chains;   // blocks of columns to add up
-    // every part sums up and writes bn / split columns: it sends the others theirs
-    const int width = kBN / split;
+    // every part sums up and writes its share of the columns: it sends the others theirs
+    const int my_col = part_col3(kBN, split, part), my_cols = part_col3(kBN, split, part + 1) - my_col;
     cluster_wait();
     if (epilogue) {
 #pragma unroll 1
       for (int i = 1; i < split; ++i) {
         const int q = part + i < split ? part + i : part + i - split;
         const uint32_t slot = part < q ? part : part - 1;
-        const uint32_t dst = map_to_cta(recv + slot * (kBM3 * width * 4), q) + row_in_tile * 16;
+        const uint32_t dst = map_to_cta(recv + slot * slot_bytes3(kBN, split), q) + row_in_tile * 16;
         const uint32_t dst_bar = map_to_cta(bar_parts, q);
+        const int first = part_col3(kBN, split, q), cols = part_col3(kBN, split, q + 1) - first;
 #pragma unroll 2
-        for (int c = 0; c < width; c += 16) {
+        for (int c = 0; c < cols; c += 16) {
           float x[16];
-          load_sum16<kBN>(t_row + q * width + c, pieces, x);
+          load_sum16<kBN>(t_row + first + c, pieces, x);
 #pragma unroll
           for (int j = 0; j < 4; ++j)
             st_async_v4(dst + (c / 4 + j) * (kBM3 * 16), dst_bar, x[4 * j], x[4 * j + 1], x[4 * j + 2], x[4 * j + 3]);
@@ -323,27 +326,27 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       if (pieces > 1) {
         // this CTA's own share is added up while the others' is on its way
 #pragma unroll 1
-        for (int c = 0; c < width; c += 16) {
+        for (int c = 0; c < my_cols; c += 16) {
           float x[16];
-          load_sum16<kBN>(t_row + part * width + c, pieces, x);
+          load_sum16<kBN>(t_row + my_col + c, pieces, x);
           uint32_t v[16];
 #pragma unroll
           for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(x[i]);
-          tmem_st16(t_row + part * width + c, v);
+          tmem_st16(t_row + my_col + c, v);
         }
         tc_wait_st();
       }
       mbar_wait<true>(bar_parts, 0, wctx, kSite3Parts);   // other CTAs' stores are read behind it
 #pragma unroll 1
-      for (int c = 0; c < width; c += 16) {
+      for (int c = 0; c < my_cols; c += 16) {
         float own[16], sum[16];
-        load_sum16<kBN>(t_row + part * width + c, 1, own);
+        load_sum16<kBN>(t_row + my_col + c, 1, own);
 #pragma unroll
         for (int i = 0; i < 16; ++i) sum[i] = 0.0f;
         // in the order of the parts, whoever adds them up
 #pragma unroll 1
         for (int q = 0; q < split; ++q) {
-          const float4* src = recv_ptr + (size_t)(q < part ? q : q - 1) * (kBM3 / 4 * width) + (c / 4) * kBM3 + row_in_tile;
+          const float4* src = recv_ptr + (q < part ? q : q - 1) * (slot_bytes3(kBN, split) / 16) + (c / 4) * kBM3 + row_in_tile;
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             float4 x = make_float4(own[4 * i], own[4 * i + 1], own[4 * i + 2], own[4 * i + 3]);
@@ -351,7 +354,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             sum[4 * i] += x.x; sum[4 * i + 1] += x.y; sum[4 * i + 2] += x.z; sum[4 * i + 3] += x.w;
           }
         }
-        const int col = col0 + part * width + c;
+        const int col = col0 + my_col + c;
         if (col < N) store_acc_chunk16<kF32Out>(c_out, row, ldc, col, sum);
       }
     }
@@ -417,36 +420,38 @@ int launch_parts3(const DeviceCtx& ctx, const GemmSplitPlan& p, const GemmSplitL
 }  // namespace
 
 bool gemm_split_choose(const DeviceCtx& ctx, int groups, int M, int N, int K, unsigned flags, GemmSplitPlan* plan) {
-  // Clusters of four CTAs that fill their SMs which the device runs at once: they do not straddle
-  // its groups of SMs, so that these are fewer than a quarter of its SMs (33 of 37).
+  // Clusters of n CTAs, each filling an SM, that the device runs at once: they do not straddle its
+  // groups of SMs, so that these are fewer than sm_count / n (33 of 37 for n = 4).
+  using Clusters = std::array<int, kMaxParts3 + 1>;
   static std::mutex mu;
-  static std::vector<int> clusters4;
-  int at_once = 0;
+  static std::vector<Clusters> known;
+  Clusters clusters;
   {
     std::lock_guard<std::mutex> lock(mu);
-    if ((int)clusters4.size() <= ctx.device) clusters4.resize(ctx.device + 1, -1);
-    int& known = clusters4[ctx.device];
-    if (known < 0) {
-      auto* kernel = gemm_split_kernel<64, false, true, false>;
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3((unsigned)(ctx.sm_count / 4 * 4));
-      cfg.blockDim = dim3(kThreads3);
-      cfg.dynamicSmemBytes = kSmemMax3;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim = {4, 1, 1};
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      known = 0;
-      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax3) != cudaSuccess ||
-          cudaOccupancyMaxActiveClusters(&known, kernel, &cfg) != cudaSuccess) {
-        known = 0;              // pairs then
-        cudaGetLastError();
+    if ((int)known.size() <= ctx.device) known.resize(ctx.device + 1, Clusters{});
+    Clusters& c = known[ctx.device];
+    if (c[1] == 0) {
+      c[1] = ctx.sm_count;
+      auto* kernel = gemm_split_kernel<128, false, true, false>;
+      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax3);
+      for (int n = 2; n <= kMaxParts3 && e == cudaSuccess; ++n) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(ctx.sm_count / n * n));
+        cfg.blockDim = dim3(kThreads3);
+        cfg.dynamicSmemBytes = kSmemMax3;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim = {(unsigned)n, 1, 1};
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        e = cudaOccupancyMaxActiveClusters(&c[n], kernel, &cfg);
+        if (e != cudaSuccess) c[n] = 0;
       }
+      if (e != cudaSuccess) cudaGetLastError();   // clusters of two then
     }
-    at_once = known;
+    clusters = c;
   }
-  return gemm_split_rule(ctx.sm_count, at_once, groups, M, N, K / kBK3, (flags & PTXB200_GEMM_NO_SPLIT) == 0, plan);
+  return gemm_split_rule(ctx.sm_count, clusters.data(), groups, M, N, K / kBK3, (flags & PTXB200_GEMM_NO_SPLIT) == 0, plan);
 }
 
 int launch_gemm_split(const DeviceCtx& ctx, const GemmSplitPlan& p, void* C, const void* A, const void* Bt, int groups,
@@ -455,6 +460,9 @@ int launch_gemm_split(const DeviceCtx& ctx, const GemmSplitPlan& p, void* C, con
   const int kiters = K / kBK3;
   const int longest = (flags & PTXB200_GEMM_NO_SPLIT) ? 0 : gemm_line(ctx.sm_count, groups, M, N, kiters).share;
   const GemmSplitLayout l = gemm_split_layout(p, kiters, f32, longest);
+  if (p.bn == 192)                    // always two parts, whose chains never fold
+    return f32 ? launch_one3<192, true, true, false>(ctx, p, l, C, A, Bt, groups, M, N, K, ldc, stream)
+               : launch_one3<192, false, true, false>(ctx, p, l, C, A, Bt, groups, M, N, K, ldc, stream);
   if (p.bn == 64)
     return f32 ? launch_parts3<64, true>(ctx, p, l, C, A, Bt, groups, M, N, K, ldc, stream)
                : launch_parts3<64, false>(ctx, p, l, C, A, Bt, groups, M, N, K, ldc, stream);

@@ -264,6 +264,15 @@ def test_grouped_gemm_pair_kernel(pkg, gpu):
     (4, 256, 64 * 19, 512),     # 152 of 64: 128 columns, the last tile half-empty
     (1, 512, 128 * 37, 576),    # 148 tiles of 128
     (1, 512, 128 * 38, 192),    # 152: the persistent kernels
+    (1, 128, 128 * 15, 12288),  # long K, 128 columns: 15 tiles in 8 parts
+    (1, 128, 64 * 41, 12352),   # 21 in 6, the last half-empty: shares of 16 and 32 columns, uneven parts of K
+    (2, 128, 128 * 12, 12352),  # 24 in 5
+    (1, 128, 128 * 31, 12352),  # 31 in 4
+    (5, 128, 64 * 17, 12288),   # 45 in 3: shares of 32 and 48 columns
+    (1, 128, 128 * 46, 12352),  # 46 in 2
+    (1, 1024, 1280, 12352),     # 192 columns in 2 parts, the last tile with 128 columns
+    (3, 384, 576, 12288),       # the same, groups, full tiles
+    (1, 1408, 1088, 12288),     # 128 columns, not split: 192 would need more than 74 clusters
     (1, 2304, 2304, 1024),      # pair tiles of 192 columns
     (1, 2432, 2368, 832),       # the same, half-filled row-tile, 64 columns over
     (5, 1024, 512, 512),        # the same, groups
