@@ -169,12 +169,13 @@ int swiglu_f32(void* out, const void* gate, const void* up, long long n, void* s
  * SMs -- and cutting pays, the items of that round are cut along the key axis into equal
  * shares for all SMs; the pieces of an item meet, unnormalised and in fp32, in scratch
  * that the library keeps per (device, stream) (about 133 KB per SM at D = 128, allocated
- * with cudaMalloc by the first such launch on a stream -- make it outside stream capture
- * -- and freed by ptxb200_shutdown; see gemm_bf16 for the table's bound), and the CTA
+ * with cudaMalloc by the first such launch on a stream, at most 16 buffers per process,
+ * recycled least recently used, and freed by ptxb200_shutdown), and the CTA
  * that holds an item's first keys merges them by the log-sum-exp rule before the one
  * rounding to bf16. Results stay reproducible from launch to launch on one GPU model;
  * they differ in the last bits from the uncut key order, which PTXB200_FA_NO_TAIL_SPLIT
- * keeps. The CTAs of such a launch wait for one another's pieces (bounded, like every
+ * keeps and which launches in a stream capture take (the scratch is the stream's, not a
+ * graph's). The CTAs of such a launch wait for one another's pieces (bounded, like every
  * wait here), so they must be able to run at the same time: do not run other work that
  * occupies the GPU's SMs for seconds concurrently with it.
  *

@@ -1503,9 +1503,21 @@ int launch_fa_fwd(const DeviceCtx& ctx, void* O, void* lse, const void* Q, const
   if ((rc = encode_tmap_bf16_3d(&tk, K, (uint64_t)B * H_kv, S, D, 128, 64)) != PTXB200_OK) return rc;
   if ((rc = encode_tmap_bf16_3d(&tv, V, (uint64_t)B * H_kv, S, D, 128, 64)) != PTXB200_OK) return rc;
   FaParams p;
-  fill_params(p, O, lse, B, H, H_kv, S, sm_scale, flags, dbg, status,
-              plan_schedule(B * H, (S + 255) / 256, (S + kAttnRows - 1) / kAttnRows, causal, flags, ctx.sm_count, true,
-                            4ll * B * H_kv * S * D));
+  const long long kv_bytes = 4ll * B * H_kv * S * D;
+  auto plan = [&](bool may_split) {
+    return plan_schedule(B * H, (S + 255) / 256, (S + kAttnRows - 1) / kAttnRows, causal, flags, ctx.sm_count, may_split,
+                         kv_bytes);
+  };
+  FaSched sched = plan(true);
+  if (sched.tail_units > 0) {
+    // Not cut in a captured launch: its replays would carry one epoch, so that the second takes the
+    // first one's pieces for its own, and could run beside the stream whose scratch they use, or
+    // after that scratch is freed.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    PTXB200_CUDA_TRY(cudaStreamIsCapturing(stream, &capture));
+    if (capture != cudaStreamCaptureStatusNone) sched = plan(false);
+  }
+  fill_params(p, O, lse, B, H, H_kv, S, sm_scale, flags, dbg, status, sched);
   ScratchLease lease;
   if (p.sched.tail_units > 0) {
     // one slot of parked pieces and one flag per CTA, kept per (device, stream)

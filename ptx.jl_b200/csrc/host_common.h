@@ -66,8 +66,8 @@ class PerDeviceOnce {
 // partial results in global memory: launches on one stream run one after the other and
 // may share a buffer, launches on different streams may overlap and must not.
 //  * scratch_acquire returns a buffer of at least `bytes` for (current device, stream,
-//    kind), allocating or growing it when needed (cudaMalloc: the first such launch on a
-//    stream must come outside stream capture).
+//    kind), allocating or growing it when needed (cudaMalloc). Not for captured launches:
+//    a graph outlives the lease and may replay on another stream.
 //  * scratch_mark_used, called after the kernels that use the buffer are enqueued, records
 //    an event so that the buffer can later be recycled safely.
 //  * At most kScratchMaxEntries buffers exist per process: when a new (device, stream,

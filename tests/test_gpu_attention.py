@@ -419,3 +419,39 @@ def test_last_tile_edges_against_64_bit(pkg, gpu, S, D, causal):
     torch.testing.assert_close(lse.view(B, H, S).double(), torch.logsumexp(scores, dim=-1), rtol=1e-5, atol=1e-4)
     if causal:
         assert torch.equal(o[:, :, 0], v.repeat_interleave(H // Hkv, dim=1)[:, :, 0])   # masked keys weigh exactly zero
+
+
+@pytest.mark.parametrize("B,H,S,D,causal", [(1, 12, 1920, 128, False), (1, 2, 4096, 64, True), (1, 3, 4000, 128, True)])
+def test_replays_of_a_captured_launch_use_their_own_inputs(pkg, gpu, B, H, S, D, causal):
+    """Launches that would cut the last round: every replay of a graph gives what its inputs
+    give uncut, whatever ran before on the stream, and eager launches go on being cut."""
+    g = torch.Generator(device=gpu).manual_seed(S)
+    q, k, v = (torch.empty(B, H, S, D, dtype=torch.bfloat16, device=gpu) for _ in range(3))
+    cut = dict(causal=causal, flags=pkg.native.FA_ALWAYS_TAIL_SPLIT)
+
+    def draw():
+        for t in (q, k, v):
+            t.copy_(torch.randn(B, H, S, D, generator=g, device=gpu))
+
+    draw()
+    stream = torch.cuda.Stream()
+    out = torch.empty_like(q)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        want_cut = pkg.ops.fa_fwd(q, k, v, **cut)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            pkg.ops.fa_fwd(q, k, v, out=out, **cut)
+        for _ in range(4):
+            draw()
+            out.fill_(float("nan"))
+            graph.replay()
+            want = pkg.ops.fa_fwd(q, k, v, causal=causal, flags=pkg.native.FA_NO_TAIL_SPLIT)
+            assert torch.equal(out, want)
+        big = torch.randn(1, 2, 4096, 128, generator=g, device=gpu).to(torch.bfloat16)
+        pkg.ops.fa_fwd(big, big, big, **cut)             # more scratch on the same stream: no error left behind
+        again = pkg.ops.fa_fwd(q, k, v, **cut)
+        torch.testing.assert_close(again.float(), want.float(), atol=2e-2, rtol=0)
+    status = pkg.ops.sync_status()
+    assert status == 0, pkg.native.strerror(status)
+    assert want_cut.shape == want.shape
