@@ -269,11 +269,20 @@ int fa_fwd_bf16_noalloc_status(uint32_t* cta_flags_out, int max_flags, void* str
  * segment (block, batch*head, first tile, end tile, tiles of the item, pieces parked by
  * following CTAs). Returns the ints written, PTXB200_E_CAPACITY if cap is too small.
  * Causal launches whose K and V (all heads) are at most 160 MiB may instead deal their
- * items by length over all heads, without pairs or a cut; that is not shown here (the
- * choice needs the head dim and the number of K/V heads).
+ * items by length over all heads, without pairs or a cut; that choice needs the head dim
+ * and the number of K/V heads: ptxb200_fa_plan_ex.
  * The reference's distribution is the round robin of flash_attention_defs.jl:269-272.
  */
 int ptxb200_fa_plan(int B, int H, int S, int causal, unsigned flags, int sm_count, int* out, int cap);
+
+/*
+ * The same for fa_fwd_bf16_ex, and what such a launch does (outside a stream capture): an
+ * eleventh int follows the first 10, 1 if the items are dealt by length -- item r in the
+ * order (block falling, then batch*head) goes to CTA r mod CTAs in even rounds and to the
+ * CTAs in reverse in odd ones -- and 0 if not.
+ */
+int ptxb200_fa_plan_ex(int B, int H, int H_kv, int S, int D, int causal, unsigned flags, int sm_count, int* out,
+                       int cap);
 
 /*
  * Synchronise `stream`, then return and clear that stream's status word on the

@@ -1279,8 +1279,9 @@ constexpr int kSplitOverheadSteps = 3;   // what a second segment, parking and m
 constexpr int kSplitMaxRounds = 64;      // beyond this many full rounds the tail is noise: not split
 constexpr int kItemOverheadSteps = 1;    // what the boundary between two items costs a CTA, in steps (measured: 1-1.5)
 // K and V of all heads together up to about L2's size (126 MB) are read from HBM once or little
-// more whatever the order of the items (measured to 134 MB); above it pairs, which keep a
-// head's CTAs together, do that.
+// more whatever the order of the items; above it pairs, which keep a head's CTAs together, do
+// that. Measured from 134 MB to this limit: 0.99 to 1.27 times as fast as pairs or a cut (5 x 32
+// heads of 1843 keys, 151 MB, 233 us and 183; 6 x 32 on 8 heads of 6400 keys, 157 MB, 1884 and 1899).
 constexpr long long kByLengthMaxKvBytes = 160ll << 20;
 constexpr int kByLengthMaxItems = 1 << 16;
 
@@ -1544,13 +1545,14 @@ int launch_fa_fwd(const DeviceCtx& ctx, void* O, void* lse, const void* Q, const
 
 // The distribution plan_schedule picks and every tail CTA's segments, for tests on a
 // machine without a GPU. out: 10 ints of FaSched (num_mblocks, bh, nt_all, causal, pair_mode,
-// grid, full_units, tail_units, tail_steps, tail_ctas), then per tail CTA its segment count
+// grid, full_units, tail_units, tail_steps, tail_ctas), by_length if kv_bytes is given, then per tail CTA its segment count
 // followed by 6 ints per segment (mb, bh, j0, j1, len, n_other). Returns the ints written,
 // or -1 if `cap` is too small.
-int describe_fa_plan(int BH, int S, int causal, unsigned flags, int sm_count, int* out, int cap) {
+int describe_fa_plan(int BH, int S, long long kv_bytes, int causal, unsigned flags, int sm_count, int* out, int cap) {
   const int nmb = (S + 255) / 256, nt_all = (S + kAttnRows - 1) / kAttnRows;
-  // neither head dim nor K/V heads are known here: as for K and V too large for the order by length
-  const FaSched sc = plan_schedule(BH, nmb, nt_all, causal, flags, sm_count, true, kByLengthMaxKvBytes + 1);
+  // not known how large K and V are: as for too large for the order by length
+  const FaSched sc = plan_schedule(BH, nmb, nt_all, causal, flags, sm_count, true,
+                                   kv_bytes < 0 ? kByLengthMaxKvBytes + 1 : kv_bytes);
   int n = 0;
   auto put = [&](int v) {
     if (n < cap) out[n] = v;
@@ -1558,6 +1560,7 @@ int describe_fa_plan(int BH, int S, int causal, unsigned flags, int sm_count, in
   };
   put(sc.num_mblocks); put(sc.bh); put(sc.nt_all); put(sc.causal); put(sc.pair_mode);
   put(sc.grid); put(sc.full_units); put(sc.tail_units); put(sc.tail_steps); put(sc.tail_ctas);
+  if (kv_bytes >= 0) put(sc.by_length);
   if (sc.tail_units > 0) {
     std::vector<int> starts(sc.tail_units + 1, 0);
     for (int u = 0; u < sc.tail_units; ++u) {

@@ -86,6 +86,8 @@ def lib() -> ctypes.CDLL:
     L.ptxb200_sync_status.argtypes = [vp]
     L.ptxb200_fa_plan.restype = ci
     L.ptxb200_fa_plan.argtypes = [ci, ci, ci, ci, cu, ci, vp, ci]
+    L.ptxb200_fa_plan_ex.restype = ci
+    L.ptxb200_fa_plan_ex.argtypes = [ci, ci, ci, ci, ci, ci, cu, ci, vp, ci]
     L.ptxb200_device_status.restype = ci
     L.ptxb200_device_status.argtypes = []
     L.ptxb200_selftest.restype = ci
