@@ -21,6 +21,11 @@ int main() {
             for (int part = 0; part <= split; ++part) std::printf(" %d", part_col3(bn, split, part));
             std::printf("\n");
           }
+  for (int tiles : {1, 2, 4, 9, 32, 40, 74, 75, 100})
+    for (int kiters : {1, 8, 15, 16, 17, 64, 128, 1024, 4096}) {
+      const GemmLine line = gemm_line(148, tiles, 128, 192, kiters);   // a product of one 128x256 tile each
+      std::printf("line %d %d %d %d\n", tiles, kiters, line.ctas, line.share);
+    }
   // the rule, for products of one row-tile and n columns of 64, on 148 SMs
   const int none[kMaxParts3 + 1] = {0, 148}, b200[kMaxParts3 + 1] = {0, 148, 74, 45, 33, 26, 22, 15, 15},
             all[kMaxParts3 + 1] = {0, 148, 74, 49, 37, 29, 24, 21, 18};

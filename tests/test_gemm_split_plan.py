@@ -107,3 +107,19 @@ def test_rule_runs_every_cluster_at_once(dump):
     assert split(34, 192, 1) == [128, 6] and split(90, 192, 1) == [128, 3]
     assert split(91, 192, 1) == [128, 2] and split(149, 192, 1) == [192, 2] and split(149, 191, 1) == [128, 1]
     assert split(223, 192, 1) == [128, 1]
+
+
+def test_shares_of_one_line_of_steps(dump):
+    """What bounds the chains of sums: at most half as many 128x256 tiles as SMs, shares of at
+    least eight steps, two shares or more per tile; otherwise all of K."""
+    n = 0
+    for tiles, kiters, ctas, share in (map(int, line[1:]) for line in dump if line[0] == "line"):
+        want = min(tiles * kiters // 8, 148)
+        if tiles > 74 or want < 2 * tiles:
+            assert (ctas, share) == (0, kiters)
+        else:
+            assert ctas == want and 8 <= share == -(-tiles * kiters // ctas) < kiters
+            n += 1
+    assert n > 20
+    line = {(int(l[1]), int(l[2])): (int(l[3]), int(l[4])) for l in dump if l[0] == "line"}
+    assert line[(1, 128)] == (16, 8) and line[(32, 128)] == (148, 28) and line[(75, 128)] == (0, 128)

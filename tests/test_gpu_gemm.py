@@ -134,17 +134,17 @@ def test_grouped_gemm_equals_per_group_calls(pkg, gpu):
 
 
 # ---------------------------------------------------------------------------
-# Tiles cut along K (no reference counterpart): at most half as many tiles as SMs,
-# K long enough for the split to pay.
+# K split over the CTAs of clusters (no reference counterpart): few tiles, K long enough
+# for the split to pay.
 # ---------------------------------------------------------------------------
 @pytest.mark.parametrize("M,N,K", [
-    (128, 256, 8192),     # one tile shared by 16 CTAs
-    (128, 128, 4096),     # one ragged tile
-    (256, 512, 4096),     # 4 tiles, 32 CTAs, 8 iterations each
-    (384, 768, 2048),     # 9 tiles: shares cross tile boundaries unevenly
-    (1024, 1024, 8192),   # 32 tiles on 148 CTAs: most CTAs hold two partial tiles
-    (1152, 2048, 4096),   # 72 tiles, just under half the SMs
-    (2048, 4096, 8192),   # 256 tiles: not split (the flag then changes nothing)
+    (128, 256, 8192),     # four tiles of 64 columns in 4 parts
+    (128, 128, 4096),     # two in 4 parts
+    (256, 512, 4096),     # 16 in 4 parts of 16 steps
+    (384, 768, 2048),     # 36 in 2 parts
+    (1024, 1024, 8192),   # 64 tiles of 128 columns in 2 parts
+    (1152, 2048, 4096),   # 144 of 128 columns, not split
+    (2048, 4096, 8192),   # too many tiles for the split kernel (the flag then changes nothing)
 ])
 @pytest.mark.parametrize("f32_out", [True, False])
 def test_gemm_split_tail_matches_oracle_and_unsplit(pkg, gpu, oracle_mod, M, N, K, f32_out):
@@ -169,7 +169,7 @@ def test_gemm_split_tail_matches_oracle_and_unsplit(pkg, gpu, oracle_mod, M, N, 
 
 
 def test_grouped_gemm_split_tail(pkg, gpu):
-    """Groups and the K split compose: 10 groups x 3 tiles shared by 148 CTAs."""
+    """Groups and the K split compose: 10 groups x 6 tiles of 128 columns in 2 parts."""
     G, M, N, K = 10, 128, 768, 4096
     g = torch.Generator().manual_seed(77)
     a = (torch.randn(G, M, K, generator=g) * 0.1).to(torch.bfloat16).to(gpu)
@@ -181,7 +181,7 @@ def test_grouped_gemm_split_tail(pkg, gpu):
 
 
 def test_gemm_split_on_two_streams(pkg, gpu):
-    """Scratch is per stream: split launches that overlap on two streams stay correct."""
+    """Split launches that overlap on two streams stay correct."""
     M, N, K = 256, 512, 8192
     g = torch.Generator().manual_seed(9)
     a = (torch.randn(M, K, generator=g) * 0.1).to(torch.bfloat16).to(gpu)

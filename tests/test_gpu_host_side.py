@@ -48,25 +48,22 @@ def test_two_threads_two_streams_match_serial(pkg, gpu):
         assert torch.equal(outs_c[i], want_c[i])
 
 
-def test_scratch_table_recycles_beyond_its_capacity(pkg, gpu):
-    """More streams than the scratch table has entries (16): the least recently used
-    buffer is waited for and recycled, results stay those of the first launch."""
+def test_split_gemm_holds_no_memory(pkg, gpu):
+    """K split over the CTAs of clusters takes no scratch: forty streams hold no more memory than
+    one, and their results are those of the first launch."""
     g = torch.Generator().manual_seed(99)
     a = (torch.randn(128, 4096, generator=g) * 0.1).to(torch.bfloat16).to(gpu)
     bt = (torch.randn(256, 4096, generator=g) * 0.1).to(torch.bfloat16).to(gpu)
     want = pkg.ops.gemm(a, bt, f32_out=True)
-    free_before = None
     streams = [torch.cuda.Stream() for _ in range(40)]
     outs = [torch.empty_like(want) for _ in streams]
-    for rnd in range(2):
-        for st, o in zip(streams, outs):
-            pkg.ops.gemm(a, bt, out=o, f32_out=True, stream=st)
-        torch.cuda.synchronize()
-        free = torch.cuda.mem_get_info()[0]
-        if free_before is None:
-            free_before = free
-        # a second pass over 40 streams holds no more memory than the first
-        assert free >= free_before - (8 << 20)
+    pkg.ops.gemm(a, bt, out=outs[0], f32_out=True, stream=streams[0])
+    torch.cuda.synchronize()
+    free_before = torch.cuda.mem_get_info()[0]
+    for st, o in zip(streams, outs):
+        pkg.ops.gemm(a, bt, out=o, f32_out=True, stream=st)
+    torch.cuda.synchronize()
+    assert torch.cuda.mem_get_info()[0] >= free_before - (8 << 20)
     assert pkg.ops.sync_status() == 0
     for o in outs:
         assert torch.equal(o, want)
@@ -93,19 +90,28 @@ def test_status_word_is_per_stream(pkg, gpu):
 
 
 def test_attention_scratch_recycles_beyond_its_capacity(pkg, gpu):
-    """The same with attention launches whose last round is cut, which park pieces in the table's
-    buffers: results stay those of the first launch on twenty streams, twice over."""
+    """More streams than the scratch table has entries (16), with launches whose cut last round
+    parks pieces in them: the least recently used buffer is waited for and freed, so that the
+    table never holds more than sixteen, and results stay those of the first launch."""
     g = torch.Generator().manual_seed(17)
     q, k, v = ((torch.randn(1, 2, 1024, 64, generator=g)).to(torch.bfloat16).to(gpu) for _ in range(3))
     cut = dict(causal=True, flags=pkg.native.FA_ALWAYS_TAIL_SPLIT)
-    want = pkg.ops.fa_fwd(q, k, v, **cut)
-    streams = [torch.cuda.Stream() for _ in range(20)]
-    outs = [torch.empty_like(want) for _ in streams]
     torch.cuda.synchronize()
+    assert pkg.native.lib().ptxb200_shutdown() == 0      # an empty table, whatever ran before
+    want = pkg.ops.fa_fwd(q, k, v, **cut)
+    streams = [torch.cuda.Stream() for _ in range(40)]   # (thirty-two of torch's pool)
+    outs = [torch.empty_like(want) for _ in streams]
+    # a slot per SM: 2 stages of 128 rows, 64 fp32 columns and two statistics each
+    buffer = torch.cuda.get_device_properties(gpu).multi_processor_count * 2 * 128 * 66 * 4
+    torch.cuda.synchronize()
+    free_before = torch.cuda.mem_get_info()[0]
     for _ in range(2):
         for st, o in zip(streams, outs):
             pkg.ops.fa_fwd(q, k, v, out=o, stream=st, **cut)
-    torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        # (every buffer is a multiple of the allocator's 2 MiB)
+        assert free_before - torch.cuda.mem_get_info()[0] <= 16 * (buffer + (2 << 20))
+    assert free_before - torch.cuda.mem_get_info()[0] >= 8 * buffer     # the launches do use scratch
     assert pkg.ops.sync_status() == 0
     for o in outs:
         assert torch.equal(o, want)
