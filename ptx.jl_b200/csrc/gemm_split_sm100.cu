@@ -103,13 +103,14 @@ template <int kBN, bool kF32Out, bool kSplit, bool kFold>
 __global__ void __launch_bounds__(kThreads3, 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                   void* __restrict__ c_out, int M, int N, int K, int ldc, int split, int stages, int chain_stages,
-                  uint32_t tmem_cols, uint32_t* status) {
+                  uint32_t tmem_cols, unsigned long long part_cols, int slot_bytes, uint32_t* status) {
   if constexpr (!kSplit) split = 1;
   constexpr int kStageK = stage_k3(kBN), kStageBytes = stage_bytes3(kBN);
   constexpr int kAtomBytes = kABytes3 + kBN * kBK3 * 2;
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t base = smem_u32(smem);
   const int part = kSplit ? (int)cluster_ctarank() : 0;   // which part of K this CTA of the cluster sums
+  const int my_col = unpack_col3(part_cols, part), my_cols = unpack_col3(part_cols, part + 1) - my_col;   // what it adds up
 
   const uint32_t ctrl = base + stages * kStageBytes;
   uint8_t* ctrl_ptr = smem + stages * kStageBytes;
@@ -172,7 +173,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     }
     mbar_init(bar_parts, 1);
     mbar_fence_init();
-    if (kSplit) mbar_arrive_expect_tx(bar_parts, (split - 1) * kBM3 * 4 * (part_col3(kBN, split, part + 1) - part_col3(kBN, split, part)));
+    if (kSplit) mbar_arrive_expect_tx(bar_parts, (split - 1) * kBM3 * 4 * my_cols);
     if (!misaligned)
       for (int i = 0; i < stages && i < steps; ++i) load(i, i);
   }
@@ -302,16 +303,15 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     }
     const int pieces = kFold ? 1 : chains;   // blocks of columns to add up
     // every part sums up and writes its share of the columns: it sends the others theirs
-    const int my_col = part_col3(kBN, split, part), my_cols = part_col3(kBN, split, part + 1) - my_col;
     cluster_wait();
     if (epilogue) {
 #pragma unroll 1
       for (int i = 1; i < split; ++i) {
         const int q = part + i < split ? part + i : part + i - split;
         const uint32_t slot = part < q ? part : part - 1;
-        const uint32_t dst = map_to_cta(recv + slot * slot_bytes3(kBN, split), q) + row_in_tile * 16;
+        const uint32_t dst = map_to_cta(recv + slot * slot_bytes, q) + row_in_tile * 16;
         const uint32_t dst_bar = map_to_cta(bar_parts, q);
-        const int first = part_col3(kBN, split, q), cols = part_col3(kBN, split, q + 1) - first;
+        const int first = unpack_col3(part_cols, q), cols = unpack_col3(part_cols, q + 1) - first;
 #pragma unroll 2
         for (int c = 0; c < cols; c += 16) {
           float x[16];
@@ -346,7 +346,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         // in the order of the parts, whoever adds them up
 #pragma unroll 1
         for (int q = 0; q < split; ++q) {
-          const float4* src = recv_ptr + (q < part ? q : q - 1) * (slot_bytes3(kBN, split) / 16) + (c / 4) * kBM3 + row_in_tile;
+          const float4* src = recv_ptr + (q < part ? q : q - 1) * (slot_bytes / 16) + (c / 4) * kBM3 + row_in_tile;
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             float4 x = make_float4(own[4 * i], own[4 * i + 1], own[4 * i + 2], own[4 * i + 3]);
@@ -406,7 +406,8 @@ int launch_one3(const DeviceCtx& ctx, const GemmSplitPlan& p, const GemmSplitLay
   cfg.attrs = attr;
   cfg.numAttrs = kSplit ? 1 : 0;
   PTXB200_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_split_kernel<kBN, kF32Out, kSplit, kFold>, ta, tb, C, M, N, K, ldc, p.split,
-                                      l.stages, l.chain_stages, (uint32_t)l.tmem_cols, status_word(ctx, stream)));
+                                      l.stages, l.chain_stages, (uint32_t)l.tmem_cols, part_cols3(kBN, p.split), slot_bytes3(kBN, p.split),
+                                      status_word(ctx, stream)));
   return PTXB200_OK;
 }
 

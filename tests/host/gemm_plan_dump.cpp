@@ -18,7 +18,7 @@ int main() {
             std::printf("layout %d %d %d %d %d %d %d %d %d %d %d %d", bn, split, kiters, f32, longest, l.stages,
                         l.chain_stages, l.fold ? 1 : 0, l.tmem_cols, l.smem_bytes, recv_bytes3(bn, split), stage_k3(bn));
             for (int part = 0; part <= split; ++part) std::printf(" %d", part_begin3(kiters, split, part));
-            for (int part = 0; part <= split; ++part) std::printf(" %d", part_col3(bn, split, part));
+            for (int part = 0; part <= split; ++part) std::printf(" %d", unpack_col3(part_cols3(bn, split), part));
             std::printf("\n");
           }
   for (int tiles : {1, 2, 4, 9, 32, 40, 74, 75, 100})
