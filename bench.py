@@ -53,7 +53,7 @@ ROWWISE_WORKLOADS = {"softmax": (65536, 4096, 20260011), "rms_norm": (65536, 409
 # read and written once: profiles/rowwise_softmax_n4096.md)
 NCU_TRAFFIC_BYTES = {"c2": 201.44e6 + 43.03e6, "c3": 201.39e6 + 45.83e6, "c4": 1649.54e6 + 517.57e6,
                      "c5": 1067.3e6 + 131.1e6,
-                     "softmax": 4 * (268.45e6 + 218.52e6)}
+                     "softmax": 4 * (268.46e6 + 213.83e6)}
 FALLBACK_PEAK_TFLOPS = 1590.0
 FALLBACK_PEAK_GBS = 6650.0
 
@@ -435,7 +435,8 @@ def quantisation_note(pkg, name, world, sm):
         M, N, K, _ = GEMM_WORKLOADS[name]
         tiles = (M // 256) * ((N // world) // 256)
         waves = tiles / (sm // 2)
-        return f"{tiles} tiles of 256x256 on {sm // 2} SM pairs = {waves:.2f} waves: at most {waves / math.ceil(waves):.2f} of linear"
+        return (f"{tiles} tiles of 256x256 on {sm // 2} SM pairs = {waves:.2f} waves: {waves / math.ceil(waves):.2f} of linear "
+                f"with these; narrower tiles are taken where they fill the last wave better")
     B, H, S, D, causal, _, _ = WORKLOADS[name]
     items = (B * H // world) * ((S + 255) // 256)
     waves = items / sm

@@ -17,17 +17,18 @@
 // 5e-8 of the result per step of a chain (1024x1152x8192 split in 2, fp32 out: one chain of 64
 // steps 4.0e-6, four of 16 8.5e-7, of 8 4.0e-7). With fp32 output a chain has at most 8 steps where
 // the accumulators suffice (64 columns: 8 of them, 128: 4), and with either output never more
-// than the shares of one line of steps over all SMs would (gemm_line: 8 to 62). Where K is split each chain has
-// an accumulator of its own and the epilogue adds them up; with more chains than that two
-// accumulators take turns and the epilogue's warps fold them into a third as they end, which
-// costs 0.1 us per chain (128x256x65536 fp32 out, 32 chains: 48.5 us and 4.1e-7; 8 chains of 32:
-// 47.4 and 1.9e-6). Where K is not split the epilogue's warps take each chain into registers while the
-// next one runs (1024x1280x4096: fp32 out 18.6 us in chains of 8, bf16 17.8 in chains of 16, 17.0 in one).
+// than the shares of one line of steps over all SMs would (gemm_line: 8 to 62). Where K is split
+// each chain has an accumulator of its own and the epilogue adds them up; with more chains than
+// that two accumulators take turns and the epilogue's warps fold them into a third as they end,
+// which costs 0.1 us per chain (128x256x65536 in 4 parts, fp32 out: 32 chains 48.5 us and 4.1e-7, 8
+// chains of 32 steps 47.4 and 1.9e-6; in 8 parts 39.6 and 4.0e-7). Where K is not split the
+// epilogue's warps take each chain into registers while the next one runs (1024x1280x4096: fp32
+// out 18.6 us in chains of 8, bf16 17.8 in chains of 16, 17.0 in one).
 //
 // Measured (device time, bf16 out unless noted; before: 128x256 tiles cut into shares of
 // one k-iteration line, partial tiles parked in global memory, a second kernel to add
-// them up): 128x4096x4096 20.4 -> 12.5 us; 1024x1152x8192 fp32 out 33.5 -> 21.0; 1024^3
-// 14.6 -> 6.7; 512^3 7.9 -> 4.9; 128x128x8192 16.6 -> 9.9.
+// them up): 128x4096x4096 19.1 -> 12.5 us; 1024x1152x8192 fp32 out 33.1 -> 23.0; 1024^3
+// 14.5 -> 6.6; 512^3 8.0 -> 4.9; 128x128x8192 14.9 -> 9.7; 128x256x65536 61.0 -> 39.3.
 //
 // Algorithmic work per launch: 2*G*M*N*K flop; compulsory bytes G*((M*K + N*K)*2 +
 // M*N*sizeof(out)).
