@@ -48,6 +48,7 @@ int current_ctx(DeviceCtx** out) {
       set_error_text("current device is not compute capability 10.x (sm_100a code only)");
       return PTXB200_E_DEVICE;
     }
+    query_clusters(c.sm_count, c.clusters);
     PTXB200_CUDA_TRY(cudaMalloc((void**)&c.workspace, kWsWords * sizeof(uint32_t)));
     PTXB200_CUDA_TRY(cudaMemset(c.workspace, 0, kWsWords * sizeof(uint32_t)));
     g_ctx[dev] = new DeviceCtx(c);

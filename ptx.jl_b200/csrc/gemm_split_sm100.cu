@@ -32,8 +32,6 @@
 //
 // Algorithmic work per launch: 2*G*M*N*K flop; compulsory bytes G*((M*K + N*K)*2 +
 // M*N*sizeof(out)).
-#include <array>
-
 #include "cta_pair.cuh"
 #include "gemm_epilogue.cuh"
 #include "host_common.h"
@@ -421,39 +419,29 @@ int launch_parts3(const DeviceCtx& ctx, const GemmSplitPlan& p, const GemmSplitL
 
 }  // namespace
 
-bool gemm_split_choose(const DeviceCtx& ctx, int groups, int M, int N, int K, unsigned flags, GemmSplitPlan* plan) {
-  // Clusters of n CTAs, each filling an SM, that the device runs at once: they do not straddle its
-  // groups of SMs, so that these are fewer than sm_count / n (33 of 37 for n = 4).
-  using Clusters = std::array<int, kMaxParts3 + 1>;
-  static std::mutex mu;
-  static std::vector<Clusters> known;
-  Clusters clusters;
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    if ((int)known.size() <= ctx.device) known.resize(ctx.device + 1, Clusters{});
-    Clusters& c = known[ctx.device];
-    if (c[1] == 0) {
-      c[1] = ctx.sm_count;
-      auto* kernel = gemm_split_kernel<128, false, true, false>;
-      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax3);
-      for (int n = 2; n <= kMaxParts3 && e == cudaSuccess; ++n) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)(ctx.sm_count / n * n));
-        cfg.blockDim = dim3(kThreads3);
-        cfg.dynamicSmemBytes = kSmemMax3;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim = {(unsigned)n, 1, 1};
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        e = cudaOccupancyMaxActiveClusters(&c[n], kernel, &cfg);
-        if (e != cudaSuccess) c[n] = 0;
-      }
-      if (e != cudaSuccess) cudaGetLastError();   // clusters of two then
-    }
-    clusters = c;
+void query_clusters(int sm_count, int (&clusters)[kMaxParts3 + 1]) {
+  for (int& c : clusters) c = 0;
+  clusters[1] = sm_count;
+  auto* kernel = gemm_split_kernel<128, false, true, false>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax3);
+  for (int n = 2; n <= kMaxParts3 && e == cudaSuccess; ++n) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(sm_count / n * n));
+    cfg.blockDim = dim3(kThreads3);
+    cfg.dynamicSmemBytes = kSmemMax3;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim = {(unsigned)n, 1, 1};
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    e = cudaOccupancyMaxActiveClusters(&clusters[n], kernel, &cfg);
+    if (e != cudaSuccess) clusters[n] = 0;
   }
-  return gemm_split_rule(ctx.sm_count, clusters.data(), groups, M, N, K / kBK3, (flags & PTXB200_GEMM_NO_SPLIT) == 0, plan);
+  if (e != cudaSuccess) cudaGetLastError();   // clusters of two then
+}
+
+bool gemm_split_choose(const DeviceCtx& ctx, int groups, int M, int N, int K, unsigned flags, GemmSplitPlan* plan) {
+  return gemm_split_rule(ctx.sm_count, ctx.clusters, groups, M, N, K / kBK3, (flags & PTXB200_GEMM_NO_SPLIT) == 0, plan);
 }
 
 int launch_gemm_split(const DeviceCtx& ctx, const GemmSplitPlan& p, void* C, const void* A, const void* Bt, int groups,

@@ -33,6 +33,9 @@ struct DeviceCtx {
   int sm_count = 0;
   int cc_major = 0;
   int cc_minor = 0;
+  // clusters of n CTAs, each filling an SM, that the device runs at once: they do not straddle its
+  // groups of SMs, so that these are fewer than sm_count / n (33 of 37 for n = 4)
+  int clusters[kMaxParts3 + 1] = {};
   uint32_t* workspace = nullptr;  // kWsWords uint32 on the device, zero-initialised once
 };
 
@@ -132,8 +135,9 @@ int describe_fa_plan(int BH, int S, long long kv_bytes, int causal, unsigned fla
 int gemm_pair_tile(const DeviceCtx& ctx, int groups, int M, int N, int K);
 int launch_gemm_pair(const DeviceCtx& ctx, int bn, void* C, const void* A, const void* Bt, int groups, int M, int N,
                      int K, int ldc, unsigned flags, cudaStream_t stream);
-// Small-tile GEMM with K split inside clusters (gemm_split_sm100.cu): false when another
-// kernel is the better choice.
+// Small-tile GEMM with K split inside clusters (gemm_split_sm100.cu): DeviceCtx::clusters of the
+// current device; false when another kernel is the better choice; its launcher.
+void query_clusters(int sm_count, int (&clusters)[kMaxParts3 + 1]);
 bool gemm_split_choose(const DeviceCtx& ctx, int groups, int M, int N, int K, unsigned flags, GemmSplitPlan* plan);
 int launch_gemm_split(const DeviceCtx& ctx, const GemmSplitPlan& plan, void* C, const void* A, const void* Bt, int groups,
                       int M, int N, int K, int ldc, unsigned flags, cudaStream_t stream);
