@@ -676,6 +676,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
     if constexpr (!kTail) {
       WorkIter<kCausal, kTail, kByLen> items;
       WorkItem w;
+      grid_wait();
       if (items.next(p, seg_table, w)) {
         mbar_arrive_expect_tx(bar(C::kBarKvFull), T::kTileBytes);
         T::load3(kv_smem, &tmap_k, 0, fa_kv_slice(p, w.bh), bar(C::kBarKvFull));
@@ -694,8 +695,10 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
   }
   FA_CTA_TIME(0);
   if (kTail && warp == 14) tail_table(p.sched, smem + C::kOffSegs);
+  grid_wait();
   tc_fence_before();
   __syncthreads();
+  grid_trigger();
   FA_CTA_TIME(1);
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
@@ -1448,24 +1451,26 @@ int launch_variant(const DeviceCtx& ctx, const CUtensorMap& tq, const CUtensorMa
   });
   if (rc != PTXB200_OK) return rc;
   const bool ragged = !kCausal && p.seqlen % kAttnRows != 0;
+  auto launch = [&](auto* kernel, int grid) {
+    return launch_after(stream, kernel, (unsigned)grid, kThreads, C::kSmemBytes, 1u, tq, tk, tv, p);
+  };
   if (p.sched.tail_units > 0) {
     // the last round is cut: every SM gets a CTA
     const int grid = p.sched.grid;
     if (ragged)
-      fa_fwd_kernel<D, false, false, true, true><<<grid, kThreads, C::kSmemBytes, stream>>>(tq, tk, tv, p);
+      PTXB200_CUDA_TRY(launch(fa_fwd_kernel<D, false, false, true, true>, grid));
     else
-      fa_fwd_kernel<D, kCausal, false, false, true><<<grid, kThreads, C::kSmemBytes, stream>>>(tq, tk, tv, p);
+      PTXB200_CUDA_TRY(launch(fa_fwd_kernel<D, kCausal, false, false, true>, grid));
   } else {
     const int units = (kCausal && p.pair_mode) ? p.bh * ((p.num_mblocks + 1) / 2) : p.total_work;   // what ItemIter deals out
     const int grid = units < ctx.sm_count ? units : ctx.sm_count;
     if (ragged)
-      fa_fwd_kernel<D, false, false, true><<<grid, kThreads, C::kSmemBytes, stream>>>(tq, tk, tv, p);
+      PTXB200_CUDA_TRY(launch(fa_fwd_kernel<D, false, false, true>, grid));
     else if (kCausal && p.sched.by_length)
-      fa_fwd_kernel<D, kCausal, false, false, false, kCausal><<<grid, kThreads, C::kSmemBytes, stream>>>(tq, tk, tv, p);
+      PTXB200_CUDA_TRY(launch(fa_fwd_kernel<D, kCausal, false, false, false, kCausal>, grid));
     else
-      fa_fwd_kernel<D, kCausal><<<grid, kThreads, C::kSmemBytes, stream>>>(tq, tk, tv, p);
+      PTXB200_CUDA_TRY(launch(fa_fwd_kernel<D, kCausal>, grid));
   }
-  PTXB200_CUDA_TRY(cudaGetLastError());
   return PTXB200_OK;
 }
 
@@ -1636,8 +1641,7 @@ template <int D, bool kCausal>
 int noalloc_launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                    const FaParams& p, int grid, cudaStream_t stream) {
   using C = FaCfg<D>;
-  fa_fwd_kernel<D, kCausal, true><<<grid, kThreads, C::kSmemBytes, stream>>>(tq, tk, tv, p);
-  PTXB200_CUDA_TRY(cudaGetLastError());
+  PTXB200_CUDA_TRY(launch_after(stream, fa_fwd_kernel<D, kCausal, true>, (unsigned)grid, kThreads, C::kSmemBytes, 1u, tq, tk, tv, p));
   return PTXB200_OK;
 }
 

@@ -113,8 +113,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     tmem_alloc_pair(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
     tmem_relinquish_pair();
   }
+  grid_wait();
   tc_fence_before();
   __syncthreads();
+  grid_trigger();
   cluster_sync_all();     // both CTAs' barriers exist before anything remote is signalled
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
@@ -282,9 +284,9 @@ int launch_one2(const DeviceCtx& ctx, void* C, const void* A, const void* Bt, in
   const long long tiles = (long long)groups * ((M + kBM2 - 1) / kBM2) * ((N + kBN - 1) / kBN);
   const int max_pairs = ctx.sm_count / 2;
   const int pairs = tiles < max_pairs ? (int)tiles : max_pairs;
-  gemm_pair_kernel<kBN, kF32Out><<<2 * pairs, kThreads2, Cfg2<kBN>::kSmemBytes, stream>>>(
-      ta, tb, C, M, N, K, ldc, groups, status_word(ctx, stream));
-  PTXB200_CUDA_TRY(cudaGetLastError());
+  // (the cluster's size is the kernel's own)
+  PTXB200_CUDA_TRY(launch_after(stream, gemm_pair_kernel<kBN, kF32Out>, 2u * pairs, kThreads2, Cfg2<kBN>::kSmemBytes, 1u, ta, tb, C,
+                                M, N, K, ldc, groups, status_word(ctx, stream)));
   return PTXB200_OK;
 }
 

@@ -113,8 +113,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), kTmemCols);
     tmem_relinquish();
   }
+  grid_wait();
   tc_fence_before();
   __syncthreads();
+  grid_trigger();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
@@ -245,11 +247,8 @@ int launch_gemm(const DeviceCtx& ctx, void* C, const void* A, const void* Bt, in
     return PTXB200_OK;
   });
   if (rc != PTXB200_OK) return rc;
-  if (flags & PTXB200_GEMM_F32_OUT)
-    gemm_kernel<true><<<grid, kThreads, kSmemBytes, stream>>>(ta, tb, C, M, N, K, ldc, groups, status);
-  else
-    gemm_kernel<false><<<grid, kThreads, kSmemBytes, stream>>>(ta, tb, C, M, N, K, ldc, groups, status);
-  PTXB200_CUDA_TRY(cudaGetLastError());
+  PTXB200_CUDA_TRY(launch_after(stream, (flags & PTXB200_GEMM_F32_OUT) ? gemm_kernel<true> : gemm_kernel<false>, (unsigned)grid,
+                                kThreads, kSmemBytes, 1u, ta, tb, C, M, N, K, ldc, groups, status));
   return PTXB200_OK;
 }
 

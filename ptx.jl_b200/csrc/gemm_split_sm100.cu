@@ -173,6 +173,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     mbar_init(bar_parts, 1);
     mbar_fence_init();
     if (kSplit) mbar_arrive_expect_tx(bar_parts, (split - 1) * kBM3 * 4 * my_cols);
+    grid_wait();
     if (!misaligned)
       for (int i = 0; i < stages && i < steps; ++i) load(i, i);
   }
@@ -181,8 +182,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     tmem_relinquish();
   }
   __syncwarp();
+  grid_wait();
   tc_fence_before();
   __syncthreads();
+  grid_trigger();
   if (kSplit) cluster_arrive();          // "this CTA has started": waited for ahead of the first store to a peer
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
@@ -394,19 +397,10 @@ int launch_one3(const DeviceCtx& ctx, const GemmSplitPlan& p, const GemmSplitLay
     return PTXB200_OK;
   });
   if (rc != PTXB200_OK) return rc;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(groups * (M / kBM3) * ((N + kBN - 1) / kBN) * p.split));
-  cfg.blockDim = dim3(kThreads3);
-  cfg.dynamicSmemBytes = (size_t)l.smem_bytes;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim = {(unsigned)p.split, 1, 1};
-  cfg.attrs = attr;
-  cfg.numAttrs = kSplit ? 1 : 0;
-  PTXB200_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_split_kernel<kBN, kF32Out, kSplit, kFold>, ta, tb, C, M, N, K, ldc, p.split,
-                                      l.stages, l.chain_stages, (uint32_t)l.tmem_cols, part_cols3(kBN, p.split), slot_bytes3(kBN, p.split),
-                                      status_word(ctx, stream)));
+  const unsigned grid = (unsigned)(groups * (M / kBM3) * ((N + kBN - 1) / kBN) * p.split);
+  PTXB200_CUDA_TRY(launch_after(stream, gemm_split_kernel<kBN, kF32Out, kSplit, kFold>, grid, kThreads3, (size_t)l.smem_bytes,
+                                kSplit ? (unsigned)p.split : 1u, ta, tb, C, M, N, K, ldc, p.split, l.stages, l.chain_stages,
+                                (uint32_t)l.tmem_cols, part_cols3(kBN, p.split), slot_bytes3(kBN, p.split), status_word(ctx, stream)));
   return PTXB200_OK;
 }
 

@@ -538,6 +538,15 @@ __device__ __forceinline__ void st_global_v4(void* p, uint32_t a, uint32_t b, ui
                : "memory");
 }
 
+// Programmatic dependent launch (launch_after, host_common.h). grid_wait: until the stream's work
+// ahead of this launch is complete and its memory visible; ahead of it a kernel touches no global
+// memory, so that only its set-up runs beside the kernel in front. grid_trigger: from the time
+// on when every CTA has called it (or left) the next such launch may take up free SMs; called
+// behind the allocation of tensor memory, so that none of this launch's CTAs waits for that of one
+// which waits for this launch.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 template <int N>
 __device__ __forceinline__ void setmaxnreg_inc() {
   asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));

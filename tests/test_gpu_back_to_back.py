@@ -1,0 +1,104 @@
+"""Launches whose set-up runs beside the end of the stream's kernel in front of them (launch_after,
+host_common.h): chains in which every call reads what the one before wrote, or writes what it
+read, give the same bits as with a wait for the GPU behind every call -- eagerly, in a replayed
+graph, beside the framework's own kernels and copies, and on two streams at once."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def chain(ops, case, g, sync):
+    """A dozen dependent calls on a few buffers, each used again and again; returns the buffers."""
+    dev = g.device
+    done = torch.cuda.synchronize if sync else (lambda: None)
+    M, N, K = case
+    a = torch.rand(M, K, device=dev, generator=g).sub_(0.5).mul_(2 * K ** -0.5).to(torch.bfloat16)
+    b = [torch.rand(N, K, device=dev, generator=g).sub_(0.5).to(torch.bfloat16) for _ in range(2)]
+    w = torch.rand(K, N, device=dev, generator=g).sub_(0.5).to(torch.bfloat16)
+    c, x = torch.empty(M, N, device=dev, dtype=torch.bfloat16), torch.empty(M, K, device=dev, dtype=torch.bfloat16)
+    q = torch.empty(1, M // 64, 64, K, device=dev, dtype=torch.bfloat16)
+    o = torch.empty_like(q)
+    y = torch.empty(M, K, device=dev)
+    ones = torch.ones(K, device=dev)
+
+    def calls():
+        yield lambda: x.copy_(a)
+        for i in range(4):
+            yield lambda: ops.gemm(x, b[i & 1], out=c)             # reads what the last turn wrote
+            yield lambda: ops.gemm(c, w, out=x)                    # over the operand just read
+            if K in (64, 128):
+                yield lambda: q.view(M, K).copy_(x)                # a copy of the framework's between
+                yield lambda: ops.fa_fwd(q, q, q, causal=bool(i & 1), out=o)
+                yield lambda: x.copy_(o.view(M, K))
+            yield lambda: ops.rms_norm(x.float(), ones, out=y)
+            yield lambda: ops.softmax(y, out=y)
+            yield lambda: x.copy_(y)
+
+    for call in calls():
+        call()
+        done()
+    return [c, x, y] + ([o] if K in (64, 128) else [])
+
+
+CASES = [(128, 128, 128), (1024, 1152, 128), (4096, 4096, 128), (2048, 2048, 512), (256, 4096, 4096)]
+
+
+@pytest.mark.parametrize("case", CASES)
+def test_chain_of_dependent_calls(pkg, gpu, case):
+    want = chain(pkg.ops, case, torch.Generator(device=gpu).manual_seed(1), True)
+    assert all(bool(torch.isfinite(t.float()).all()) for t in want)
+    for _ in range(5):
+        for got, ref in zip(chain(pkg.ops, case, torch.Generator(device=gpu).manual_seed(1), False), want):
+            assert torch.equal(got, ref)
+    assert pkg.ops.sync_status() == 0
+
+
+def test_chain_in_a_graph_and_on_two_streams(pkg, gpu):
+    case = (1024, 1152, 128)
+    M, N, K = case
+    g = torch.Generator(device=gpu).manual_seed(2)
+    a = torch.rand(M, K, device=gpu, generator=g).sub_(0.5).to(torch.bfloat16)
+    b = torch.rand(N, K, device=gpu, generator=g).sub_(0.5).to(torch.bfloat16)
+    w = torch.rand(K, N, device=gpu, generator=g).sub_(0.5).mul_(0.05).to(torch.bfloat16)
+    bufs = [(a.clone(), torch.empty(M, N, device=gpu, dtype=torch.bfloat16)) for _ in range(2)]
+
+    def turn(x, c):
+        pkg.ops.gemm(x, b, out=c)
+        pkg.ops.gemm(c, w, out=x)
+        q = x.view(1, M // 64, 64, K)
+        pkg.ops.fa_fwd(q, q, q, out=c.view(-1)[:M * K].view(1, M // 64, 64, K))
+        x.copy_(c.view(-1)[:M * K].view(M, K))
+
+    x, c = a.clone(), torch.empty(M, N, device=gpu, dtype=torch.bfloat16)
+    for _ in range(8):
+        turn(x, c)
+        torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    graphs = []
+    for s, (xs, cs) in zip(streams, bufs):        # captured with a fork and a join in front
+        with torch.cuda.stream(s):
+            turn(xs, cs)                          # first calls on the stream, outside the capture
+            xs.copy_(a)
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=s):
+                side = torch.cuda.Stream()
+                side.wait_stream(s)
+                with torch.cuda.stream(side):
+                    xs.mul_(1.0)
+                s.wait_stream(side)
+                turn(xs, cs)
+                turn(xs, cs)
+            graphs.append(graph)
+    torch.cuda.synchronize()
+    for xs, _ in bufs:
+        xs.copy_(a)
+    torch.cuda.synchronize()
+    for _ in range(4):
+        for s, graph in zip(streams, graphs):
+            with torch.cuda.stream(s):
+                graph.replay()
+    torch.cuda.synchronize()
+    for xs, _ in bufs:
+        assert torch.equal(xs, x)
+    assert pkg.ops.sync_status() == 0
