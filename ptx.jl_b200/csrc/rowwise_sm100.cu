@@ -27,6 +27,8 @@
 //     rows of 2048 columns, layer norm: 4.2 us, now 2.1); long ones over 1024 threads;
 //   * X and Y are accessed with the streaming cache hints (read once, written once), the
 //     weight vectors through the read-only path;
+//   * a launch's blocks are set up while the kernel in front ends (launch_after): 300 rows of 2048
+//     columns, back to back, 4.1 us a launch without, 2.4-2.75 with; 4096 x 30000, softmax, 158 and 156;
 //   * softmax merges (max, sum of exponentials) pairs by the online-softmax rule and
 //     rescales once; layer norm takes the mean, then the centred sums of the values on chip and
 //     of their squares, which keeps its accuracy for rows with a large mean, where the
@@ -85,7 +87,24 @@ __device__ __forceinline__ T warp_reduce(T v) {
   return v;
 }
 
-__device__ __forceinline__ float4 load_once(const float4* p) { return __ldcs(p); }
+// Global loads stay behind grid_wait: they go through pointers that the compiler only knows behind
+// it (behind). The weights use the read-only path all the same, whose loads pass this kernel's
+// stores (plain loads, which do not: layer norm, 423 x 23104 19.8 us against 16.7; 1500 x 20000 49 and
+// 44). What it caches on an SM dates from behind the start of this kernel there, which is behind the
+// last CTA of the kernel in front unless that one lets its successor in early (grid_trigger): the
+// kernels of this library that do (attention, GEMM) read global memory through TMA and L2 alone.
+// For the same reason, and because the waiting blocks of the next launch took the place of this
+// one's (4000 x 1024, layer norm: 7.2 us against 5.6), the kernels here do not.
+__device__ __forceinline__ float4 load_once(const float4* p) {   // streaming: read once
+  float4 v;
+  asm("ld.global.cs.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+template <class T>
+__device__ __forceinline__ const T* behind(const T* p) {
+  asm volatile("" : "+l"(p)::"memory");
+  return p;
+}
 __device__ __forceinline__ void cp_async16(uint32_t dst_smem, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_smem), "l"(src) : "memory");
 }
@@ -104,10 +123,11 @@ rowwise_kernel(const RowParams p) {
   const int t = kWarpRows ? threadIdx.x & 31 : threadIdx.x;
   const int row = kWarpRows ? blockIdx.x * 4 + (threadIdx.x >> 5) : blockIdx.x;
   if (kWarpRows && row >= p.rows) return;            // the last block's rows may be fewer; no block barrier follows
-  const float4* x4 = reinterpret_cast<const float4*>(p.x) + (size_t)row * p.n4;
+  grid_wait();
+  const float4* x4 = behind(reinterpret_cast<const float4*>(p.x)) + (size_t)row * p.n4;
   float4* y4 = reinterpret_cast<float4*>(p.y) + (size_t)row * p.n4;
-  const float4* w4 = reinterpret_cast<const float4*>(p.w);
-  const float4* b4 = reinterpret_cast<const float4*>(p.bias);
+  const float4* w4 = behind(reinterpret_cast<const float4*>(p.w));
+  const float4* b4 = behind(reinterpret_cast<const float4*>(p.bias));
   const float fill = kOp == kOpSoftmax ? -INFINITY : 0.0f;
 
   int parity = 0;
@@ -250,10 +270,10 @@ constexpr int kSwigluThreads = 256;
 // kUnroll: independent 128-bit load pairs in flight per thread
 template <int kUnroll>
 __global__ void __launch_bounds__(kSwigluThreads)
-swiglu_kernel(float* __restrict__ out, const float* __restrict__ gate, const float* __restrict__ up,
-              size_t n4) {
-  const float4* g4 = reinterpret_cast<const float4*>(gate);
-  const float4* u4 = reinterpret_cast<const float4*>(up);
+swiglu_kernel(float* out, const float* gate, const float* up, size_t n4) {
+  grid_wait();
+  const float4* g4 = behind(reinterpret_cast<const float4*>(gate));
+  const float4* u4 = behind(reinterpret_cast<const float4*>(up));
   float4* o4 = reinterpret_cast<float4*>(out);
   const size_t base = (size_t)blockIdx.x * (kSwigluThreads * kUnroll) + threadIdx.x;
   float4 g[kUnroll], u[kUnroll];
@@ -261,8 +281,8 @@ swiglu_kernel(float* __restrict__ out, const float* __restrict__ gate, const flo
   for (int i = 0; i < kUnroll; ++i) {
     const size_t c = base + i * kSwigluThreads;
     if (c < n4) {
-      g[i] = __ldcs(g4 + c);
-      u[i] = __ldcs(u4 + c);
+      g[i] = load_once(g4 + c);
+      u[i] = load_once(u4 + c);
     }
   }
 #pragma unroll
@@ -276,8 +296,7 @@ swiglu_kernel(float* __restrict__ out, const float* __restrict__ gate, const flo
 
 template <int kOp, int kVec>
 int launch_warp_rows(const RowParams& p, cudaStream_t stream) {
-  rowwise_kernel<kOp, true, kVec, 0, 128, 1><<<(p.rows - 1) / 4 + 1, 128, 0, stream>>>(p);
-  PTXB200_CUDA_TRY(cudaGetLastError());
+  PTXB200_CUDA_TRY(launch_after(stream, rowwise_kernel<kOp, true, kVec, 0, 128, 1>, (unsigned)((p.rows - 1) / 4 + 1), 128u, 0, 1u, p));
   return PTXB200_OK;
 }
 
@@ -286,9 +305,8 @@ template <int kOp, int kVec, int kMaxT, int kMinBlocks, int kPark = 0>
 int launch_block_rows(const RowParams& p, cudaStream_t stream) {
   constexpr int per = kVec + kPark;
   const int threads = kMaxT == 1024 ? 1024 : ((p.n4 + per - 1) / per + 31) / 32 * 32;
-  rowwise_kernel<kOp, false, kVec, kPark, kMaxT, kMinBlocks>
-      <<<p.rows, threads, (size_t)kPark * threads * 16, stream>>>(p);
-  PTXB200_CUDA_TRY(cudaGetLastError());
+  PTXB200_CUDA_TRY(launch_after(stream, rowwise_kernel<kOp, false, kVec, kPark, kMaxT, kMinBlocks>, (unsigned)p.rows, (unsigned)threads,
+                                (size_t)kPark * threads * 16, 1u, p));
   return PTXB200_OK;
 }
 
@@ -369,9 +387,8 @@ int launch_swiglu(const DeviceCtx& ctx, float* out, const float* gate, const flo
   const size_t per_block = (size_t)kSwigluThreads * (small ? 1 : 4);
   const size_t blocks = (n4 + per_block - 1) / per_block;
   if (blocks > 0x7fffffffu) return PTXB200_E_SHAPE;
-  if (small) swiglu_kernel<1><<<(unsigned)blocks, kSwigluThreads, 0, stream>>>(out, gate, up, n4);
-  else swiglu_kernel<4><<<(unsigned)blocks, kSwigluThreads, 0, stream>>>(out, gate, up, n4);
-  PTXB200_CUDA_TRY(cudaGetLastError());
+  PTXB200_CUDA_TRY(launch_after(stream, small ? swiglu_kernel<1> : swiglu_kernel<4>, (unsigned)blocks, kSwigluThreads, 0, 1u, out, gate,
+                                up, n4));
   return PTXB200_OK;
 }
 

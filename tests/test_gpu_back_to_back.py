@@ -102,3 +102,29 @@ def test_chain_in_a_graph_and_on_two_streams(pkg, gpu):
     for xs, _ in bufs:
         assert torch.equal(xs, x)
     assert pkg.ops.sync_status() == 0
+
+
+@pytest.mark.parametrize("rows,N", [(16, 2048), (300, 512), (4000, 1024), (2000, 4096), (148, 20000), (600, 30000)])
+def test_weights_written_right_ahead_of_the_call(pkg, gpu, rows, N):
+    """Every norm reads a weight vector and rows that the call ahead of it wrote; swiglu works in place."""
+    g = torch.Generator(device=gpu).manual_seed(rows)
+    x0 = torch.randn(rows, N, device=gpu, generator=g)
+    w0 = torch.randn(N, device=gpu, generator=g).mul_(0.1).add_(1.0)
+
+    def run(sync):
+        done = torch.cuda.synchronize if sync else (lambda: None)
+        x, y, w, b = x0.clone(), torch.empty_like(x0), w0.clone(), w0.clone()
+        for i in range(12):
+            for call in (lambda: w.add_(0.125), lambda: b.copy_(w).mul_(-0.5),
+                         lambda: pkg.ops.layer_norm(x, w, b, out=y), lambda: w.copy_(y[i]),
+                         lambda: pkg.ops.rms_norm(y, w, out=x), lambda: pkg.ops.swiglu(x, y, out=x),
+                         lambda: pkg.ops.layer_norm(x, w0, b, out=x), lambda: w.copy_(w0),
+                         lambda: pkg.ops.softmax(y, out=y)):
+                call()
+                done()
+        return x, y
+
+    want = run(True)
+    assert all(bool(torch.isfinite(t).all()) for t in want)
+    for _ in range(3):
+        assert all(torch.equal(a, b) for a, b in zip(run(False), want))
