@@ -269,8 +269,9 @@ int fa_fwd_bf16_noalloc_status(uint32_t* cta_flags_out, int max_flags, void* str
  * segment (block, batch*head, first tile, end tile, tiles of the item, pieces parked by
  * following CTAs). Returns the ints written, PTXB200_E_CAPACITY if cap is too small.
  * Causal launches whose K and V (all heads) are at most 160 MiB may instead deal their
- * items by length over all heads, without pairs or a cut; that choice needs the head dim
- * and the number of K/V heads: ptxb200_fa_plan_ex.
+ * items by length over all heads, without pairs or a cut, and whether a last round is cut
+ * depends on the head dim (128 is taken here): ptxb200_fa_plan_ex, which is given both the
+ * head dim and the number of K/V heads, shows what a launch does.
  * The reference's distribution is the round robin of flash_attention_defs.jl:269-272.
  */
 int ptxb200_fa_plan(int B, int H, int S, int causal, unsigned flags, int sm_count, int* out, int cap);

@@ -370,13 +370,13 @@ int swiglu_f32(void* out, const void* gate, const void* up, long long n, void* s
 }
 
 namespace {
-int fa_plan_entry(int B, int H, int S, long long kv_bytes, int causal, unsigned flags, int sm_count, int* out, int cap) {
+int fa_plan_entry(int B, int H, int S, long long kv_bytes, int D, int causal, unsigned flags, int sm_count, int* out, int cap) {
   if (B <= 0 || H <= 0 || S <= 0 || sm_count <= 0 || cap < 0 || (out == nullptr && cap > 0)) return PTXB200_E_INVALID;
   if (causal != 0 && causal != 1) return PTXB200_E_INVALID;
   if (flags & ~(PTXB200_FA_NO_LAZY_RESCALE | PTXB200_FA_SINGLE_BLOCKS | PTXB200_FA_NO_TAIL_SPLIT |
                 PTXB200_FA_ALWAYS_TAIL_SPLIT)) return PTXB200_E_INVALID;
   if ((long long)B * H * S >= (1ll << 31)) return PTXB200_E_SHAPE;
-  const int n = describe_fa_plan(B * H, S, kv_bytes, causal, flags, sm_count, out, cap);
+  const int n = describe_fa_plan(B * H, S, kv_bytes, D, causal, flags, sm_count, out, cap);
   return n < 0 ? PTXB200_E_CAPACITY : n;
 }
 }  // namespace
@@ -407,13 +407,13 @@ int fa_fwd_bf16(void* O, const void* Q, const void* K, const void* V, int B, int
 }
 
 int ptxb200_fa_plan(int B, int H, int S, int causal, unsigned flags, int sm_count, int* out, int cap) {
-  return fa_plan_entry(B, H, S, -1, causal, flags, sm_count, out, cap);
+  return fa_plan_entry(B, H, S, -1, 128, causal, flags, sm_count, out, cap);
 }
 
 int ptxb200_fa_plan_ex(int B, int H, int H_kv, int S, int D, int causal, unsigned flags, int sm_count, int* out, int cap) {
   if (B <= 0 || H <= 0 || H_kv <= 0 || S <= 0) return PTXB200_E_INVALID;
   if ((D != 64 && D != 128) || H % H_kv != 0) return PTXB200_E_SHAPE;
-  return fa_plan_entry(B, H, S, 4ll * B * H_kv * S * D, causal, flags, sm_count, out, cap);
+  return fa_plan_entry(B, H, S, 4ll * B * H_kv * S * D, D, causal, flags, sm_count, out, cap);
 }
 
 int ptxb200_sync_status(void* stream) {

@@ -1279,7 +1279,13 @@ long long worst_round_robin(const FaSched& sc, int units, int grid) {
   return worst;
 }
 
-constexpr int kSplitOverheadSteps = 3;   // what a second segment, parking and merging cost a CTA, in steps (measured: 2.5-3)
+constexpr int kSplitOverheadSteps = 3;   // what a second segment costs the busiest CTA at least, in steps
+// What a cut costs the launch, in steps of its busiest CTA, and a step more for each further piece of an
+// item: parking, the flag, and a merge that starts when the last piece is there. Measured over 1-100
+// heads of 512-8192 keys, cut against whole (a step 1.58 us at head dim 128, 1.38 at 64): 9-12 and 7-9
+// with one or two further pieces, 12-20 and 11-13 with five. The rule so far counted 3 in all: 16 heads of 1024 keys
+// 30.9 us cut, 20.6 whole; 12 of 1920 39.2 and 31.4; 40 of 1024 46.3 and 37.0; causal, 16 of 1024 28.8 and 20.8.
+constexpr int kCutSteps128 = 8, kCutSteps64 = 6;
 constexpr int kSplitMaxRounds = 64;      // beyond this many full rounds the tail is noise: not split
 constexpr int kItemOverheadSteps = 1;    // what the boundary between two items costs a CTA, in steps (measured: 1-1.5)
 // K and V of all heads together up to about L2's size (126 MB) are read from HBM once or little
@@ -1302,30 +1308,31 @@ long long worst_by_length(int bh, int nmb, int nt_all, int grid) {
   return worst;
 }
 
-FaSched plan_uncached(int bh, int nmb, int nt_all, int causal, unsigned flags, int sm_count, bool may_split, bool kv_in_l2);
+FaSched plan_uncached(int bh, int nmb, int nt_all, int causal, unsigned flags, int sm_count, bool may_split, bool kv_in_l2,
+                      int head_dim);
 
 // The distribution of a launch; the last few shapes' are kept, since finding one walks every CTA.
 FaSched plan_schedule(int bh, int nmb, int nt_all, int causal, unsigned flags, int sm_count, bool may_split,
-                      long long kv_bytes) {
+                      long long kv_bytes, int head_dim) {
   const bool kv_in_l2 = kv_bytes <= kByLengthMaxKvBytes;
   struct Key {
-    int bh, nmb, nt_all, causal, sm;
+    int bh, nmb, nt_all, causal, sm, head_dim;
     unsigned flags;
     bool may_split, kv_in_l2;
     bool operator==(const Key& o) const {
-      return bh == o.bh && nmb == o.nmb && nt_all == o.nt_all && causal == o.causal && sm == o.sm && flags == o.flags &&
+      return bh == o.bh && nmb == o.nmb && nt_all == o.nt_all && causal == o.causal && sm == o.sm && head_dim == o.head_dim && flags == o.flags &&
              may_split == o.may_split && kv_in_l2 == o.kv_in_l2;
     }
   };
   static std::mutex mu;
   static std::vector<std::pair<Key, FaSched>> cache;
-  const Key key{bh, nmb, nt_all, causal, sm_count, flags, may_split, kv_in_l2};
+  const Key key{bh, nmb, nt_all, causal, sm_count, head_dim, flags, may_split, kv_in_l2};
   {
     std::lock_guard<std::mutex> lock(mu);
     for (const auto& kv : cache)
       if (kv.first == key) return kv.second;
   }
-  const FaSched sc = plan_uncached(bh, nmb, nt_all, causal, flags, sm_count, may_split, kv_in_l2);
+  const FaSched sc = plan_uncached(bh, nmb, nt_all, causal, flags, sm_count, may_split, kv_in_l2, head_dim);
   std::lock_guard<std::mutex> lock(mu);
   if (cache.size() >= 16) cache.erase(cache.begin());
   cache.emplace_back(key, sc);
@@ -1335,7 +1342,8 @@ FaSched plan_schedule(int bh, int nmb, int nt_all, int causal, unsigned flags, i
 // Round robin over whole units (the reference's distribution); causal items by length; or
 // round robin with the last, partly filled round cut along the key axis when that shortens
 // the busiest CTA's work by more than the overhead of the cut.
-FaSched plan_uncached(int bh, int nmb, int nt_all, int causal, unsigned flags, int sm_count, bool may_split, bool kv_in_l2) {
+FaSched plan_uncached(int bh, int nmb, int nt_all, int causal, unsigned flags, int sm_count, bool may_split, bool kv_in_l2,
+                      int head_dim) {
   FaSched legacy;
   legacy.num_mblocks = nmb;
   legacy.bh = bh;
@@ -1395,7 +1403,7 @@ FaSched plan_uncached(int bh, int nmb, int nt_all, int causal, unsigned flags, i
   // the kernel's per-CTA table and the combiner's reads are bounded: walk every tail CTA,
   // and take the busiest one's steps from the walk (cuts snap to item edges, so spans differ)
   HostLocator loc{starts.data(), (int)starts.size() - 1};
-  int tail_worst = 0;
+  int tail_worst = 0, pieces = 0;
   for (int c = 0; c < sc.tail_ctas; ++c) {
     FaSeg segs[kTailMaxSegs];
     const int n = fa_tail_segments(sc, c, loc, segs);
@@ -1404,18 +1412,21 @@ FaSched plan_uncached(int bh, int nmb, int nt_all, int causal, unsigned flags, i
     for (int i = 0; i < n; ++i) {
       if (segs[i].n_other + 1 > kTailMaxParts) return legacy;
       steps += segs[i].j1 - segs[i].j0;
+      pieces = segs[i].n_other > pieces ? segs[i].n_other : pieces;
     }
     tail_worst = steps > tail_worst ? steps : tail_worst;
   }
   const long long split_worst = worst_round_robin(sc, sc.full_units, sc.grid) + tail_worst + kSplitOverheadSteps;
   if (flags & PTXB200_FA_ALWAYS_TAIL_SPLIT) return sc;
-  // cut only for a gain of a twelfth or more
+  // cut only for a gain of a twelfth or more beside the least that it costs, and of 3 % beside all
+  const long long cut_cost = split_worst - kSplitOverheadSteps + (head_dim == 64 ? kCutSteps64 : kCutSteps128) + pieces;
   if (legacy.by_length) {
     const long long boundaries = kItemOverheadSteps * ((sc.pair_mode ? 2 : 1) * (sc.full_units / sm_count) + 1);
+    if ((cut_cost + boundaries) * 100 > legacy_cost * 97) return legacy;
     return (split_worst + boundaries) * 100 > legacy_cost * 92 ? legacy : sc;
   }
   const long long legacy_worst = worst_round_robin(legacy, legacy.full_units, legacy.grid);
-  if (split_worst * 100 > legacy_worst * 92) return legacy;
+  if (split_worst * 100 > legacy_worst * 92 || cut_cost * 100 > legacy_worst * 97) return legacy;
   return sc;
 }
 
@@ -1513,7 +1524,7 @@ int launch_fa_fwd(const DeviceCtx& ctx, void* O, void* lse, const void* Q, const
   const long long kv_bytes = 4ll * B * H_kv * S * D;
   auto plan = [&](bool may_split) {
     return plan_schedule(B * H, (S + 255) / 256, (S + kAttnRows - 1) / kAttnRows, causal, flags, ctx.sm_count, may_split,
-                         kv_bytes);
+                         kv_bytes, D);
   };
   FaSched sched = plan(true);
   if (sched.tail_units > 0) {
@@ -1554,11 +1565,11 @@ int launch_fa_fwd(const DeviceCtx& ctx, void* O, void* lse, const void* Q, const
 // grid, full_units, tail_units, tail_steps, tail_ctas), by_length if kv_bytes is given, then per tail CTA its segment count
 // followed by 6 ints per segment (mb, bh, j0, j1, len, n_other). Returns the ints written,
 // or -1 if `cap` is too small.
-int describe_fa_plan(int BH, int S, long long kv_bytes, int causal, unsigned flags, int sm_count, int* out, int cap) {
+int describe_fa_plan(int BH, int S, long long kv_bytes, int head_dim, int causal, unsigned flags, int sm_count, int* out, int cap) {
   const int nmb = (S + 255) / 256, nt_all = (S + kAttnRows - 1) / kAttnRows;
   // not known how large K and V are: as for too large for the order by length
   const FaSched sc = plan_schedule(BH, nmb, nt_all, causal, flags, sm_count, true,
-                                   kv_bytes < 0 ? kByLengthMaxKvBytes + 1 : kv_bytes);
+                                   kv_bytes < 0 ? kByLengthMaxKvBytes + 1 : kv_bytes, head_dim);
   int n = 0;
   auto put = [&](int v) {
     if (n < cap) out[n] = v;
@@ -1704,7 +1715,7 @@ extern "C" int fa_fwd_bf16_noalloc(void* O, const void* Q, const void* K, const 
   // to the SM count, which this entry point does not have
   fill_params(p, O, nullptr, B, H, H, S, sm_scale, flags, nullptr, nd.scratch,
               plan_schedule(B * H, (S + 255) / 256, (S + kAttnRows - 1) / kAttnRows, causal, flags, nd.sm_count, false,
-                            kByLengthMaxKvBytes + 1));
+                            kByLengthMaxKvBytes + 1, D));
   p.cta_flags = nd.scratch + kNoAllocFlagBase;
   const int units = (causal && p.pair_mode) ? p.bh * ((p.num_mblocks + 1) / 2) : p.total_work;
   const int grid = units < nd.sm_count ? units : nd.sm_count;

@@ -151,7 +151,7 @@ int launch_fa_fwd(const DeviceCtx& ctx, void* O, void* lse, const void* Q, const
                   unsigned flags, void* dbg, uint32_t* status, cudaStream_t stream);
 // The work distribution launch_fa_fwd would pick, as plain ints (fa_fwd_sm100.cu); kv_bytes: K and
 // V of all heads, or negative.
-int describe_fa_plan(int BH, int S, long long kv_bytes, int causal, unsigned flags, int sm_count, int* out, int cap);
+int describe_fa_plan(int BH, int S, long long kv_bytes, int head_dim, int causal, unsigned flags, int sm_count, int* out, int cap);
 // CTA-pair GEMM (gemm2_sm100.cu): the tile width it would run a product with (0: not at
 // all), and its launcher.
 int gemm_pair_tile(const DeviceCtx& ctx, int groups, int M, int N, int K);
