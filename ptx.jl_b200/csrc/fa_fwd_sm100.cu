@@ -65,6 +65,7 @@ namespace ptxb200 {
 namespace {
 
 constexpr int kThreads = 512;
+constexpr unsigned kLetInMaxCtas = 74;   // half of the SMs
 #ifndef PTXB200_FA_REGS_SOFTMAX
 #define PTXB200_FA_REGS_SOFTMAX 168
 #define PTXB200_FA_REGS_CORRECTION 104
@@ -695,11 +696,13 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
   }
   FA_CTA_TIME(0);
   if (kTail && warp == 14) tail_table(p.sched, smem + C::kOffSegs);
-  // (No grid_trigger: CTAs of the next launch that move in while this one's last run measured 1.5 %
-  // slower, 32 heads on 8 of 3001 keys 88.7 us a launch and 87.2; 2 heads of 512 keys 10.6 and 10.9.)
   grid_wait();
   tc_fence_before();
   __syncthreads();
+  // The next launch is let in where it finds SMs without a CTA of this one (2 heads of 512 keys 10.55 us a
+  // launch, 10.85 without). CTAs of it that move in beside the last ones of a full grid measured 1.5 %
+  // slower (32 heads on 8 of 3001 keys 88.7 us and 87.2).
+  if (gridDim.x <= kLetInMaxCtas) grid_trigger();
   FA_CTA_TIME(1);
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;

@@ -92,7 +92,7 @@ __device__ __forceinline__ T warp_reduce(T v) {
 // stores (plain loads, which do not: layer norm, 423 x 23104 19.8 us against 16.7; 1500 x 20000 49 and
 // 44). What it caches on an SM dates from behind the start of this kernel there, which is behind the
 // last CTA of the kernel in front unless that one lets its successor in early (grid_trigger): the
-// kernels of this library that do (the GEMMs) read global memory through TMA alone.
+// kernels of this library that do (the GEMMs, attention on few SMs) read global memory through TMA alone.
 // For the same reason, and because the waiting blocks of the next launch took the place of this
 // one's (4000 x 1024, layer norm: 7.2 us against 5.6), the kernels here do not.
 __device__ __forceinline__ float4 load_once(const float4* p) {   // streaming: read once
