@@ -25,8 +25,7 @@
 //   * few rows (at most two per SM, up to 4096 columns) are spread over four times the
 //     threads, and the weights are fetched ahead of the reduction: latency counts there (16
 //     rows of 2048 columns, layer norm: 4.2 us, now 2.1); long ones over 1024 threads;
-//   * X and Y are accessed with the streaming cache hints (read once, written once), the
-//     weight vectors through the read-only path;
+//   * X and Y are accessed with the streaming cache hints (read once, written once);
 //   * a launch's blocks are set up while the kernel in front ends (launch_after): 300 rows of 2048
 //     columns, back to back, 4.1 us a launch without, 2.4-2.75 with; 4096 x 30000, softmax, 158 and 156;
 //   * softmax merges (max, sum of exponentials) pairs by the online-softmax rule and
@@ -88,16 +87,22 @@ __device__ __forceinline__ T warp_reduce(T v) {
 }
 
 // Global loads stay behind grid_wait: they go through pointers that the compiler only knows behind
-// it (behind). The weights use the read-only path all the same, whose loads pass this kernel's
-// stores (plain loads, which do not: layer norm, 423 x 23104 19.8 us against 16.7; 1500 x 20000 49 and
-// 44). What it caches on an SM dates from behind the start of this kernel there, which is behind the
-// last CTA of the kernel in front unless that one lets its successor in early (grid_trigger): the
-// kernels of this library that do (the GEMMs, attention on few SMs) read global memory through TMA alone.
-// For the same reason, and because the waiting blocks of the next launch took the place of this
-// one's (4000 x 1024, layer norm: 7.2 us against 5.6), the kernels here do not.
+// it (behind). The weights are loaded plainly and not through the read-only path (ld.global.nc), which
+// wants memory that nothing writes while this kernel runs: it starts ahead of the end of the kernel in
+// front, which may be writing them. The compiler moves no plain load past a store, so that the
+// weights of a thread's next groups are fetched ahead of the stores in the source (kAhead; 423 x 23104, layer
+// norm: 19.7 us through the read-only path, 20.1 this way, 22.7 with each group's loads behind the store of the one
+// before; 4096 x 30000 194, 194 and 204; RMS norm 161, 162 and 170).
+// These kernels do not let their successor in early (grid_trigger): 4000 x 1024, layer norm, 7.2 us
+// with it at the start of a block, 5.6 without.
 __device__ __forceinline__ float4 load_once(const float4* p) {   // streaming: read once
   float4 v;
   asm("ld.global.cs.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float4 load_shared_by_rows(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
   return v;
 }
 template <class T>
@@ -155,20 +160,27 @@ rowwise_kernel(const RowParams p) {
     const int c = t + i * tpr;
     v[i] = c < p.n4 ? load_once(x4 + c) : make_float4(fill, fill, fill, fill);
   }
-  // short shares: the vectors are fetched ahead of the reduction, so that their latency
-  // does not follow it (longer shares have no registers for that)
-  constexpr bool kEarly = kOp != kOpSoftmax && kVec <= 2;
-  float4 w[kEarly ? kVec : 1], b[kEarly && kOp == kOpLayerNorm ? kVec : 1];
-  if constexpr (kEarly) {
-#pragma unroll
-    for (int i = 0; i < kVec; ++i) {
-      const int c = t + i * tpr;
-      if (c < p.n4) {
-        w[i] = __ldg(w4 + c);
-        if constexpr (kOp == kOpLayerNorm) b[i] = __ldg(b4 + c);
-      }
+  // The weights of the thread's first kAhead groups are fetched ahead of the last reduction (short shares:
+  // of all, so that their latency does not follow it), the others' as these are written: as many as registers
+  // allow (layer norm holds two vectors: with four ahead 2000 x 8192 takes 30 us, 23 with two).
+  // A warp's rows: six, behind the reduction (layer norm, 65536 x 1024 78.5 us, 82 with all eight).
+  constexpr bool kNorm = kOp != kOpSoftmax;
+  constexpr int kAhead = kVec <= 2 ? kVec : kWarpRows ? (kVec < 6 ? kVec : 6) : kOp == kOpLayerNorm ? (kVec == 4 ? 1 : 2)
+                         : kPark > 0 || kMaxT == 1024 ? 4 : 2;
+  float4 w[kNorm ? kAhead : 1], b[kOp == kOpLayerNorm ? kAhead : 1];
+  auto fetch_into = [&](int i, float4& wi, float4& bi) {
+    const int c = t + i * tpr;
+    if (c < p.n4) {
+      wi = load_shared_by_rows(w4 + c);
+      if constexpr (kOp == kOpLayerNorm) bi = load_shared_by_rows(b4 + c);
     }
-  }
+  };
+  auto fetch = [&](int i) { fetch_into(i, w[i % kAhead], b[kOp == kOpLayerNorm ? i % kAhead : 0]); };
+  auto fetch_first = [&]() {
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i) fetch(i);
+  };
+  if constexpr (kNorm && kVec <= 2) fetch_first();
   if (kPark > 0) cp_async_wait_all();
 
   // f(element group, its index in the row) over everything this thread holds
@@ -203,7 +215,9 @@ rowwise_kernel(const RowParams p) {
   } else if constexpr (kOp == kOpRmsNorm) {
     float s = 0.0f;
     each([&](float4& x, int) { s += (x.x * x.x + x.y * x.y) + (x.z * x.z + x.w * x.w); });
+    if constexpr (kVec > 2 && !kWarpRows) fetch_first();
     mul = rsqrtf(reduce(s) * p.inv_n + p.eps);
+    if constexpr (kVec > 2 && kWarpRows) fetch_first();
   } else {
     // The mean is a sum in fp32 and off by its rounding, up to a few 1e-7 of itself. The mean of
     // the centred values is that error: it is taken off the values and, squared, off their mean
@@ -221,7 +235,9 @@ rowwise_kernel(const RowParams p) {
         d.b += (x.x * x.x + x.y * x.y) + (x.z * x.z + x.w * x.w);
       }
     });
+    if constexpr (kVec > 2 && !kWarpRows) fetch_first();
     d = reduce(d);
+    if constexpr (kVec > 2 && kWarpRows) fetch_first();
     const float off = d.a * p.inv_n;
     float var = d.b * p.inv_n;
     if (var < INFINITY) var = fmaxf(fmaf(-off, off, var), 0.0f);   // two rounded values: may cross zero (NaN: left alone)
@@ -229,37 +245,54 @@ rowwise_kernel(const RowParams p) {
     add = -off * mul;
   }
 
-  auto write = [&](const float4& x, int c, const float4* early_w, const float4* early_b) {
+  auto write = [&](const float4& x, int c, const float4& wi, const float4& bi) {
     float4 o;
     if constexpr (kOp == kOpLayerNorm)
       o = make_float4(fmaf(x.x, mul, add), fmaf(x.y, mul, add), fmaf(x.z, mul, add), fmaf(x.w, mul, add));
     else
       o = make_float4(x.x * mul, x.y * mul, x.z * mul, x.w * mul);
-    if constexpr (kOp != kOpSoftmax) {
-      const float4 wi = early_w != nullptr ? *early_w : __ldg(w4 + c);
-      if constexpr (kOp == kOpRmsNorm) {
-        o = make_float4(o.x * wi.x, o.y * wi.y, o.z * wi.z, o.w * wi.w);
-      } else {
-        const float4 bi = early_b != nullptr ? *early_b : __ldg(b4 + c);
-        o = make_float4(fmaf(o.x, wi.x, bi.x), fmaf(o.y, wi.y, bi.y), fmaf(o.z, wi.z, bi.z), fmaf(o.w, wi.w, bi.w));
-      }
-    }
+    if constexpr (kOp == kOpRmsNorm)
+      o = make_float4(o.x * wi.x, o.y * wi.y, o.z * wi.z, o.w * wi.w);
+    else if constexpr (kOp == kOpLayerNorm)
+      o = make_float4(fmaf(o.x, wi.x, bi.x), fmaf(o.y, wi.y, bi.y), fmaf(o.z, wi.z, bi.z), fmaf(o.w, wi.w, bi.w));
     __stcs(y4 + c, o);
   };
+  if constexpr (kOp == kOpSoftmax) {
 #pragma unroll
-  for (int i = 0; i < kVec; ++i) {
-    const int c = t + i * tpr;
-    if (c < p.n4)
-      write(v[i], c, kEarly ? &w[kEarly ? i : 0] : nullptr,
-            kEarly && kOp == kOpLayerNorm ? &b[kEarly && kOp == kOpLayerNorm ? i : 0] : nullptr);
-  }
-  // (Two at a time for softmax, whose groups need nothing fetched: 4096 x 30000 155.5 us with four, 152.5 with
-  // two, 600 x 30000 29.5 and 27.5, 8000 x 24000 236.6 and 229.3; the norms, 4096 x 30000, 166 and 173, 154 and 157.)
-  constexpr int kStoreUnroll = kOp == kOpSoftmax ? 2 : 4;
-#pragma unroll(kStoreUnroll)
-  for (int i = 0; i < kPark; ++i) {
-    const int c = t + (kVec + i) * tpr;
-    if (c < p.n4) write(parked[i * tpr + t], c, nullptr, nullptr);
+    for (int i = 0; i < kVec; ++i) {
+      const int c = t + i * tpr;
+      if (c < p.n4) write(v[i], c, v[i], v[i]);
+    }
+    // (Two at a time: 4096 x 30000 155.5 us with four, 152.5 with two, 600 x 30000 29.5 and 27.5, 8000 x 24000
+    // 236.6 and 229.3.)
+#pragma unroll 2
+    for (int i = 0; i < kPark; ++i) {
+      const int c = t + (kVec + i) * tpr;
+      if (c < p.n4) write(parked[i * tpr + t], c, v[0], v[0]);
+    }
+  } else {
+    // Layer norm fetches a parked half four groups at a time, behind the stores of the first, whose
+    // registers that takes; RMS norm goes on one by one (423 x 23104 17.3 us, 18.0 four at a time).
+    constexpr int kRolling = kOp == kOpLayerNorm ? kVec : kVec + kPark;
+#pragma unroll
+    for (int i = 0; i < kRolling; ++i) {
+      const int c = t + i * tpr;
+      if (c < p.n4)
+        write(i < kVec ? v[i < kVec ? i : 0] : parked[(i - kVec) * tpr + t], c, w[i % kAhead],
+              b[kOp == kOpLayerNorm ? i % kAhead : 0]);
+      if (i + kAhead < kRolling) fetch(i + kAhead);
+    }
+#pragma unroll 1
+    for (int g = kRolling - kVec; g < kPark; g += 4) {
+      float4 wg[4], bg[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) fetch_into(kVec + g + i, wg[i], bg[i]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int c = t + (kVec + g + i) * tpr;
+        if (c < p.n4) write(parked[(g + i) * tpr + t], c, wg[i], bg[i]);
+      }
+    }
   }
 }
 

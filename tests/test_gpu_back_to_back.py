@@ -2,6 +2,10 @@
 host_common.h): chains in which every call reads what the one before wrote, or writes what it
 read, give the same bits as with a wait for the GPU behind every call -- eagerly, in a replayed
 graph, beside the framework's own kernels and copies, and on two streams at once."""
+import ctypes
+import os
+import subprocess
+
 import pytest
 import torch
 
@@ -128,3 +132,37 @@ def test_weights_written_right_ahead_of_the_call(pkg, gpu, rows, N):
     assert all(bool(torch.isfinite(t).all()) for t in want)
     for _ in range(3):
         assert all(torch.equal(a, b) for a, b in zip(run(False), want))
+
+
+@pytest.fixture(scope="module")
+def early_writer(pkg, tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("early") / "early_writer.so")
+    src = os.path.join(os.path.dirname(os.path.abspath(__file__)), "device", "early_writer.cu")
+    subprocess.run([pkg.build._nvcc(), *pkg.build.NVCC_FLAGS, "-shared", src, "-o", so], check=True)
+    lib = ctypes.CDLL(so)
+    lib.launch_early_writer.argtypes = [ctypes.c_void_p] * 3 + [ctypes.c_int, ctypes.c_longlong, ctypes.c_int, ctypes.c_void_p]
+    return lib.launch_early_writer
+
+
+@pytest.mark.parametrize("rows,N", [(16, 512), (16, 2048), (3000, 256), (2000, 1024), (2000, 4096), (148, 12000), (148, 20000),
+                                    (600, 20000)])
+def test_weights_written_late_by_a_kernel_that_lets_the_norm_in_early(pkg, gpu, early_writer, rows, N):
+    """The norm's blocks start while the kernel in front still has the old weights in every SM's L1
+    cache and has not written the new ones; the result is the new ones' all the same."""
+    g = torch.Generator(device=gpu).manual_seed(N)
+    x = torch.randn(rows, N, device=gpu, generator=g)
+    old, new = (torch.randn(2 * N, device=gpu, generator=g) for _ in range(2))
+    blocks = torch.cuda.get_device_properties(gpu).multi_processor_count
+    data, sink, out = old.clone(), torch.empty(blocks * 256, device=gpu), torch.empty_like(x)
+    w, b = data[:N], data[N:]
+    norms = {"layer": lambda w, b: pkg.ops.layer_norm(x, w, b, out=out), "rms": lambda w, b: pkg.ops.rms_norm(x, w, out=out)}
+    for norm in norms.values():
+        want = norm(new[:N], new[N:]).clone()
+        for _ in range(4):
+            data.copy_(old)
+            norm(w, b)                       # the old weights' lines in the caches of the norm's own path too
+            torch.cuda.synchronize()
+            assert early_writer(data.data_ptr(), new.data_ptr(), sink.data_ptr(), 2 * N, 40000, blocks,
+                                torch.cuda.current_stream().cuda_stream) == 0
+            norm(w, b)
+            assert torch.equal(out, want)
