@@ -65,7 +65,6 @@ namespace ptxb200 {
 namespace {
 
 constexpr int kThreads = 512;
-constexpr unsigned kLetInMaxCtas = 74;   // half of the SMs
 #ifndef PTXB200_FA_REGS_SOFTMAX
 #define PTXB200_FA_REGS_SOFTMAX 168
 #define PTXB200_FA_REGS_CORRECTION 104
@@ -187,6 +186,7 @@ struct FaParams {
   int heads_q;          // query heads per batch entry
   int heads_kv;         // key/value heads per batch entry (divides heads_q)
   int pair_mode;        // causal only: items are dealt out in pairs (see ItemIter)
+  int let_in;           // the next launch may start as this one's last loads are under way (see let_in_next)
   // Launches whose last round is cut along the key axis (the kTail kernels) only:
   FaSched sched;          // the round-robin part and the cut part of the distribution (attn_sched.cuh)
   float* parts;           // one slot of parked pieces per CTA
@@ -699,10 +699,6 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
   grid_wait();
   tc_fence_before();
   __syncthreads();
-  // The next launch is let in where it finds SMs without a CTA of this one (2 heads of 512 keys 10.55 us a
-  // launch, 10.85 without). CTAs of it that move in beside the last ones of a full grid measured 1.5 %
-  // slower (32 heads on 8 of 3001 keys 88.7 us and 87.2).
-  if (gridDim.x <= kLetInMaxCtas) grid_trigger();
   FA_CTA_TIME(1);
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
@@ -749,6 +745,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
             if (j + 1 < nt1) kv_load(&tmap_k, kv_row0 + (j + 1) * kAttnRows, kv_slice);
           }
         }
+        if (p.let_in) grid_trigger();
         if (p.dbg != nullptr && blockIdx.x == 0) p.dbg[0] = kv_it;
       }
     } else if (warp == 12) {
@@ -1438,9 +1435,15 @@ constexpr size_t kPartsHeaderBytes = 4096;   // one flag word per CTA, ahead of 
 template <int D>
 constexpr size_t parts_slot_bytes() { return (size_t)2 * (256 + kAttnRows * D) * sizeof(float); }
 
+// The next launch is let in where it finds at least as many SMs without a CTA of this one (2 heads of
+// 512 keys 10.6 us a launch, 11.1 without; 8 heads of 2048 29.4 and 29.8). Its CTAs beside the last ones
+// of a fuller grid cost more than that gains (12 heads of 1920 keys, 96 CTAs, 29.5 us and 28.5 without; 32
+// heads of 300, causal, on all SMs 46.6 and 45.7).
+int let_in_next(int grid, int sm_count) { return 2 * grid <= sm_count ? 1 : 0; }
+
 template <int D, bool kCausal>
 int launch_variant(const DeviceCtx& ctx, const CUtensorMap& tq, const CUtensorMap& tk,
-                   const CUtensorMap& tv, const FaParams& p, cudaStream_t stream) {
+                   const CUtensorMap& tv, FaParams& p, cudaStream_t stream) {
   using C = FaCfg<D>;
   static PerDeviceOnce attr_once;   // one per <D, kCausal> instantiation
   const int rc = attr_once.run(ctx.device, []() -> int {
@@ -1467,6 +1470,7 @@ int launch_variant(const DeviceCtx& ctx, const CUtensorMap& tq, const CUtensorMa
   if (rc != PTXB200_OK) return rc;
   const bool ragged = !kCausal && p.seqlen % kAttnRows != 0;
   auto launch = [&](auto* kernel, int grid) {
+    p.let_in = let_in_next(grid, ctx.sm_count);
     return launch_after(stream, kernel, (unsigned)grid, kThreads, C::kSmemBytes, 1u, tq, tk, tv, p);
   };
   if (p.sched.tail_units > 0) {
@@ -1507,6 +1511,7 @@ void fill_params(FaParams& p, void* O, void* lse, int B, int H, int H_kv, int S,
   p.heads_q = H;
   p.heads_kv = H_kv;
   p.pair_mode = sc.pair_mode;
+  p.let_in = 0;
   p.sched = sc;
   p.parts = nullptr;
   p.part_flags = nullptr;
@@ -1722,6 +1727,7 @@ extern "C" int fa_fwd_bf16_noalloc(void* O, const void* Q, const void* K, const 
   p.cta_flags = nd.scratch + kNoAllocFlagBase;
   const int units = (causal && p.pair_mode) ? p.bh * ((p.num_mblocks + 1) / 2) : p.total_work;
   const int grid = units < nd.sm_count ? units : nd.sm_count;
+  p.let_in = let_in_next(grid, nd.sm_count);
   if (grid > kNoAllocMaxCtas) {
     set_error_text("fa_fwd_bf16_noalloc: launch needs more CTAs than the 240 flag slots of the "
                    "static scratch array");

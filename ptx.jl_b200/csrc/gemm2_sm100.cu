@@ -116,7 +116,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   grid_wait();
   tc_fence_before();
   __syncthreads();
-  grid_trigger();
   cluster_sync_all();     // both CTAs' barriers exist before anything remote is signalled
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
@@ -153,6 +152,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           tma_load_2d_pair(b_base + s * C::kBStage, &tmap_b, k * kBK2, b_row, leader_full + 8 * s);
         }
       }
+      grid_trigger();
     }
   } else if (warp == 1) {
     // ---------------- MMA issue (leader only; converged warp, elected lane) ----------------

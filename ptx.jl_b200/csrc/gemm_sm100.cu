@@ -116,7 +116,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   grid_wait();
   tc_fence_before();
   __syncthreads();
-  grid_trigger();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
@@ -147,6 +146,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
           tma_load_2d(b_base + s * kBStageBytes, &tmap_b, k * kBK, b_row, bar_full + 8 * s);
         }
       }
+      grid_trigger();
     }
   } else if (warp == 1) {
     // ---------------- MMA issue ----------------

@@ -185,7 +185,6 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   grid_wait();
   tc_fence_before();
   __syncthreads();
-  grid_trigger();
   if (kSplit) cluster_arrive();          // "this CTA has started": waited for ahead of the first store to a peer
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
@@ -199,6 +198,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         load(i, s);
         if (++s == stages) { s = 0; ph ^= 1u; }
       }
+      grid_trigger();
     }
     __syncwarp();
   } else if (!misaligned && warp == 1) {

@@ -541,9 +541,13 @@ __device__ __forceinline__ void st_global_v4(void* p, uint32_t a, uint32_t b, ui
 // Programmatic dependent launch (launch_after, host_common.h). grid_wait: until the stream's work
 // ahead of this launch is complete and its memory visible; ahead of it a kernel touches no global
 // memory, so that only its set-up runs beside the kernel in front. grid_trigger: from the time
-// on when every CTA has called it (or left) the next such launch may take up free SMs; called
-// behind the allocation of tensor memory, so that none of this launch's CTAs waits for that of one
-// which waits for this launch.
+// on when a thread of every CTA has called it (or the CTA has left) the next such launch may take up
+// free SMs, and keeps them while it waits. So it is called as late as the next launch's set-up still fits
+// in: by the thread that loads, behind its last load. (At a kernel's start: no faster, and work on another
+// stream, which could have run beside a long launch on few SMs, had to wait for its end: five
+// products of 512 x 512 x 128 beside one of 128 x 256 x 131072 766 us with another behind that, 21 this
+// way.) And behind the allocation of tensor memory, so that none of this launch's CTAs waits for that of
+// one which waits for this launch.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

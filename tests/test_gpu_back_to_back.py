@@ -166,3 +166,51 @@ def test_weights_written_late_by_a_kernel_that_lets_the_norm_in_early(pkg, gpu, 
                                 torch.cuda.current_stream().cuda_stream) == 0
             norm(w, b)
             assert torch.equal(out, want)
+
+
+FRONTS = {"attention": None, "one CTA": dict(M=128, N=256, K=131072, no_split=True, one_cta=True),
+          "pair": dict(M=256, N=256, K=131072, no_split=True), "split": dict(M=128, N=128, K=262144)}
+
+
+@pytest.mark.parametrize("front", FRONTS)
+def test_the_launch_behind_leaves_the_sms_to_other_streams(pkg, gpu, front):
+    """A long launch on at most half of the SMs, and one behind it that fills the machine: what
+    another stream brings meanwhile runs on the SMs left, and does not wait for the first's end."""
+    def bf16(*shape):
+        return torch.zeros(*shape, device=gpu, dtype=torch.bfloat16)
+
+    if FRONTS[front] is None:
+        q = bf16(1, 1, 256 * (torch.cuda.get_device_properties(gpu).multi_processor_count // 2), 128)
+        o = torch.empty_like(q)
+        first = lambda s: pkg.ops.fa_fwd(q, q, q, out=o, flags=pkg.native.FA_NO_TAIL_SPLIT, stream=s)
+    else:
+        kw = dict(FRONTS[front])
+        M, N, K = kw.pop("M"), kw.pop("N"), kw.pop("K")
+        a, b, c = bf16(M, K), bf16(N, K), bf16(M, N)
+        first = lambda s: pkg.ops.gemm(a, b, out=c, stream=s, **kw)
+    a2, b2, c2 = bf16(4096, 512), bf16(4096, 512), bf16(4096, 4096)
+    a3, b3, c3 = bf16(512, 128), bf16(512, 128), bf16(512, 512)
+    main, side = torch.cuda.Stream(), torch.cuda.Stream()
+    event = lambda: torch.cuda.Event(enable_timing=True)
+
+    def times(second):
+        torch.cuda.synchronize()
+        start, end, side_end = event(), event(), event()
+        with torch.cuda.stream(main):
+            torch.cuda._sleep(1000000)               # half a millisecond: all is queued before anything runs
+            start.record(main)
+            first(main)
+            if second:
+                pkg.ops.gemm(a2, b2, out=c2, stream=main)
+            end.record(main)
+        side.wait_event(start)
+        for _ in range(3):
+            pkg.ops.gemm(a3, b3, out=c3, stream=side)
+        side_end.record(side)
+        torch.cuda.synchronize()
+        return start.elapsed_time(end), start.elapsed_time(side_end)
+
+    times(True)
+    alone = min(times(False)[0] for _ in range(3))
+    assert min(times(True)[1] for _ in range(3)) < 0.6 * alone
+    assert pkg.ops.sync_status() == 0
