@@ -628,7 +628,9 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
   const uint32_t base = smem_u32(smem_raw);
   if ((base & 1023u) != 0) {
     // the 128-byte swizzle needs 1024-byte aligned tiles; every thread leaves before
-    // any barrier or allocation exists
+    // any barrier or allocation exists, but not before the stream's work in front is complete:
+    // the launch behind waits for no more than this one
+    grid_wait();
     if (threadIdx.x == 0 && p.status != nullptr) atomicCAS(p.status, 0u, kStatusTimeoutTag | (17u << 8));
     return;
   }

@@ -95,7 +95,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   const int lane = threadIdx.x & 31;
   // the swizzled tiles need a 1024-byte aligned base; both CTAs of a pair see the same offset
   const bool misaligned = (base & 1023u) != 0;
-  if (misaligned && threadIdx.x == 0 && status != nullptr) atomicCAS(status, 0u, kStatusTimeoutTag | (17u << 8));
+  if (misaligned && threadIdx.x == 0 && status != nullptr) {
+    grid_wait();
+    atomicCAS(status, 0u, kStatusTimeoutTag | (17u << 8));
+  }
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;

@@ -124,7 +124,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const bool misaligned = (base & 1023u) != 0;   // the swizzled tiles need a 1024-byte aligned base
-  if (misaligned && threadIdx.x == 0 && status != nullptr) atomicCAS(status, 0u, kStatusTimeoutTag | (17u << 8));
+  if (misaligned && threadIdx.x == 0 && status != nullptr) {
+    grid_wait();
+    atomicCAS(status, 0u, kStatusTimeoutTag | (17u << 8));
+  }
 
   const int tiles_m = M / kBM3, tiles_n = (N + kBN - 1) / kBN;
   const int tiles_per_group = tiles_m * tiles_n;

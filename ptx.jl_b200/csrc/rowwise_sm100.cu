@@ -127,8 +127,8 @@ rowwise_kernel(const RowParams p) {
   const int tpr = kWarpRows ? 32 : blockDim.x;       // threads per row
   const int t = kWarpRows ? threadIdx.x & 31 : threadIdx.x;
   const int row = kWarpRows ? blockIdx.x * 4 + (threadIdx.x >> 5) : blockIdx.x;
-  if (kWarpRows && row >= p.rows) return;            // the last block's rows may be fewer; no block barrier follows
   grid_wait();
+  if (kWarpRows && row >= p.rows) return;            // the last block's rows may be fewer; no block barrier follows
   const float4* x4 = behind(reinterpret_cast<const float4*>(p.x)) + (size_t)row * p.n4;
   float4* y4 = reinterpret_cast<float4*>(p.y) + (size_t)row * p.n4;
   const float4* w4 = behind(reinterpret_cast<const float4*>(p.w));
