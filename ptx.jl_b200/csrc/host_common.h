@@ -140,7 +140,9 @@ cudaError_t launch_after(cudaStream_t stream, void (*kernel)(P...), unsigned gri
   attr[1].val.clusterDim = {cluster, 1, 1};
   cfg.attrs = attr;
   cfg.numAttrs = cluster > 1 ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, kernel, args...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+  if (e != cudaSuccess) cudaGetLastError();   // reported by the caller: not left for the next check of the runtime's last error
+  return e;
 }
 
 // Kernel launchers (one per .cu file).
