@@ -134,7 +134,8 @@ def test_every_tile_once_and_never_busier_than_round_robin(pkg, causal):
         if BH * S > 1_000_000:
             continue
         for flags in ([0, FA_SINGLE_BLOCKS] if causal else [0]):
-            # the default policy cuts only where it expects a gain of a twelfth or more ...
+            # the default policy cuts only where it expects a gain (test_attention_cut_choice.py), beside
+            # the three steps that a second segment costs at least a twelfth or more ...
             sc, ctas = plan(pkg, BH, S, causal, flags)
             worst, _ = check_plan(sc, ctas)
             if sc["tail_units"] > 0:
@@ -158,8 +159,8 @@ def test_an_eighth_of_the_headline_problem_fills_every_sm(pkg):
     """B*H = 8 heads of S = 4096 (one GPU's share of the headline problem split eight
     ways): 128 items of 32 steps on 148 SMs. The round robin leaves 20 SMs idle for the whole
     launch; cut, every SM runs 27-28 steps. The default policy leaves this launch whole --
-    a second segment with its parking and merging costs about three steps, measured, and
-    four are saved -- so the cut is forced here."""
+    a cut costs nine steps and more, measured, and four are saved -- so the cut is forced
+    here."""
     assert plan(pkg, 8, 4096, False)[0]["tail_units"] == 0
     sc, ctas = plan(pkg, 8, 4096, False, FA_ALWAYS)
     assert (sc["grid"], sc["full"], sc["tail_units"], sc["tail_steps"], sc["tail_ctas"]) == (148, 0, 128, 4096, 148)

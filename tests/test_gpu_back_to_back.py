@@ -31,7 +31,7 @@ def chain(ops, case, g, sync):
         for i in range(4):
             yield lambda: ops.gemm(x, b[i & 1], out=c)             # reads what the last turn wrote
             yield lambda: ops.gemm(c, w, out=x)                    # over the operand just read
-            if K in (64, 128):
+            if K == 128:
                 yield lambda: q.view(M, K).copy_(x)                # a copy of the framework's between
                 yield lambda: ops.fa_fwd(q, q, q, causal=bool(i & 1), out=o)
                 yield lambda: x.copy_(o.view(M, K))
@@ -42,7 +42,7 @@ def chain(ops, case, g, sync):
     for call in calls():
         call()
         done()
-    return [c, x, y] + ([o] if K in (64, 128) else [])
+    return [c, x, y] + ([o] if K == 128 else [])
 
 
 CASES = [(128, 128, 128), (1024, 1152, 128), (4096, 4096, 128), (2048, 2048, 512), (256, 4096, 4096)]
@@ -132,6 +132,155 @@ def test_weights_written_right_ahead_of_the_call(pkg, gpu, rows, N):
     assert all(bool(torch.isfinite(t).all()) for t in want)
     for _ in range(3):
         assert all(torch.equal(a, b) for a, b in zip(run(False), want))
+
+
+def turns(calls, state, n, sync, turn_buffer=None):
+    """`n` turns of the calls, behind each other or with a wait for the GPU behind every one. With
+    `turn_buffer`, that buffer must hold something else after every turn: what an earlier turn left would show."""
+    seen = []
+    for i in range(n):
+        for call in calls(state, i):
+            call()
+            if sync:
+                torch.cuda.synchronize()
+        if turn_buffer is not None:
+            seen.append(state[turn_buffer].clone())
+    torch.cuda.synchronize()
+    assert not any(torch.equal(a, b) for i, a in enumerate(seen) for b in seen[:i])
+    return {k: t.clone() for k, t in state.items()}
+
+
+def check_turns(calls, make, n, turn_buffer):
+    want = turns(calls, make(), n, True, turn_buffer)
+    assert all(bool(torch.isfinite(t.float()).all()) for t in want.values())
+    for _ in range(4):
+        got = turns(calls, make(), n, False)
+        assert all(torch.equal(got[k], want[k]) for k in want)
+
+
+# what launch: B, H, H_kv, S, causal, flags of ops.fa_fwd, and what ptxb200_fa_plan_ex says of it
+ATTENTION = {
+    "few items": ((1, 2, 2, 512, False, 0), dict(tail=False, by_length=0, fits=True)),
+    "several items a CTA": ((1, 40, 40, 1024, False, 0x4), dict(tail=False, by_length=0, fits=False)),
+    "ragged": ((2, 40, 10, 1000, False, 0x4), dict(tail=False, by_length=0, fits=False)),
+    "cut": ((1, 16, 16, 1024, False, 0x8), dict(tail=True, by_length=0, fits=False)),
+    "cut, ragged": ((1, 20, 4, 1500, False, 0x8), dict(tail=True, by_length=0, fits=False)),
+    "cut, causal": ((1, 20, 20, 1100, True, 0x8), dict(tail=True, by_length=0, fits=False)),
+    "by length": ((1, 32, 8, 1501, True, 0x4), dict(tail=False, by_length=1, fits=False)),
+    "pairs": ((1, 37, 37, 1024, True, 0x4), dict(tail=False, by_length=0, fits=False)),
+}
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("kind", ATTENTION)
+def test_attention_behind_attention(pkg, gpu, kind, D):
+    """Two calls of one kind over the same buffers in turn, each reading as queries and as keys what the
+    one ahead wrote, with the log-sum-exp going through a softmax in between. The scores are wide
+    enough (scale 0.5) that the outputs stay apart."""
+    (B, H, H_kv, S, causal, flags), expect = ATTENTION[kind]
+    buf = (ctypes.c_int * 20000)()
+    sm = torch.cuda.get_device_properties(gpu).multi_processor_count
+    assert pkg.native.lib().ptxb200_fa_plan_ex(B, H, H_kv, S, D, int(causal), flags, sm, buf, 20000) > 0
+    assert (buf[7] > 0) == expect["tail"] and buf[10] == expect["by_length"] and (2 * buf[5] <= sm) == expect["fits"]
+
+    def make():
+        g = torch.Generator(device=gpu).manual_seed(S + D)
+        bf = lambda h: torch.randn(B, h, S, D, device=gpu, generator=g).to(torch.bfloat16)
+        return dict(q=bf(H), k=bf(H_kv), v=bf(H_kv), o=torch.empty(B, H, S, D, device=gpu, dtype=torch.bfloat16),
+                    lse=torch.empty(B * H, S, device=gpu), y=torch.zeros(B * H, S // 4 * 4, device=gpu))
+
+    def calls(t, i):
+        fa = lambda q, o, lse=None: pkg.ops.fa_fwd(q, t["k"], t["v"], causal=causal, sm_scale=0.5, flags=flags, out=o, lse=lse)
+        yield lambda: fa(t["q"], t["o"])
+        yield lambda: fa(t["o"], t["q"], t["lse"])
+        if S % 4 == 0:
+            yield lambda: pkg.ops.softmax(t["lse"], out=t["y"])
+        if H == H_kv:
+            yield lambda: pkg.ops.fa_fwd(t["q"], t["o"], t["v"], causal=causal, sm_scale=0.5, flags=flags, out=t["k"])
+        else:
+            yield lambda: t["k"].copy_(t["q"][:, i % 4::H // H_kv][:, :H_kv])
+
+    check_turns(calls, make, 4, "q")
+    assert pkg.ops.sync_status() == 0
+
+
+def test_attention_without_allocations_behind_attention(pkg, gpu):
+    """fa_fwd_bf16_noalloc clears its status words ahead of every launch."""
+    B, H, S, D = 1, 20, 1024, 128
+    lib, stream = pkg.native.lib(), torch.cuda.current_stream().cuda_stream
+
+    def make():
+        g = torch.Generator(device=gpu).manual_seed(3)
+        bf = lambda: torch.randn(B, H, S, D, device=gpu, generator=g).to(torch.bfloat16)
+        return dict(q=bf(), k=bf(), v=bf(), o=bf())
+
+    def calls(t, i):
+        def fa(q, k, o, causal):
+            assert lib.fa_fwd_bf16_noalloc(t[o].data_ptr(), t[q].data_ptr(), t[k].data_ptr(), t["v"].data_ptr(), B, H, S, D, 0.5,
+                                           causal, 0, stream) == 0
+        yield lambda: fa("q", "k", "o", 0)
+        yield lambda: fa("o", "k", "q", 1)
+        yield lambda: fa("q", "o", "k", 0)
+        yield lambda: pkg.ops.fa_fwd(t["k"], t["q"], t["v"], sm_scale=0.5, out=t["o"])
+
+    check_turns(calls, make, 4, "q")
+    flags = (ctypes.c_uint32 * 240)()
+    assert lib.fa_fwd_bf16_noalloc_status(flags, 240, stream) == 0 and not any(flags)
+
+
+# M, N, K and options of the product; which kernel runs it
+PRODUCTS = {"split": (128, 1024, 1024, {}), "pair": (2560, 4096, 256, dict(no_split=True)),
+            "one CTA": (640, 512, 256, dict(no_split=True, one_cta=True)), "few steps": (256, 512, 64, {})}
+
+
+@pytest.mark.parametrize("norm", ["layer", "rms"])
+@pytest.mark.parametrize("kind", PRODUCTS)
+def test_norm_directly_behind_the_product_that_makes_its_weights(pkg, gpu, kind, norm):
+    """A product lets the launch behind it in early: here a norm whose weights, bias and rows are that
+    product's, and then the next product over the same buffer."""
+    M, N, K, kw = PRODUCTS[kind]
+
+    def make():
+        g = torch.Generator(device=gpu).manual_seed(M)
+        bf = lambda r: torch.randn(r, K, device=gpu, generator=g).mul_(K ** -0.25).to(torch.bfloat16)
+        return dict(a=bf(M), b0=bf(N), b1=bf(N), b2=bf(N), c=torch.empty(M, N, device=gpu), y=torch.empty(M - 4, N, device=gpu))
+
+    def calls(t, i):
+        rows, w, bias = t["c"][4:], t["c"][i % 4], t["c"][(i + 1) % 4]
+        yield lambda: pkg.ops.gemm(t["a"], t["b%d" % (i % 3)], f32_out=True, out=t["c"], **kw)
+        if norm == "layer":
+            yield lambda: pkg.ops.layer_norm(rows, w, bias, out=t["y"])
+        else:
+            yield lambda: pkg.ops.rms_norm(rows, w, out=t["y"])
+        yield lambda: pkg.ops.gemm(t["a"], t["b%d" % ((i + 1) % 3)], f32_out=True, out=t["c"], **kw)
+        yield lambda: pkg.ops.swiglu(t["y"], rows, out=t["y"])
+        yield lambda: t["a"][:M - 4].copy_(t["y"][:, :K].clamp(-2, 2))
+
+    check_turns(calls, make, 6, "y")
+    assert pkg.ops.sync_status() == 0
+
+
+@pytest.mark.parametrize("G,M,N,K,f32", [(64, 256, 1024, 512, False), (8, 128, 512, 512, True), (6, 128, 256, 256, True)])
+def test_groups_of_products_behind_one_another(pkg, gpu, G, M, N, K, f32):
+    def make():
+        g = torch.Generator(device=gpu).manual_seed(G)
+        bf = lambda *s: torch.randn(*s, device=gpu, generator=g).mul_(K ** -0.25).to(torch.bfloat16)
+        dtype = torch.float32 if f32 else torch.bfloat16
+        return dict(a=bf(G, M, K), b=bf(G, N, K), w=bf(G, K, N), c=torch.empty(G, M, N, device=gpu, dtype=dtype),
+                    x=torch.zeros(G, M, K, device=gpu, dtype=torch.bfloat16), y=torch.zeros(G * M, N, device=gpu))
+
+    def calls(t, i):
+        yield lambda: pkg.ops.gemm_grouped(t["a"], t["b"], f32_out=f32, out=t["c"])
+        if f32:
+            yield lambda: pkg.ops.softmax(t["c"].view(G * M, N), out=t["y"])
+            yield lambda: t["a"].copy_(t["c"][:, :, :K].clamp(-2, 2))
+        else:
+            yield lambda: pkg.ops.gemm_grouped(t["c"], t["w"], out=t["x"])
+            yield lambda: pkg.ops.gemm_grouped(t["x"], t["b"], out=t["c"])
+            yield lambda: t["a"].copy_(t["x"].clamp(-2, 2))
+
+    check_turns(calls, make, 5, "a")
+    assert pkg.ops.sync_status() == 0
 
 
 @pytest.fixture(scope="module")
