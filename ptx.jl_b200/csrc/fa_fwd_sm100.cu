@@ -1343,7 +1343,8 @@ FaSched plan_schedule(int bh, int nmb, int nt_all, int causal, unsigned flags, i
 
 // Round robin over whole units (the reference's distribution); causal items by length; or
 // round robin with the last, partly filled round cut along the key axis when that shortens
-// the busiest CTA's work by more than the overhead of the cut.
+// the busiest CTA's work by more than all that a cut costs the launch (kCutSteps128, kCutSteps64 and a
+// step per further piece).
 FaSched plan_uncached(int bh, int nmb, int nt_all, int causal, unsigned flags, int sm_count, bool may_split, bool kv_in_l2,
                       int head_dim) {
   FaSched legacy;
@@ -1361,7 +1362,7 @@ FaSched plan_uncached(int bh, int nmb, int nt_all, int causal, unsigned flags, i
   if (causal && kv_in_l2 && !(flags & (PTXB200_FA_SINGLE_BLOCKS | PTXB200_FA_ALWAYS_TAIL_SPLIT)) &&
       (long long)bh * nmb <= kByLengthMaxItems && (long long)bh * nmb > sm_count) {
     // 32 heads on 8 K/V heads, head dim 128: 2048 keys 43.6 us in pairs, 40.5 by length; 3001 keys
-    // 99.9 with the last round cut, 78.8 by length (32 steps on average, the busiest CTA has 36
+    // 99.9 with the last round cut, 78.8 by length (33.7 steps on average, the busiest CTA has 38
     // and two boundaries, no merging); 2 x 32 heads of 4096 keys, K and V 134 MB, 293 and 257.
     const long long by_length = worst_by_length(bh, nmb, nt_all, sm_count);
     const long long items = (long long)bh * nmb;

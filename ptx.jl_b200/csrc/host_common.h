@@ -123,8 +123,9 @@ int encode_tmap_bf16_3d(CUtensorMap* out, const void* base, uint64_t slices, uin
 
 // Launches `kernel` in clusters of `cluster` CTAs (1: none) so that its set-up may run beside the end
 // of the stream's kernel in front of it: the kernel waits (grid_wait) before it touches global
-// memory. Back-to-back launches are 3.0-4.2 us apart beyond their own time, and in steps of 2.05 us,
-// without this, 1.0-1.4 us with it (a kernel of 7 us on 148 SMs: 10.3 and 8.1 us a launch).
+// memory. Back-to-back launches are 2.9-4.5 us apart beyond their own time, and in steps of about 2 us,
+// without this, 1.5-2.0 us with it and 1.3-1.4 behind a kernel that lets the next one in (grid_trigger). A
+// kernel of 6.6 us on 148 SMs: 10.3, 8.6 and 8.0 us a launch.
 template <class... P, class... A>
 cudaError_t launch_after(cudaStream_t stream, void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem, unsigned cluster,
                          A... args) {
